@@ -279,8 +279,8 @@ template <typename T, int V, int TX, int TY, int NS, int MINB, bool HINT = false
 // one ens_pad_kernel for the periodic padding of the buffer written. An odd
 // step count first copies the state arena (padding included) to the work
 // arena, so that the last step writes the state arena.
-template <int TX, int TY, int NS, int THREADS> struct EnsFusedConfig {
-    using S = LevelFusedShape<TX, TY, NS, THREADS>;
+template <int TX, int TY> struct EnsFusedConfig {
+    using S = LevelFusedShape<TX, TY>;
 
     static int prepare()
     {
@@ -358,12 +358,11 @@ template <int TX, int TY, int NS, int THREADS> struct EnsFusedConfig {
     }
 };
 
-// Whether every box suits a fused tiling of tile height ty: ny a multiple of
-// ty, nx even (the last tile column may be partial, its sites come in pairs).
+// Whether every box suits a fused tiling of tile height ty.
 static bool fused_fits(const int32_t *dims, int nboxes, int ty)
 {
     for (int b = 0; b < nboxes; ++b)
-        if (dims[3 * b] % 2 != 0 || dims[3 * b + 1] % ty != 0) return false;
+        if (!fused_takes_ny(dims[3 * b + 1], ty)) return false;
     return true;
 }
 
@@ -373,7 +372,7 @@ static bool fused_fits(const int32_t *dims, int nboxes, int ty)
 // 16-wide tiles leave no idle columns on boxes whose width is a multiple of
 // 16 but read 96-byte rows.
 static const EnsTiling kEnsF32[] = {
-    EnsFusedConfig<32, 16, 6, 640>::entry("f32 fused 32x16 ring6 t640"),
+    EnsFusedConfig<32, 16>::entry("f32 fused 32x16 columns"),
     EnsConfig<float, 2, 64, 8, 8, 2>::entry("f32 v2 64x8 ring8"),
     EnsConfig<float, 2, 32, 8, 8, 3>::entry("f32 v2 32x8 ring8"),
     EnsConfig<float, 1, 32, 8, 8, 3>::entry("f32 v1 32x8 ring8"),
@@ -508,7 +507,7 @@ int axs_ensemble_init(const axs_ensemble *e, axs_ensemble_plan *plan, void *stre
     AXS_REQUIRE(cfg != nullptr, AXS_ERR_INVALID_ARGUMENT, "tile_config %d out of range (0..%d)", plan->tile_config,
                 ens_config_count(e->dtype));
     AXS_REQUIRE(!cfg->fused || fused_fits(e->dims, e->nboxes, cfg->ty), AXS_ERR_UNSUPPORTED,
-                "tiling '%s' needs every box's ny a multiple of %d and nx even", cfg->name, cfg->ty);
+                "tiling '%s' needs every box's ny to be %d or at least %d", cfg->name, cfg->ty, cfg->ty + 4);
     AXS_REQUIRE(plan->z_chunk >= 0, AXS_ERR_INVALID_ARGUMENT, "negative z_chunk");
     int cap_a = 0, cap_b = 0;
     if ((rc = cfg->caps(cap_a, cap_b))) return rc;
@@ -561,7 +560,7 @@ int axs_ensemble_init(const axs_ensemble *e, axs_ensemble_plan *plan, void *stre
         const char *sbase = static_cast<const char *>(e->state) + geo.base[b] * es;
         const char *wbase = static_cast<const char *>(e->work) + geo.base[b] * es;
         if (cfg->fused) {
-            // full box, TY + 4 rows of one component, 2 rows of one component (level_fused.cuh)
+            // full box, TY + 4 rows of one component, 4 rows of one component (level_fused.cuh)
             auto *maps = reinterpret_cast<CUtensorMap *>(img.data() + maps_off) + kEnsMapsPerBox * b;
             for (int sel = 0; sel < 2; ++sel) {
                 const char *base = sel ? wbase : sbase;
@@ -571,7 +570,7 @@ int axs_ensemble_init(const axs_ensemble *e, axs_ensemble_plan *plan, void *stre
                                              1, 4)) ||
                     (rc = make_tensor_map_4d(&m[1], base, e->dtype, d0, d1, nz, 4, sj, sk, sc, cfg->box_x,
                                              (uint32_t)cfg->ty + 4, 1, 1)) ||
-                    (rc = make_tensor_map_4d(&m[2], base, e->dtype, d0, d1, nz, 4, sj, sk, sc, cfg->box_x, 2, 1, 1)))
+                    (rc = make_tensor_map_4d(&m[2], base, e->dtype, d0, d1, nz, 4, sj, sk, sc, cfg->box_x, 4, 1, 1)))
                     return rc;
             }
             continue;

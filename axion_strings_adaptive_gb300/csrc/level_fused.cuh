@@ -5,9 +5,8 @@
 // back. This kernel keeps them on chip. A CTA owns a TX x TY tile of the xy
 // plane over a chunk of z planes and marches in z. Per plane it
 //   - runs sweep A on the tile plus a 2-cell halo (the A region) from a TMA
-//     ring of (psi, Pi) planes with a 4-cell halo,
-//   - keeps d3, d4 (A region, 6 planes) and E, Q (tile, 4 planes) in shared
-//     memory,
+//     ring of (psi, Pi) planes with a 4-cell halo, and leaves d3, d4 and (on the
+//     tile) E, Q in a window of planes in shared memory,
 //   - runs sweep B two planes behind on the tile and writes psi, Pi of the
 //     step's end to the other state buffer.
 // level_pad_kernel then writes the periodic copies of that buffer's padding
@@ -20,98 +19,85 @@
 // and out) plus the halo rows the L2 does not catch, against 28 for the two
 // sweeps; in return sweep A runs on (TX+4)(TY+4) sites per TX*TY.
 //
-// The per-site arithmetic is the two sweeps' own (lap_pair, stage_a,
+// Columns in registers. The march is bound by the shared-memory pipe, the FP32
+// pipe and issue together (76 %, 64 % and 65 % busy), not by HBM, so the work
+// per plane is kept to arithmetic. A thread owns two neighbouring sites for the
+// whole march and keeps their column, of (psi, Pi) for sweep A or (d3, d4) for
+// sweep B, in registers as the differences the z taps are made of
+// (FusedColumn): a plane takes 28 shared loads for a unit of sweep A and 36 for
+// one of sweep B, where 13 taps a Laplacian from shared memory took 44 and 52,
+// and two packed additions fewer a Laplacian. The march is unrolled by three,
+// so that the columns rotate by renaming.
+// Warps: 12 of sweep A (the tile's and the halo's units), 8 of sweep B, one
+// that issues the TMA loads. They hand planes on through four sets of
+// mbarriers (a ring slot has landed / was read, a window slot was stored / was
+// read), so sweep A runs ahead of sweep B and no warp waits for the block. 24
+// warps of 80 registers fill the register file (one CTA per SM); setmaxnreg
+// moves the producer's to the others (88 for sweep A, 96 for sweep B: at 80
+// both spilled and ran 40 % slower).
+// Measured, this kernel alone at 512^3: 1.64 ms, against 2.57 ms with all taps
+// from shared memory and a block barrier per plane; the same columns in 12
+// warps that ran both sweeps took 2.34 ms (three warps a scheduler left the
+// latencies of shared loads and additions open). Window slots: with 5 instead
+// of 4 sweep A runs two planes ahead and the step takes 6 % longer.
+//
+// The per-site arithmetic is the two sweeps' own (lap_taps, stage_a,
 // stage_b), so both paths give the same bits.
 //
-// Halo: the box is (TX+16) x (TY+8) x 1 plane x 4 components, starting 8
-// columns and 4 rows before the tile. In x the level's 8 padding columns hold
-// the periodic copies; reading 8 columns (not the 4 the stencil needs) on
-// either side makes two box rows a whole number of 128-byte lines, so each
-// piece of a split box below lands 128-byte aligned. In y the padding holds 2
-// rows: tiles in the first or last row of tiles load their 4 components as
-// three pieces each (2 rows from the wrapped edge, the TY+4 rows through the
-// padding, 2 more wrapped rows). z wraps by plane index. The corners of the
-// padding are read here: the periodic stores write them.
+// Halo: the box is (TX+8) x (TY+8) x 1 plane x 4 components, starting 4
+// columns and 4 rows before the tile. In x the level's padding columns hold
+// the periodic copies. In y the padding holds 2 rows of the 4 a box needs:
+// tiles in the first or last row of tiles load their planes as pieces that
+// skip the padding (4 wrapped rows beside TY+4 rows; pieces of 4 rows alone
+// where one row of tiles wraps at both ends). Pieces of 4 rows keep every
+// destination 128-byte aligned. z wraps by plane index. Extents that are no
+// multiple of the tile: in x the last tile column runs past the box and masks
+// its stores (it reads up to 4 padding columns; sites further right feed only
+// masked ones); in y the tile rows are spread evenly and overlap, so that
+// every tile is whole and only the first and the last touch the box's edge
+// (fused_tiles_ny). Sites that two tiles own are written twice with the same
+// bits.
 #pragma once
 
 #include "rk4_ops.cuh"
 
 namespace axs {
 
-template <int TX_, int TY_, int NS_, int THREADS_ = 512, bool COMP_ = false> struct LevelFusedShape {
+// Whether the fused step takes a box of ny rows, and its rows of tiles: one
+// tile, or evenly spread tiles of which no inner one reaches within 2 rows of
+// the padding's end (ny >= TY + 4 keeps two wrapped pieces apart).
+__host__ __device__ constexpr bool fused_takes_ny(int ny, int ty) { return ny == ty || ny >= ty + 4; }
+__host__ __device__ constexpr int fused_tiles_ny(int ny, int ty) { return (ny + ty - 1) / ty; }
+
+template <int TX_, int TY_, bool COMP_ = false> struct LevelFusedShape {
     using T = float;
     static constexpr bool COMP = COMP_;  // the compensated FP32 step (stage_a in rk4_ops.cuh)
-    static constexpr int V = 2, TX = TX_, TY = TY_, NS = NS_;
-    // sweep A units run on the first NA threads and sweep B units on the last NB:
-    // with 640 threads no thread runs both, so sweep B of one plane overlaps sweep
-    // A of the next; with 512 some threads run both every plane
-    static constexpr int THREADS = THREADS_;
-    static constexpr int BX = TX + 16, BY = TY + 8;  // TMA box: the A region, its stencil halo, alignment columns
-    static constexpr int AX = TX + 4, AY = TY + 4;   // A region
-    static constexpr int RING = 4 * BX * BY, SWIN = 4 * AX * AY, EQW = 4 * TX * TY;
-    // d3, d4 slots (sweep B reads 5 planes; one more so that sweep A of the next
-    // plane never overwrites a slot a slower thread still reads) and E, Q slots
-    // (written two planes before sweep B reads them, plus the same margin)
-    static constexpr int NSW = 6, NEQ = 4;
-    static_assert(NS >= 6 && NS <= 10 && NEQ == 4, "slot arithmetic below (wrap by one subtraction, E/Q by xor)");
-    static constexpr int NA = AX * AY / V;  // sweep A units (V sites each)
-    static constexpr int NB = TX * TY / V;  // sweep B units, one per thread of the last NB threads
-    static constexpr size_t SMEM = sizeof(T) * ((size_t)NS * RING + NSW * (size_t)SWIN + NEQ * (size_t)EQW);
+    static constexpr int V = 2, TX = TX_, TY = TY_;
+    static constexpr int U = 4;                     // window slots
+    static constexpr int NS = 8;                    // ring slots
+    static constexpr int BX = TX + 8, BY = TY + 8;  // TMA box: the A region and its stencil halo
+    static constexpr int AX = TX + 4, AY = TY + 4;  // A region
+    static constexpr int RING = 4 * BX * BY, WIN = 4 * AX * AY, EQW = 4 * TX * TY;
+    static constexpr int NT = TX * TY / V;          // units of the tile: threads of sweep B, and of sweep A
+    static constexpr int NH = 4 * (AX / V) + 2 * TY;  // halo units: 4 whole rows and 2 a tile row
+    static constexpr int WA = (NT + NH + 31) / 32, WB = NT / 32;     // warps of sweep A and of sweep B
+    static constexpr int THREADS = 32 * (WA + WB + 4);               // and the producer's warpgroup
+    static constexpr size_t SMEM = sizeof(T) * ((size_t)NS * RING + U * ((size_t)WIN + EQW));
     static constexpr uint32_t SLOT_BYTES = RING * sizeof(T);
-    static_assert(NA <= THREADS && NB <= THREADS, "at most one unit of each sweep per thread");
-    static_assert(THREADS % 32 == 0 && THREADS <= 1024, "whole warps");
-    static_assert((2 * BX * sizeof(T)) % 128 == 0 && ((TY + 6) * BX * sizeof(T)) % 128 == 0,
+    static_assert(THREADS <= 1024 && NT % 32 == 0, "whole warps of each kind");
+    static_assert((4 * BX * sizeof(T)) % 128 == 0 && ((TY + 4) * BX * sizeof(T)) % 128 == 0,
                   "the pieces of a split box land 128-byte aligned");
-    static_assert((BX * sizeof(T)) % 16 == 0, "TMA box rows of whole 16-byte units");
     static_assert((RING * sizeof(T)) % 128 == 0 && (BX * BY * sizeof(T)) % 128 == 0, "ring slots and components");
-    static_assert(AX / V > 32 / V, "the A region is wider than one bank row");
-    static_assert(BX <= 256 && BY <= 256, "TMA box extent limit");
+    static_assert(TY % 4 == 0 && BX <= 256 && BY <= 256, "pieces of 4 rows; TMA box extent limit");
+    static_assert(NS >= 5 + U - 2, "sweep A's five planes, up to U - 2 ahead of sweep B's");
     static_assert(SMEM + 1024 <= 227 * 1024, "shared memory");
+    static_assert(WA == 12 && WB == 8, "whole warpgroups and the register split of the kernel");
 };
 
-// Shared-memory accesses by 32-bit shared address plus a compile-time byte
-// offset, one instruction each.
-template <int OFF> __device__ __forceinline__ float2 lds2(uint32_t addr)
-{
-    float2 v;
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2+%3];" : "=f"(v.x), "=f"(v.y) : "r"(addr), "n"(OFF));
-    return v;
-}
-template <int OFF> __device__ __forceinline__ void sts2(uint32_t addr, float x, float y)
-{
-    asm volatile("st.shared.v2.f32 [%0+%1], {%2, %3};" ::"r"(addr), "n"(OFF), "f"(x), "f"(y) : "memory");
-}
-
-// Laplacian and centre of two sites of one component: p[d] = shared address of
-// the first site in planes z-2 .. z+2, RB the row length in bytes, CO the
-// component's byte offset. The arithmetic is lap_pair's, as in every FP32 sweep.
-template <int RB, int CO, bool COMP>
-__device__ __forceinline__ void star_pair_sh(const SweepArgs<float> &a, const uint32_t (&p)[5], float (&lap)[2],
-                                             float (&ctr)[2])
-{
-    const float2 a0 = lds2<CO - 8>(p[2]), a1 = lds2<CO>(p[2]), a2 = lds2<CO + 8>(p[2]);
-    const float r[6] = {a0.x, a0.y, a1.x, a1.y, a2.x, a2.y};
-    lap_pair<COMP>(a, r, lds2<CO - RB>(p[2]), lds2<CO + RB>(p[2]), lds2<CO - 2 * RB>(p[2]), lds2<CO + 2 * RB>(p[2]),
-                   lds2<CO>(p[1]), lds2<CO>(p[3]), lds2<CO>(p[0]), lds2<CO>(p[4]), lap[0], lap[1]);
-    ctr[0] = a1.x;
-    ctr[1] = a1.y;
-}
-
-// the same for the four components, CS bytes apart
-template <int RB, int CS, bool COMP>
-__device__ __forceinline__ void star4_sh(const SweepArgs<float> &a, const uint32_t (&p)[5], float (&lap)[4][2],
-                                         float (&ctr)[4][2])
-{
-    star_pair_sh<RB, 0 * CS, COMP>(a, p, lap[0], ctr[0]);
-    star_pair_sh<RB, 1 * CS, COMP>(a, p, lap[1], ctr[1]);
-    star_pair_sh<RB, 2 * CS, COMP>(a, p, lap[2], ctr[2]);
-    star_pair_sh<RB, 3 * CS, COMP>(a, p, lap[3], ctr[3]);
-}
-
-// The three tensor maps over one state buffer: the whole box (interior tile
-// rows), one component of TY + 4 rows, one component of 2 rows.
+// The three tensor maps over one state buffer: the whole box (inner tile
+// rows), one component of TY + 4 rows, one component of 4 rows.
 struct LevelFusedMaps {
-    CUtensorMap full, mid, rows2;
+    CUtensorMap full, mid, rows4;
 };
 
 // A work item of the fused step: a TX x TY tile over a chunk of z planes of
@@ -121,7 +107,7 @@ struct FusedItem {
     int x0, y0, z0, len;
     int nx, ny, nz;
     int64_t js, ks, base;  // base: element offset of the box in every component plane
-    const CUtensorMap *full, *mid, *rows2;
+    const CUtensorMap *full, *mid, *rows4;
 };
 
 // A block's walk over its work items (the producer thread and the consumers
@@ -130,38 +116,39 @@ struct FusedCursor {
     int64_t pos, end;
 };
 
+// First row of tile row t of `rows`: evenly spread from 0 to ny - TY.
+template <int TY> __device__ __forceinline__ int fused_tile_y0(int t, int rows, int ny)
+{
+    return rows > 1 ? t * (ny - TY) / (rows - 1) : 0;
+}
+
 // Work-item sources of the fused step: begin / valid / item / next.
 // One periodic level in (tile, z-chunk) items, taken by blocks in turn;
-// geometry from the launch parameters, nx a multiple of TX.
+// geometry from the launch parameters.
 struct FusedLevel {
-    static constexpr bool kPartialX = false;
     static constexpr bool kMapsInTable = false;  // maps by value in the launch parameters
     __device__ __forceinline__ static FusedCursor begin(const SweepArgs<float> &a) { return {blockIdx.x, a.n_items}; }
     __device__ __forceinline__ static bool valid(const FusedCursor &c) { return c.pos < c.end; }
-    __device__ __forceinline__ static void next(FusedCursor &c, int) { c.pos += gridDim.x; }
+    __device__ __forceinline__ static void next(FusedCursor &c) { c.pos += gridDim.x; }
     template <int TX, int TY>
     __device__ __forceinline__ static FusedItem item(const SweepArgs<float> &a, const LevelFusedMaps &m,
                                                      const FusedCursor &c)
     {
         const int tile = (int)(c.pos % a.ntiles);
         const int z0 = (int)(c.pos / a.ntiles) * a.zchunk;
-        return FusedItem{(tile % a.tiles_x) * TX, (tile / a.tiles_x) * TY, z0, min(a.zchunk, a.nz - z0), a.nx, a.ny,
-                         a.nz, a.js, a.ks, 0, &m.full, &m.mid, &m.rows2};
+        const int y0 = fused_tile_y0<TY>(tile / a.tiles_x, a.ntiles / a.tiles_x, a.ny);
+        return FusedItem{(tile % a.tiles_x) * TX, y0, z0, min(a.zchunk, a.nz - z0), a.nx, a.ny, a.nz, a.js, a.ks, 0,
+                         &m.full, &m.mid, &m.rows4};
     }
 };
 // The boxes of an ensemble: the item list and box descriptors of a box table,
-// and per box six tensor maps in the table (full, mid, rows2 over each of the
-// two state buffers; map_sel picks the buffer read). ny is a multiple of TY.
-// The last tile column of a box whose width is not a multiple of TX runs past
-// the box: its stores are masked. Its sweep A sites up to nx + 1 read the
-// padding copies (8 columns) and feed the last valid sites; the ones further
-// right read zero-filled or unused columns and feed only masked sites.
+// and per box six tensor maps in the table (full, mid, rows4 over each of the
+// two state buffers; map_sel picks the buffer read).
 struct FusedBoxes {
-    static constexpr bool kPartialX = true;
     static constexpr bool kMapsInTable = true;  // written by a host copy: acquired before use
     __device__ __forceinline__ static FusedCursor begin(const SweepArgs<float> &a) { return {blockIdx.x, a.n_items}; }
     __device__ __forceinline__ static bool valid(const FusedCursor &c) { return c.pos < c.end; }
-    __device__ __forceinline__ static void next(FusedCursor &c, int) { c.pos += gridDim.x; }
+    __device__ __forceinline__ static void next(FusedCursor &c) { c.pos += gridDim.x; }
     template <int TX, int TY>
     __device__ __forceinline__ static FusedItem item(const SweepArgs<float> &a, const LevelFusedMaps &,
                                                      const FusedCursor &c)
@@ -171,242 +158,362 @@ struct FusedBoxes {
         const int local = (int)(e & ((1u << kEnsItemBits) - 1));
         const int tile = local % d.ntiles;
         const int z0 = (local / d.ntiles) * d.zchunk;
+        const int y0 = fused_tile_y0<TY>(tile / d.tiles_x, d.ntiles / d.tiles_x, d.ny);
         const CUtensorMap *m = a.maps + 3 * (2 * d.map_box + a.map_sel);
-        return FusedItem{(tile % d.tiles_x) * TX, (tile / d.tiles_x) * TY, z0, min(d.zchunk, d.nz - z0), d.nx, d.ny,
-                         d.nz, d.js, d.ks, d.base, m, m + 1, m + 2};
+        return FusedItem{(tile % d.tiles_x) * TX, y0, z0, min(d.zchunk, d.nz - z0), d.nx, d.ny, d.nz, d.js, d.ks,
+                         d.base, m, m + 1, m + 2};
     }
 };
+
+__device__ __forceinline__ float2 lds2(const unsigned char *p) { return *reinterpret_cast<const float2 *>(p); }
+
+// A thread's column of four components through the march, as the differences
+// the stencil is made of: f(z+1) - f(z) serves z and, negated, z+1; f(z+2) - f(z)
+// serves z and z+2. Step: the plane z+2 comes in as `f[P + 2]`; the z sums of
+// plane z are handed out and the column moves on. P, the step modulo 3, makes
+// the indices constants.
+struct FusedColumn {
+    F2 f[3][4];   // planes z, z+1, z+2
+    F2 u1[4];     // f(z) - f(z-1)
+    F2 u2[3][4];  // f(z+1) - f(z-1), f(z) - f(z-2); the third: room for f(z+2) - f(z)
+    template <int P> __device__ __forceinline__ const F2 &mid(int c) const { return f[P % 3][c]; }
+    template <int P> __device__ __forceinline__ F2 &in(int c) { return f[(P + 2) % 3][c]; }
+    template <int P> __device__ __forceinline__ void sums(int c, F2 &z1, F2 &z2)
+    {
+        const F2 d1 = f[(P + 1) % 3][c] - f[P % 3][c], d2 = f[(P + 2) % 3][c] - f[P % 3][c];
+        z1 = d1 - u1[c];
+        z2 = d2 - u2[P % 3][c];  // u2[P % 3]: f(z) - f(z-2), of the step before last
+        u1[c] = d1;
+        u2[(P + 2) % 3][c] = d2;
+    }
+};
+
+// Laplacians of a thread's two sites of the four components: xy taps from a
+// plane in shared memory (p: the first site, component 0; RB the row length and
+// CB the component stride in bytes), centre and z sums from the column.
+template <int P, int RB, int CB, bool COMP>
+__device__ __forceinline__ void star4_column(const SweepArgs<float> &a, const unsigned char *p, FusedColumn &col,
+                                             F2 (&lap)[4])
+{
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const unsigned char *q = p + c * CB;
+        F2 z1, z2;
+        col.sums<P>(c, z1, z2);
+        lap[c] = lap_taps<COMP>(a, lds2(q - 8), col.mid<P>(c).v, lds2(q + 8), lds2(q - RB), lds2(q + RB),
+                                lds2(q - 2 * RB), lds2(q + 2 * RB), z1, z2);
+    }
+}
 
 template <class S, class Src = FusedLevel>
 __global__ void __launch_bounds__(S::THREADS, 1)
     level_fused_kernel(const __grid_constant__ LevelFusedMaps maps, const SweepArgs<float> a)
 {
-    using T = float;
-    constexpr int V = S::V, TX = S::TX, TY = S::TY, NS = S::NS, BX = S::BX, BY = S::BY, AX = S::AX, AY = S::AY;
+    constexpr int V = S::V, TX = S::TX, TY = S::TY, NS = S::NS, U = S::U, BX = S::BX, BY = S::BY, AX = S::AX,
+                  AY = S::AY;
+    constexpr int SLOT = (int)S::SLOT_BYTES, WSLOT = S::WIN * 4, ESLOT = S::EQW * 4;
+    // row and component strides in a ring slot, a (d3, d4) window slot and an (E, Q) window slot, bytes
+    constexpr int RB = BX * 4, RC = BX * BY * 4, WB = AX * 4, WC = AX * AY * 4, EC = TX * TY * 4;
     extern __shared__ __align__(128) unsigned char lf_smem[];
-    T *ring = reinterpret_cast<T *>(lf_smem);
-    T *swin = ring + (size_t)NS * S::RING;
-    T *eqw = swin + (size_t)S::NSW * S::SWIN;
-    __shared__ uint64_t full[NS];
-    const int tid = threadIdx.x;
+    unsigned char *const win = lf_smem + (size_t)NS * SLOT, *const eqw = win + (size_t)U * WSLOT;
+    // ring slots: landed, and read (by sweep B, last); window slots: stored, and read
+    __shared__ uint64_t bars[2 * NS + 2 * U];
+    __shared__ int failed;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const bool lane0 = (tid & 31) == 0;
     constexpr int oy = 2;  // padded row of y = 0 in the level layout
 
     if (tid == 0) {
-        for (int s = 0; s < NS; ++s) mbar_init(&full[s], 1);
+        for (int k = 0; k < NS; ++k) {
+            mbar_init(&bars[k], 1);
+            mbar_init(&bars[NS + k], S::WB);
+        }
+        for (int k = 0; k < U; ++k) {
+            mbar_init(&bars[2 * NS + k], S::WA);
+            mbar_init(&bars[2 * NS + U + k], S::WB);
+        }
         fence_mbar_init();
-        prefetch_tensormap(&maps.full);
-        prefetch_tensormap(&maps.mid);
-        prefetch_tensormap(&maps.rows2);
+        failed = 0;
     }
     __syncthreads();
 
-    // ---- producer cursor (thread 0 only): planes z0 - 4 .. z0 + len + 3 of each item
-    FusedCursor p_cur = Src::begin(a);
-    int p_k = 0;
-    FusedItem p{};
-    bool p_edge = false;
-    auto p_start = [&]() {
-        if (!Src::valid(p_cur)) return;
-        p = Src::template item<TX, TY>(a, maps, p_cur);
-        p_edge = p.y0 == 0 || p.y0 + TY == p.ny;  // rows y0 - 4, y0 - 3 or y0 + TY + 2, + 3 lie past the padding
-        if constexpr (Src::kMapsInTable) {
-            fence_tensormap_acquire(p.full);
-            fence_tensormap_acquire(p.mid);
-            fence_tensormap_acquire(p.rows2);
+    // A wait is a test whose answer is looked at a step later, and a bounded wait
+    // where it said no: the latency of a wait at its point of use would lie on the
+    // warp's path. An expired wait ends the block: every other wait sees `failed`.
+    uint32_t bar0 = smem_addr(bars);
+    asm volatile("" : "+r"(bar0));  // kept, not recomputed
+    auto landed = [&](int k) { return bar0 + 8u * k; };
+    auto ring_read = [&](int k) { return bar0 + 8u * (NS + k); };
+    auto stored = [&](int k) { return bar0 + 8u * (2 * NS + k); };
+    auto win_read = [&](int k) { return bar0 + 8u * (2 * NS + U + k); };
+    auto slow_wait = [&](uint32_t bar, uint32_t phase) -> bool {
+        for (uint32_t it = 0; it < a.wait_polls; ++it) {
+            if (mbar_try_wait_at(bar, phase)) return true;
+            if ((it & 63) == 63 && *(volatile int *)&failed) return false;
         }
+        if (*(volatile int *)&failed) return false;
+        atomicOr(a.status, kDevTimeout);
+        *(volatile int *)&failed = 1;
+        return false;
     };
-    int64_t q_issued = 0;
-    int p_slot = 0;  // ring slot of plane q_issued
-    auto issue_one = [&]() -> bool {
-        if (!Src::valid(p_cur)) return false;
-        int zp = (p.z0 - 4 + p_k) % p.nz;
-        if (zp < 0) zp += p.nz;
-        const int slot = p_slot;
-        if (++p_slot == NS) p_slot = 0;
-        T *dst = ring + (size_t)slot * S::RING;
-        mbar_arrive_expect_tx(&full[slot], S::SLOT_BYTES);
-        const int xc = a.ox - 8 + p.x0;  // padded column of the box's first column (16-byte aligned)
-        if (!p_edge) {
-            tma_load_4d(dst, p.full, xc, p.y0 - 4 + oy, zp, 0, &full[slot]);
+    auto ended = [&]() { return __any_sync(0xffffffffu, *(volatile int *)&failed != 0) != 0; };
+
+    if (warp >= S::WA + S::WB) {
+        // registers: 24 warps x 80 at launch = 12 x 88 + 8 x 96 + 4 x 24
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+        // ---- producer: planes z0 - 4 .. z0 + len + 3 of each item, one after the other
+        if (tid != 32 * (S::WA + S::WB)) return;
+        prefetch_tensormap(&maps.full);
+        prefetch_tensormap(&maps.mid);
+        prefetch_tensormap(&maps.rows4);
+        int slot = 0;
+        int64_t sent = 0;
+        uint32_t phase = 1;  // of ring_read: the first round of slots is free
+        bool ok = true;
+        for (FusedCursor cur = Src::begin(a); ok && Src::valid(cur); Src::next(cur)) {
+            const FusedItem p = Src::template item<TX, TY>(a, maps, cur);
+            if constexpr (Src::kMapsInTable) {
+                fence_tensormap_acquire(p.full);
+                fence_tensormap_acquire(p.mid);
+                fence_tensormap_acquire(p.rows4);
+            }
+            int zp = p.z0 - 4;  // nz may be smaller than 4
+            while (zp < 0) zp += p.nz;
+            const int xc = a.ox - 4 + p.x0;  // padded column of the box's first column (16-byte aligned)
+            const bool lo = p.y0 == 0, hi = p.y0 + TY == p.ny;
+            for (int k = 0; k < p.len + 8; ++k) {
+                if (!(ok = slow_wait(ring_read(slot), phase))) break;
+                unsigned char *dst = lf_smem + (size_t)slot * SLOT;
+                uint64_t *bar = &bars[slot];
+                mbar_arrive_expect_tx(bar, S::SLOT_BYTES);
+                ++sent;
+                if (!lo && !hi) {
+                    tma_load_4d(dst, p.full, xc, p.y0 - 4 + oy, zp, 0, bar);
+                } else if (lo && hi) {
+                    for (int c = 0; c < 4; ++c)
+                        for (int r = 0; r < BY; r += 4)
+                            tma_load_4d(dst + c * RC + r * RB, p.rows4, xc, (r + TY - 4) % TY + oy, zp, c, bar);
+                } else {
+                    // rows y0 - 4 .. y0 + TY + 3 as 4 wrapped rows below the others (first tile row) or above them
+                    const int r4 = lo ? 0 : TY + 4, y4 = lo ? p.ny - 4 : 0, rm = lo ? 4 : 0, ym = lo ? 0 : p.y0 - 4;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        tma_load_4d(dst + c * RC + r4 * RB, p.rows4, xc, y4 + oy, zp, c, bar);
+                        tma_load_4d(dst + c * RC + rm * RB, p.mid, xc, ym + oy, zp, c, bar);
+                    }
+                }
+                if (++zp == p.nz) zp = 0;
+                if (++slot == NS) {
+                    slot = 0;
+                    phase ^= 1;
+                }
+            }
+        }
+        // No bulk copy may still be landing in shared memory when the block ends
+        // (after an expired wait; bounded as well).
+        for (int64_t v = sent > NS ? sent - NS : 0; v < sent; ++v)
+            mbar_wait_bounded(&bars[v % NS], (uint32_t)((v / NS) & 1), 1u << 20);
+        return;
+    }
+
+    // March of an item. Planes are numbered from z0 - 4. Step i = 0 .. len + 3: sweep A
+    // at plane i + 2 = z0 - 2 + i, with plane i + 4 new in the column; sweep B at plane
+    // i = z0 - 4 + i, from i = 4 on, with d3, d4 of step i new in its column.
+    auto need = [&](bool ready, uint32_t bar, uint32_t phase) {
+        if (__any_sync(0xffffffffu, !ready)) slow_wait(bar, phase);
+    };
+    if (warp < S::WA) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
+        // ---- sweep A. Units: the tile's, 16 pairs to a row; 16 pairs of each of the
+        // halo's four rows; then groups of 8, four rows' pairs at the left and right
+        // end, and the rest of the four halo rows (idle lanes of the last warp repeat
+        // that group and store nothing). Half a warp reads whole bank rows, and a
+        // group's 8 pairs lie in different banks of a ring plane (rows 40 words
+        // apart); halo units in row order took 180 more wavefronts of 1670 a plane.
+        static_assert(TX == 32 && TY % 4 == 0, "16 pairs to a row, groups of four rows");
+        const bool tile_site = tid < S::NT;
+        const int h = tid - S::NT;
+        const bool has_a = h < S::NH;
+        int alx, aly;  // A-region-local first site
+        if (tile_site) {
+            alx = 2 + V * (tid % 16);
+            aly = 2 + tid / 16;
+        } else if (h < 64) {
+            alx = V * (h % 16);
+            aly = h / 16 < 2 ? h / 16 : TY + h / 16;
         } else {
-            const int rt = ((p.y0 - 4) % p.ny + p.ny) % p.ny + oy;  // rows y0 - 4, y0 - 3 (wrapped)
-            const int rb = (p.y0 + TY + 2) % p.ny + oy;            // rows y0 + TY + 2, + 3 (wrapped)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                T *dc = dst + (size_t)c * BX * BY;
-                tma_load_4d(dc, p.rows2, xc, rt, zp, c, &full[slot]);
-                tma_load_4d(dc + 2 * BX, p.mid, xc, p.y0 - 2 + oy, zp, c, &full[slot]);
-                tma_load_4d(dc + (TY + 6) * BX, p.rows2, xc, rb, zp, c, &full[slot]);
-            }
+            const int g = min((h - 64) / 8, TY / 4), row = h & 3, right = (h >> 2) & 1;
+            alx = right ? AX - 2 : g < TY / 4 ? 0 : AX - 4;
+            aly = g < TY / 4 ? 2 + 4 * g + row : row < 2 ? row : TY + row;
         }
-        ++q_issued;
-        if (++p_k == p.len + 8) {
-            p_k = 0;
-            Src::next(p_cur, p.len);
-            p_start();
-        }
-        return true;
-    };
-    if (tid == 0) {
-        p_start();
-        for (int s = 0; s < NS; ++s)
-            if (!issue_one()) break;
-    }
-
-    // sweep B unit of this thread (bt < 0: none), tile-local sites (bxl, byl) .. (bxl + V - 1, byl)
-    const int bt = tid - (S::THREADS - S::NB);
-    const bool has_b = bt >= 0;
-    const int bxl = has_b ? V * (bt % (TX / V)) : 0, byl = has_b ? bt / (TX / V) : 0;
-    // sweep A unit of this thread: units of the A region's first 32 / V columns row by
-    // row (a warp covers whole 128-byte bank rows: conflict-free), then the others
-    const bool has_a = tid < S::NA;
-    int alx = 0, aly = 0;  // A-region-local first site
-    {
-        constexpr int PR = AX / V, MAIN = 32 / V, EDGE = PR - MAIN;
-        const int u = tid;
-        const int row = u < MAIN * AY ? u / MAIN : (u - MAIN * AY) / EDGE;
-        const int col = u < MAIN * AY ? u % MAIN : MAIN + (u - MAIN * AY) % EDGE;
-        alx = V * col;
-        aly = row;
-    }
-    const int atx = alx - 2, aty = aly - 2;  // tile-local (V sites lie all inside or all outside the tile)
-    const bool a_in_tile = atx >= 0 && atx < TX && aty >= 0 && aty < TY;
-    // shared addresses of the three regions and this thread's byte offsets in them
-    const uint32_t ring_sh = smem_addr(ring), swin_sh = smem_addr(swin), eqw_sh = smem_addr(eqw);
-    const uint32_t a_at = 4u * (uint32_t)((aly + 2) * BX + (alx + 6));      // A site in the ring box
-    const uint32_t a_so = 4u * (uint32_t)(aly * AX + alx);                  // A site in the d3, d4 window
-    const uint32_t a_eo = 4u * (uint32_t)(a_in_tile ? aty * TX + atx : 0);  // A site in the E, Q window
-    const uint32_t b_ro = 4u * (uint32_t)((byl + 4) * BX + (bxl + 8));     // B site in the ring box
-    const uint32_t b_so = 4u * (uint32_t)((byl + 2) * AX + (bxl + 2));     // B site in the d3, d4 window
-    const uint32_t b_eo = 4u * (uint32_t)(byl * TX + bxl);                 // B site in the E, Q window
-
-    // Ring slots, their mbarrier phases and the window slots advance by one per
-    // plane: rotating small counters (a modulo by the slot count per plane and
-    // thread is a real cost in this issue-bound loop).
-    int r0 = 0;                   // ring slot of plane q_base + i (the oldest plane sweep A reads)
-    int w_slot = 0, w_phase = 0;  // the next plane to wait for: its slot and mbarrier parity
-    int s0 = 0, e0 = 0;           // d3, d4 slot and E, Q slot of sweep A's plane
-    int64_t q_waited = 0;
-    bool aborted = false;
-    for (FusedCursor cur = Src::begin(a); Src::valid(cur);) {
-        const FusedItem w = Src::template item<TX, TY>(a, maps, cur);
-        const int z0 = w.z0, len = w.len;
-        // this thread's sweep B sites: element offset of their row at z = 0, and
-        // whether they lie in the box
-        const int64_t b_row = w.base + (int64_t)(w.x0 + bxl + a.ox) + (int64_t)(w.y0 + byl + oy) * w.js;
-        const bool b_in = !Src::kPartialX || w.x0 + bxl < w.nx;
-        // iteration i: sweep A at plane za = z0 - 2 + i (ring planes q_base + i .. + 4),
-        // sweep B at zb = za - 2 = z0 - 4 + i for i >= 4
-        for (int i = 0; i < len + 4; ++i) {
-            // planes up to q_base + i + 4 must have landed: the first iteration of an
-            // item waits for five, every later one for one more
-            bool late = false;  // this thread's wait expired
-            for (int need = i == 0 ? 5 : 1; need > 0; --need) {
-                if (!mbar_wait_bounded(&full[w_slot], (uint32_t)w_phase, a.wait_polls)) {
-                    atomicOr(a.status, kDevTimeout);
-                    late = true;
-                }
-                ++q_waited;
-                if (++w_slot == NS) {
-                    w_slot = 0;
-                    w_phase ^= 1;
-                }
+        const int site = 4 * ((aly + 2) * BX + alx + 2);
+        unsigned char *const wsite = win + 4 * (aly * AX + alx), *const esite = eqw + 8 * tid;
+        int slot = 0, off_new = site, off_mid;  // ring slot of plane i + 4; this site in it and in plane i + 2's
+        int ws = 0;                             // window slot of step i
+        uint32_t landed_phase = 0, read_phase = 1;  // of slot's next landing; of win_read (the first round is free)
+        auto next_off = [&](int &off) {
+            off += SLOT;
+            if (off >= NS * SLOT) off -= NS * SLOT;
+        };
+        auto take_plane = [&](bool ready) {
+            need(ready, landed(slot), landed_phase);
+            if (++slot == NS) {
+                slot = 0;
+                landed_phase ^= 1;
             }
-            uint32_t pl[5];  // shared addresses of ring planes q_base + i .. + 4
+        };
+        FusedColumn col;
+        for (FusedCursor cur = Src::begin(a); Src::valid(cur); Src::next(cur)) {
+            const int n = Src::template item<TX, TY>(a, maps, cur).len + 4;
+            {
+                F2 first[4][4];
 #pragma unroll
-            for (int d = 0; d < 5; ++d) {
-                const int sd = r0 + d < NS ? r0 + d : r0 + d - NS;
-                pl[d] = ring_sh + (uint32_t)sd * (uint32_t)(S::RING * 4);
-            }
-            if (has_a) {
-                uint32_t pa[5];
+                for (int k = 0; k < 4; ++k) {
+                    take_plane(false);
+                    if (k == 2) off_mid = off_new;
 #pragma unroll
-                for (int d = 0; d < 5; ++d) pa[d] = pl[d] + a_at;
-                T lap[4][V], ctr[4][V];
-                star4_sh<BX * 4, BX * BY * 4, S::COMP>(a, pa, lap, ctr);
-                T o[8][V];
-                stage_a<T, V, S::COMP>(a, lap, ctr, o);
-                const uint32_t sz = swin_sh + (uint32_t)s0 * (uint32_t)(S::SWIN * 4) + a_so;  // d3, d4 of plane za
-                sts2<0 * AX * AY * 4>(sz, o[0][0], o[0][1]);
-                sts2<1 * AX * AY * 4>(sz, o[1][0], o[1][1]);
-                sts2<2 * AX * AY * 4>(sz, o[2][0], o[2][1]);
-                sts2<3 * AX * AY * 4>(sz, o[3][0], o[3][1]);
-                if (a_in_tile) {
-                    const uint32_t ez = eqw_sh + (uint32_t)e0 * (uint32_t)(S::EQW * 4) + a_eo;  // E, Q of plane za
-                    sts2<0 * TX * TY * 4>(ez, o[4][0], o[4][1]);
-                    sts2<1 * TX * TY * 4>(ez, o[5][0], o[5][1]);
-                    sts2<2 * TX * TY * 4>(ez, o[6][0], o[6][1]);
-                    sts2<3 * TX * TY * 4>(ez, o[7][0], o[7][1]);
+                    for (int c = 0; c < 4; ++c) first[k][c] = F2(lds2(lf_smem + off_new + c * RC));
+                    next_off(off_new);
                 }
-            }
-            // sweep B's psi_n, Pi_n at plane zb: ring plane q_base + i, refilled after the barrier
-            float2 pn[4];
-            if (has_b && i >= 4) {
-                const uint32_t r0p = pl[0] + b_ro;
-                pn[0] = lds2<0 * BX * BY * 4>(r0p);
-                pn[1] = lds2<1 * BX * BY * 4>(r0p);
-                pn[2] = lds2<2 * BX * BY * 4>(r0p);
-                pn[3] = lds2<3 * BX * BY * 4>(r0p);
-            }
-            // d3, d4, E, Q of plane za are in place; ring plane q_base + i is read no
-            // more. The barrier also ORs the threads' expired waits: a thread whose
-            // wait expired ran its sweeps on a slot that may still be landing, and
-            // the block drops those results here, before any global store (one
-            // block-wide flag in shared memory, read three times a plane, cost
-            // 1.4 % of the step).
-            if (__syncthreads_or(late)) {
-                aborted = true;
-                break;
-            }
-            if (tid == 0) {
-                // the oldest plane still needed: q_base + i + 1, or the next item's first
-                const int64_t next_needed = q_waited - 4 + (i + 1 < len + 4 ? 0 : 4);
-                fence_proxy_async_smem();
-                while (q_issued < next_needed + NS && issue_one()) {
-                }
-            }
-            if (has_b && i >= 4) {
-                const int zb = z0 - 4 + i;
-                const int b0 = s0 + 2 < S::NSW ? s0 + 2 : s0 + 2 - S::NSW;  // slot of plane za - 4 = zb - 2
-                uint32_t sp[5];
-#pragma unroll
-                for (int d = 0; d < 5; ++d) {
-                    const int sd = b0 + d < S::NSW ? b0 + d : b0 + d - S::NSW;
-                    sp[d] = swin_sh + (uint32_t)sd * (uint32_t)(S::SWIN * 4) + b_so;
-                }
-                const uint32_t ez = eqw_sh + (uint32_t)(e0 ^ 2) * (uint32_t)(S::EQW * 4) + b_eo;  // E, Q of plane zb
-                T lap[4][V], ctr[4][V], o[4][V], pq[8][V];
-                star4_sh<AX * 4, AX * AY * 4, S::COMP>(a, sp, lap, ctr);
-                const float2 e[4] = {lds2<0 * TX * TY * 4>(ez), lds2<1 * TX * TY * 4>(ez), lds2<2 * TX * TY * 4>(ez),
-                                     lds2<3 * TX * TY * 4>(ez)};
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    pq[c][0] = e[c].x;
-                    pq[c][1] = e[c].y;
-                    pq[4 + c][0] = pn[c].x;
-                    pq[4 + c][1] = pn[c].y;
-                }
-                stage_b<T, V, decltype(pq), S::COMP>(a, lap, ctr, pq, o);
-                const int64_t off = b_row + (int64_t)zb * w.ks;
-                if (b_in) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) stv<T, V>(a.out[c] + off, o[c]);
+                    col.f[0][c] = first[2][c];
+                    col.f[1][c] = first[3][c];
+                    col.u1[c] = first[2][c] - first[1][c];
+                    col.u2[1][c] = first[3][c] - first[1][c];
+                    col.u2[0][c] = first[2][c] - first[0][c];
                 }
             }
-            if (++r0 == NS) r0 = 0;
-            if (++s0 == S::NSW) s0 = 0;
-            e0 = (e0 + 1) & (S::NEQ - 1);
+            bool ready = false;
+            auto step = [&](auto ph) {
+                constexpr int P = decltype(ph)::value;
+                take_plane(ready);
+                ready = mbar_test_at(landed(slot), landed_phase);
+                const bool free = mbar_test_at(win_read(ws), read_phase);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) col.in<P>(c) = F2(lds2(lf_smem + off_new + c * RC));
+                next_off(off_new);
+                F2 lap[4];
+                star4_column<P, RB, RC, S::COMP>(a, lf_smem + off_mid, col, lap);
+                next_off(off_mid);
+                const StageAPair sa = stage_a_pair<S::COMP>(a, col.mid<P>(0), col.mid<P>(1), col.mid<P>(2),
+                                                            col.mid<P>(3), lap[0], lap[1], lap[2], lap[3]);
+                need(free, win_read(ws), read_phase);
+                unsigned char *const wz = wsite + ws * WSLOT, *const ez = esite + ws * ESLOT;
+                if (has_a) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) *reinterpret_cast<float2 *>(wz + c * WC) = sa.d[c].v;
+                }
+                if (tile_site) {
+                    F2 eq[4];
+                    stage_a_eq<S::COMP>(a, sa, lap[0], lap[1], eq);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) *reinterpret_cast<float2 *>(ez + c * EC) = eq[c].v;
+                }
+                __syncwarp();
+                if (lane0) mbar_arrive_at(stored(ws));
+                if (++ws == U) {
+                    ws = 0;
+                    read_phase ^= 1;
+                }
+            };
+            for (int i = 0;;) {
+                step(std::integral_constant<int, 0>{});
+                if (++i == n) break;
+                step(std::integral_constant<int, 1>{});
+                if (++i == n) break;
+                step(std::integral_constant<int, 2>{});
+                if (++i == n || ended()) break;
+            }
+            if (ended()) return;
         }
-        if (aborted) break;
-        // the next item's window starts 4 planes past this item's last window start + 1
-        r0 += 4;
-        if (r0 >= NS) r0 -= NS;
-        Src::next(cur, len);
-    }
-    // A wait expired: make sure no bulk copy is still landing in shared memory
-    // before the block exits (bounded as well).
-    if (aborted && tid == 0) {
-        for (int64_t q = q_waited; q < q_issued; ++q) mbar_wait_bounded(&full[q % NS], (uint32_t)((q / NS) & 1), 1u << 20);
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
+        // ---- sweep B, a unit of the tile to a thread
+        const int bt = tid - 32 * S::WA;
+        const int bx = V * (bt % (TX / V)), by = bt / (TX / V);  // tile-local first site
+        const unsigned char *const wsite = win + 4 * ((by + 2) * AX + bx + 2), *const esite = eqw + 8 * bt;
+        int slot = 0, off_y = 4 * ((by + 4) * BX + bx + 4);  // ring slot of plane i, this site in it
+        int ws = 0, wm = 0;                                  // window slots of steps i and i - 2
+        uint32_t stored_phase = 0, landed_phase = 0;
+        auto release_plane = [&]() {  // after the warp's reads of it
+            if (lane0) mbar_arrive_at(ring_read(slot));
+            off_y += SLOT;
+            if (++slot == NS) {
+                slot = 0;
+                off_y -= NS * SLOT;
+                landed_phase ^= 1;
+            }
+        };
+        auto release_window = [&]() {
+            if (lane0) mbar_arrive_at(win_read(wm));
+            if (++wm == U) wm = 0;
+        };
+        FusedColumn col;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            for (int k = 0; k < 3; ++k) col.f[k][c] = col.u2[k][c] = F2(0.f);
+            col.u1[c] = F2(0.f);
+        }
+        for (FusedCursor cur = Src::begin(a); Src::valid(cur); Src::next(cur)) {
+            const FusedItem w = Src::template item<TX, TY>(a, maps, cur);
+            const bool in_box = w.x0 + bx < w.nx;
+            int64_t off = w.base + (int64_t)(w.x0 + bx + a.ox) + (int64_t)(w.y0 + by + oy) * w.js + (int64_t)w.z0 * w.ks;
+            const int n = w.len + 4;
+            bool ready = false;
+            auto step = [&](auto ph, int i) {
+                constexpr int P = decltype(ph)::value;
+                need(ready, stored(ws), stored_phase);
+                const unsigned char *const wz = wsite + ws * WSLOT;
+                if (++ws == U) {
+                    ws = 0;
+                    stored_phase ^= 1;
+                }
+                ready = mbar_test_at(stored(ws), stored_phase);
+                const bool here = mbar_test_at(landed(slot), landed_phase);  // long since: sweep A has read the plane
+#pragma unroll
+                for (int c = 0; c < 4; ++c) col.in<P>(c) = F2(lds2(wz + c * WC));
+                if (i >= 4) {
+                    // (E, Q) of plane i with its d3, d4, stored at step i - 2, and its psi_n, Pi_n
+                    need(here, landed(slot), landed_phase);
+                    F2 lap[4], e[4], y[4], o[4];
+                    star4_column<P, WB, WC, S::COMP>(a, wsite + wm * WSLOT, col, lap);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        e[c] = F2(lds2(esite + wm * ESLOT + c * EC));
+                        y[c] = F2(lds2(lf_smem + off_y + c * RC));
+                    }
+                    stage_b_pair<S::COMP>(a, col.mid<P>(0), col.mid<P>(1), col.mid<P>(2), col.mid<P>(3), lap, e, y, o);
+                    if (in_box) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) *reinterpret_cast<float2 *>(a.out[c] + off) = o[c].v;
+                    }
+                    off += w.ks;
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        F2 z1, z2;
+                        col.sums<P>(c, z1, z2);
+                    }
+                }
+                __syncwarp();
+                release_plane();
+                if (i >= 2) release_window();
+            };
+            for (int i = 0;;) {
+                step(std::integral_constant<int, 0>{}, i);
+                if (++i == n) break;
+                step(std::integral_constant<int, 1>{}, i);
+                if (++i == n) break;
+                step(std::integral_constant<int, 2>{}, i);
+                if (++i == n || ended()) break;
+            }
+            if (ended()) return;
+            // the item's last planes: sweep A is done with them, and nothing reads the last two window slots
+            for (int k = 0; k < 4; ++k) release_plane();
+            release_window();
+            release_window();
+        }
     }
 }
 
@@ -442,7 +549,9 @@ __device__ __forceinline__ void pad_box(T *__restrict__ buf, int nx, int ny, int
                     x = rr - k * nx;
                     y = k < 2 ? k - 2 : ny + (k - 2);
                 }
-                const int xs = x < 0 ? x + nx : (x >= nx ? x - nx : x), ys = y < 0 ? y + ny : (y >= ny ? y - ny : y);
+                int xs = x < 0 ? x + nx : (x >= nx ? x - nx : x);
+                xs = xs < 0 ? xs + nx : (xs >= nx ? xs - nx : xs);  // 8 columns may wrap twice: nx is at least 4
+                const int ys = y < 0 ? y + ny : (y >= ny ? y - ny : y);
                 on[u] = r < per_plane;
                 dst[u] = x + (int64_t)y * js;
                 src[u] = on[u] ? xs + (int64_t)ys * js : 0;

@@ -160,19 +160,21 @@ struct SweepConfig {
     }
 };
 
-// The one-pass fused step (level_fused.cuh) over FP32 levels whose extents are
-// multiples of its tile; single sweeps and other extents run the two sweeps of
-// the fastest two-sweep tiling. Steps alternate between the level's state and
+// The one-pass fused step (level_fused.cuh) over FP32 levels whose row count
+// its tiles take; single sweeps and other levels run the two sweeps of the
+// fastest two-sweep tiling. Steps alternate between the level's state and
 // the first 4 component planes of its work buffer (same layout); each step is
 // the fused launch and the padding launch. An odd step count runs its first
 // step as the two sweeps, which step the state in place.
-template <int TX, int TY, int NS, int THREADS = 512, bool COMP = false> struct FusedConfig {
-    using S = LevelFusedShape<TX, TY, NS, THREADS, COMP>;
+template <int TX, int TY, bool COMP = false> struct FusedConfig {
+    using S = LevelFusedShape<TX, TY, COMP>;
     using Fallback = SweepConfig<float, 2, 32, 8, 8, 3, true, COMP>;  // the fastest two-sweep tiling at 512^3
 
+    // nx >= 8: narrower levels keep the two sweeps, which leave the outer 4 of
+    // their 8 padding columns alone
     static bool applies(const axs_level *lv)
     {
-        return lv->dtype == AXS_F32 && lv->nx % TX == 0 && lv->ny % TY == 0;
+        return lv->dtype == AXS_F32 && lv->nx >= 8 && fused_takes_ny(lv->ny, TY);
     }
 
     static int maps_for(LevelFusedMaps &m, const float *base, const LevelGeom &g, int ny, int nz)
@@ -184,8 +186,8 @@ template <int TX, int TY, int NS, int THREADS = 512, bool COMP = false> struct F
         if ((rc = make_tensor_map_4d(&m.mid, base, AXS_F32, g.js, ny + 4, nz, 4, g.js * es, g.ks * es, g.cs * es,
                                      S::BX, TY + 4, 1, 1)))
             return rc;
-        return make_tensor_map_4d(&m.rows2, base, AXS_F32, g.js, ny + 4, nz, 4, g.js * es, g.ks * es, g.cs * es,
-                                  S::BX, 2, 1, 1);
+        return make_tensor_map_4d(&m.rows4, base, AXS_F32, g.js, ny + 4, nz, 4, g.js * es, g.ks * es, g.cs * es,
+                                  S::BX, 4, 1, 1);
     }
 
     static int run(const SweepRunArgs &r)
@@ -219,8 +221,8 @@ template <int TX, int TY, int NS, int THREADS = 512, bool COMP = false> struct F
         a.nx = lv->nx;
         a.ny = lv->ny;
         a.nz = lv->nz;
-        a.tiles_x = lv->nx / TX;
-        a.ntiles = a.tiles_x * (lv->ny / TY);
+        a.tiles_x = (lv->nx + TX - 1) / TX;
+        a.ntiles = a.tiles_x * fused_tiles_ny(lv->ny, TY);
         // (tile, z-chunk) items taken by blocks in turn: the blocks running at
         // one time march neighbouring tiles through the same planes, so the
         // halo rows they share are L2 hits. (One contiguous tile-major range per
@@ -267,7 +269,7 @@ struct TileConfigEntry {
 
 static const TileConfigEntry kF32Configs[] = {
     // the default: the fastest FP32 step at 512^3 (two sweeps where it does not apply)
-    {"f32 fused 32x16 ring6 t640", &FusedConfig<32, 16, 6, 640>::run, &FusedConfig<32, 16, 6, 640, true>::run},
+    {"f32 fused 32x16 columns", &FusedConfig<32, 16>::run, &FusedConfig<32, 16, true>::run},
     {"f32 v2 64x8 ring8", &SweepConfig<float, 2, 64, 8, 8, 2>::run, nullptr},
     {"f32 v2 32x16 ring8", &SweepConfig<float, 2, 32, 16, 8, 2>::run, nullptr},
     {"f32 v4 32x16 ring8", &SweepConfig<float, 4, 32, 16, 8, 2>::run, nullptr},
@@ -283,10 +285,11 @@ static const TileConfigEntry kF32Configs[] = {
     {"f32 v2 32x8 ring8 l2", &SweepConfig<float, 2, 32, 8, 8, 3, true>::run,
      &SweepConfig<float, 2, 32, 8, 8, 3, true, true>::run},
     {"f32 v4 64x16 ring6 l2", &SweepConfig<float, 4, 64, 16, 6, 1, true>::run, nullptr},
-    // one-pass fused step (level_fused.cuh)
-    {"f32 fused 32x16 ring6", &FusedConfig<32, 16, 6>::run, nullptr},
-    {"f32 fused 32x16 ring7", &FusedConfig<32, 16, 7>::run, nullptr},
-    {"f32 fused 32x16 ring7 t640", &FusedConfig<32, 16, 7, 640>::run, nullptr},
+    // earlier names of the one-pass fused step
+    {"f32 fused 32x16 ring6 t640", &FusedConfig<32, 16>::run, &FusedConfig<32, 16, true>::run},
+    {"f32 fused 32x16 ring6", &FusedConfig<32, 16>::run, nullptr},
+    {"f32 fused 32x16 ring7", &FusedConfig<32, 16>::run, nullptr},
+    {"f32 fused 32x16 ring7 t640", &FusedConfig<32, 16>::run, nullptr},
 };
 static const TileConfigEntry kF64Configs[] = {
     {"f64 v1 32x8 ring6", &SweepConfig<double, 1, 32, 8, 6, 2>::run, nullptr},

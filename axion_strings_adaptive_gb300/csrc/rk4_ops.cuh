@@ -7,6 +7,67 @@
 
 namespace axs {
 
+// Two sites of sweep A with packed FP32 (the arithmetic of stage_a below): the
+// increments d3, d4 with what E and Q are made of, and E, Q themselves, apart
+// because the halo sites of the one-pass step need d3, d4 only.
+struct StageAPair {
+    F2 d[4];                // d3_1, d3_2, d4_1, d4_2
+    F2 f11, f12, f21, f22;  // F1, F2
+    F2 hq1, hq2;            // h Pi
+};
+template <bool COMP>
+__device__ __forceinline__ StageAPair stage_a_pair(const SweepArgs<float> &a, F2 p1, F2 p2, F2 q1, F2 q2, F2 l0, F2 l1,
+                                                   F2 l2, F2 l3)
+{
+    StageAPair s;
+    const F2 hh(a.h_half);
+    rhs_pair(a.c1, p1, p2, l0, l1, s.f11, s.f12);
+    if constexpr (!COMP) {
+        const F2 c1 = fma(hh, q1, p1), c2 = fma(hh, q2, p2);
+        rhs_pair(a.c2, c1, c2, fma(hh, l2, l0), fma(hh, l3, l1), s.f21, s.f22);
+        s.hq1 = F2(a.h) * q1;
+        s.hq2 = F2(a.h) * q2;
+        s.d[0] = fma(F2(a.h2_quarter), s.f11, hh * q1);
+        s.d[1] = fma(F2(a.h2_quarter), s.f12, hh * q2);
+        s.d[2] = fma(F2(a.h2_half), s.f21, s.hq1);
+        s.d[3] = fma(F2(a.h2_half), s.f22, s.hq2);
+    } else {
+        auto cm = [](F2 c, F2 cl, F2 x, F2 y) { return fma(cl, x, fma(c, x, y)); };  // (c + c_lo) x + y
+        const F2 hhl(a.h_half_lo), z(0.f, 0.f);
+        const F2 c1 = cm(hh, hhl, q1, p1), c2 = cm(hh, hhl, q2, p2);
+        rhs_pair(a.c2, c1, c2, cm(hh, hhl, l2, l0), cm(hh, hhl, l3, l1), s.f21, s.f22);
+        s.hq1 = cm(F2(a.h), F2(a.h_lo), q1, z);
+        s.hq2 = cm(F2(a.h), F2(a.h_lo), q2, z);
+        const F2 hhq1 = cm(hh, hhl, q1, z), hhq2 = cm(hh, hhl, q2, z);
+        const F2 H2Q(a.h2_quarter), H2Ql(a.h2_quarter_lo), H2H(a.h2_half), H2Hl(a.h2_half_lo);
+        s.d[0] = cm(H2Q, H2Ql, s.f11, hhq1);
+        s.d[1] = cm(H2Q, H2Ql, s.f12, hhq2);
+        s.d[2] = cm(H2H, H2Hl, s.f21, s.hq1);
+        s.d[3] = cm(H2H, H2Hl, s.f22, s.hq2);
+    }
+    return s;
+}
+template <bool COMP>
+__device__ __forceinline__ void stage_a_eq(const SweepArgs<float> &a, const StageAPair &s, F2 l0, F2 l1, F2 (&eq)[4])
+{
+    const F2 hh(a.h_half);
+    if constexpr (!COMP) {
+        eq[0] = fma(F2(a.h2_sixth), (s.f11 + s.f21) + l0, s.hq1);
+        eq[1] = fma(F2(a.h2_sixth), (s.f12 + s.f22) + l1, s.hq2);
+        eq[2] = fma(hh, l0, fma(F2(a.h_third), s.f21, F2(a.h_sixth) * s.f11));
+        eq[3] = fma(hh, l1, fma(F2(a.h_third), s.f22, F2(a.h_sixth) * s.f12));
+    } else {
+        auto cm = [](F2 c, F2 cl, F2 x, F2 y) { return fma(cl, x, fma(c, x, y)); };
+        const F2 hhl(a.h_half_lo), z(0.f, 0.f);
+        const F2 H26(a.h2_sixth), H26l(a.h2_sixth_lo), H3(a.h_third), H3l(a.h_third_lo);
+        const F2 H6(a.h_sixth), H6l(a.h_sixth_lo);
+        eq[0] = cm(H26, H26l, (s.f11 + s.f21) + l0, s.hq1);
+        eq[1] = cm(H26, H26l, (s.f12 + s.f22) + l1, s.hq2);
+        eq[2] = cm(hh, hhl, l0, cm(H3, H3l, s.f21, cm(H6, H6l, s.f11, z)));
+        eq[3] = cm(hh, hhl, l1, cm(H3, H3l, s.f22, cm(H6, H6l, s.f12, z)));
+    }
+}
+
 // Stage arithmetic of sweep A on V sites: from the Laplacians and centre
 // values of (psi1, psi2, Pi1, Pi2) to the increments
 //   o = (d3_1, d3_2, d4_1, d4_2, E_1, E_2, Q_1, Q_2),
@@ -31,48 +92,14 @@ __device__ __forceinline__ void stage_a(const SweepArgs<T> &a, const T (&lap)[4]
                                         T (&o)[8][V])
 {
     if constexpr (kPackedPairs<T, V>) {
-        // the expressions below, two sites per instruction
 #pragma unroll
         for (int v = 0; v < V; v += 2) {
-            const F2 p1(ctr[0][v], ctr[0][v + 1]), p2(ctr[1][v], ctr[1][v + 1]);
-            const F2 q1(ctr[2][v], ctr[2][v + 1]), q2(ctr[3][v], ctr[3][v + 1]);
-            const F2 l0(lap[0][v], lap[0][v + 1]), l1(lap[1][v], lap[1][v + 1]);
-            const F2 l2(lap[2][v], lap[2][v + 1]), l3(lap[3][v], lap[3][v + 1]);
-            const F2 hh(a.h_half);
-            F2 f11, f12, f21, f22;
-            F2 r[8];
-            rhs_pair(a.c1, p1, p2, l0, l1, f11, f12);
-            if constexpr (!COMP) {
-                const F2 c1 = fma(hh, q1, p1), c2 = fma(hh, q2, p2);
-                rhs_pair(a.c2, c1, c2, fma(hh, l2, l0), fma(hh, l3, l1), f21, f22);
-                const F2 hq1 = F2(a.h) * q1, hq2 = F2(a.h) * q2;
-                r[0] = fma(F2(a.h2_quarter), f11, hh * q1);
-                r[1] = fma(F2(a.h2_quarter), f12, hh * q2);
-                r[2] = fma(F2(a.h2_half), f21, hq1);
-                r[3] = fma(F2(a.h2_half), f22, hq2);
-                r[4] = fma(F2(a.h2_sixth), (f11 + f21) + l0, hq1);
-                r[5] = fma(F2(a.h2_sixth), (f12 + f22) + l1, hq2);
-                r[6] = fma(hh, l0, fma(F2(a.h_third), f21, F2(a.h_sixth) * f11));
-                r[7] = fma(hh, l1, fma(F2(a.h_third), f22, F2(a.h_sixth) * f12));
-            } else {
-                auto cm = [](F2 c, F2 cl, F2 x, F2 y) { return fma(cl, x, fma(c, x, y)); };  // (c + c_lo) x + y
-                const F2 hhl(a.h_half_lo), z(0.f, 0.f);
-                const F2 c1 = cm(hh, hhl, q1, p1), c2 = cm(hh, hhl, q2, p2);
-                rhs_pair(a.c2, c1, c2, cm(hh, hhl, l2, l0), cm(hh, hhl, l3, l1), f21, f22);
-                const F2 hq1 = cm(F2(a.h), F2(a.h_lo), q1, z), hq2 = cm(F2(a.h), F2(a.h_lo), q2, z);
-                const F2 hhq1 = cm(hh, hhl, q1, z), hhq2 = cm(hh, hhl, q2, z);
-                const F2 H2Q(a.h2_quarter), H2Ql(a.h2_quarter_lo), H2H(a.h2_half), H2Hl(a.h2_half_lo);
-                const F2 H26(a.h2_sixth), H26l(a.h2_sixth_lo), H3(a.h_third), H3l(a.h_third_lo);
-                const F2 H6(a.h_sixth), H6l(a.h_sixth_lo);
-                r[0] = cm(H2Q, H2Ql, f11, hhq1);
-                r[1] = cm(H2Q, H2Ql, f12, hhq2);
-                r[2] = cm(H2H, H2Hl, f21, hq1);
-                r[3] = cm(H2H, H2Hl, f22, hq2);
-                r[4] = cm(H26, H26l, (f11 + f21) + l0, hq1);
-                r[5] = cm(H26, H26l, (f12 + f22) + l1, hq2);
-                r[6] = cm(hh, hhl, l0, cm(H3, H3l, f21, cm(H6, H6l, f11, z)));
-                r[7] = cm(hh, hhl, l1, cm(H3, H3l, f22, cm(H6, H6l, f12, z)));
-            }
+            auto pr = [&](const T (&x)[V]) { return F2(x[v], x[v + 1]); };
+            const StageAPair s = stage_a_pair<COMP>(a, pr(ctr[0]), pr(ctr[1]), pr(ctr[2]), pr(ctr[3]), pr(lap[0]),
+                                                    pr(lap[1]), pr(lap[2]), pr(lap[3]));
+            F2 eq[4];
+            stage_a_eq<COMP>(a, s, pr(lap[0]), pr(lap[1]), eq);
+            const F2 r[8] = {s.d[0], s.d[1], s.d[2], s.d[3], eq[0], eq[1], eq[2], eq[3]};
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 o[c][v] = r[c].v.x;
@@ -102,6 +129,31 @@ __device__ __forceinline__ void stage_a(const SweepArgs<T> &a, const T (&lap)[4]
     }
 }
 
+// Two sites of sweep B with packed FP32 (the arithmetic of stage_b below): d =
+// (d3_1, d3_2, d4_1, d4_2) and their Laplacians, e = (E, Q), y = (psi_n, Pi_n).
+template <bool COMP>
+__device__ __forceinline__ void stage_b_pair(const SweepArgs<float> &a, F2 d0, F2 d1, F2 d2, F2 d3, const F2 (&lap)[4],
+                                             const F2 (&e)[4], const F2 (&y)[4], F2 (&o)[4])
+{
+    F2 g31, g32, g41, g42;
+    rhs_pair(a.c2, y[0] + d0, y[1] + d1, lap[0], lap[1], g31, g32);
+    rhs_pair(a.c4, y[0] + d2, y[1] + d3, lap[2], lap[3], g41, g42);
+    if constexpr (!COMP) {
+        o[0] = y[0] + fma(F2(a.h2_sixth), g31, e[0]);
+        o[1] = y[1] + fma(F2(a.h2_sixth), g32, e[1]);
+        o[2] = y[2] + fma(F2(a.h_sixth), g41, fma(F2(a.h_third), g31, e[2]));
+        o[3] = y[3] + fma(F2(a.h_sixth), g42, fma(F2(a.h_third), g32, e[3]));
+    } else {
+        auto cm = [](F2 c, F2 cl, F2 x, F2 y) { return fma(cl, x, fma(c, x, y)); };
+        const F2 H26(a.h2_sixth), H26l(a.h2_sixth_lo), H3(a.h_third), H3l(a.h_third_lo);
+        const F2 H6(a.h_sixth), H6l(a.h_sixth_lo);
+        o[0] = y[0] + cm(H26, H26l, g31, e[0]);
+        o[1] = y[1] + cm(H26, H26l, g32, e[1]);
+        o[2] = y[2] + cm(H6, H6l, g41, cm(H3, H3l, g31, e[2]));
+        o[3] = y[3] + cm(H6, H6l, g42, cm(H3, H3l, g32, e[3]));
+    }
+}
+
 // Stage arithmetic of sweep B on V sites: from the Laplacians and centre
 // values of (d3_1, d3_2, d4_1, d4_2) and the pointwise
 // pq = (E_1, E_2, Q_1, Q_2, psi1, psi2, Pi1, Pi2) of the step's start to
@@ -113,29 +165,14 @@ __device__ __forceinline__ void stage_b(const SweepArgs<T> &a, const T (&lap)[4]
                                         const PQ &pq, T (&o)[4][V])
 {
     if constexpr (kPackedPairs<T, V>) {
-        // the expressions below, two sites per instruction
 #pragma unroll
         for (int v = 0; v < V; v += 2) {
             auto pr = [&](const T (&x)[V]) { return F2(x[v], x[v + 1]); };
-            const F2 p1 = pr(pq[4]), p2 = pr(pq[5]);
-            F2 g31, g32, g41, g42;
-            rhs_pair(a.c2, p1 + pr(ctr[0]), p2 + pr(ctr[1]), pr(lap[0]), pr(lap[1]), g31, g32);
-            rhs_pair(a.c4, p1 + pr(ctr[2]), p2 + pr(ctr[3]), pr(lap[2]), pr(lap[3]), g41, g42);
+            const F2 l[4] = {pr(lap[0]), pr(lap[1]), pr(lap[2]), pr(lap[3])};
+            const F2 e[4] = {pr(pq[0]), pr(pq[1]), pr(pq[2]), pr(pq[3])};
+            const F2 y[4] = {pr(pq[4]), pr(pq[5]), pr(pq[6]), pr(pq[7])};
             F2 r[4];
-            if constexpr (!COMP) {
-                r[0] = p1 + fma(F2(a.h2_sixth), g31, pr(pq[0]));
-                r[1] = p2 + fma(F2(a.h2_sixth), g32, pr(pq[1]));
-                r[2] = pr(pq[6]) + fma(F2(a.h_sixth), g41, fma(F2(a.h_third), g31, pr(pq[2])));
-                r[3] = pr(pq[7]) + fma(F2(a.h_sixth), g42, fma(F2(a.h_third), g32, pr(pq[3])));
-            } else {
-                auto cm = [](F2 c, F2 cl, F2 x, F2 y) { return fma(cl, x, fma(c, x, y)); };
-                const F2 H26(a.h2_sixth), H26l(a.h2_sixth_lo), H3(a.h_third), H3l(a.h_third_lo);
-                const F2 H6(a.h_sixth), H6l(a.h_sixth_lo);
-                r[0] = p1 + cm(H26, H26l, g31, pr(pq[0]));
-                r[1] = p2 + cm(H26, H26l, g32, pr(pq[1]));
-                r[2] = pr(pq[6]) + cm(H6, H6l, g41, cm(H3, H3l, g31, pr(pq[2])));
-                r[3] = pr(pq[7]) + cm(H6, H6l, g42, cm(H3, H3l, g32, pr(pq[3])));
-            }
+            stage_b_pair<COMP>(a, pr(ctr[0]), pr(ctr[1]), pr(ctr[2]), pr(ctr[3]), l, e, y, r);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 o[c][v] = r[c].v.x;

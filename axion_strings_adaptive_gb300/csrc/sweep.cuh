@@ -220,28 +220,41 @@ __device__ __forceinline__ void rhs_adjoint_pair(const StageCoef<T> &c, T u1, T 
     o2 = fma(k, a2, la2) - ua * u2;
 }
 
-// The FP32 Laplacian of two neighbouring sites x, x+1 from their neighbours:
-// r[0..5] = f(x-2 .. x+3) along the row, and the y / z neighbour pairs. The
-// stencil as differences from the centre, lap = wA sum(f+-1 - f0) + wB
-// sum(f+-2 - f0): a neighbour within a factor 2 of f0 gives an exact
-// difference, so the -30 f0 term of the plain sum does not cancel against the
-// neighbours. f - f0 is formed as f + (-f0), the same IEEE result. Every FP32
-// sweep evaluates its stencils through this function. COMP (the compensated
-// FP32 step) adds the weights' FP32 remainders times d1, d2: FP32 rounds 16/3
-// and -1/3 in the same direction for every site, a bias that the plain form
-// carries into every step.
+// The FP32 Laplacian of two neighbouring sites x, x+1 from their taps: xl =
+// f(x-2, x-1), f0 = f(x, x+1), xr = f(x+2, x+3) along the row, the y neighbour
+// pairs, and the z neighbours' sums z1 = sum(f+-1 - f0), z2 = sum(f+-2 - f0). The stencil as differences from the centre, lap = wA
+// sum(f+-1 - f0) + wB sum(f+-2 - f0): a neighbour within a factor 2 of f0 gives
+// an exact difference, so the -30 f0 term of the plain sum does not cancel
+// against the neighbours. f - f0 is formed as f + (-f0), the same IEEE result.
+// Every FP32 sweep evaluates its stencils through this function. The x+-1 taps
+// go site by site: their pairs straddle the register pairs the packed
+// instructions need, and f(x+1) - f(x) serves both sites (negated, exactly).
+// COMP (the compensated FP32 step) adds the weights' FP32 remainders times d1,
+// d2: FP32 rounds 16/3 and -1/3 in the same direction for every site, a bias
+// that the plain form carries into every step.
+template <bool COMP = false>
+__device__ __forceinline__ F2 lap_taps(const SweepArgs<float> &a, float2 xl, float2 f0, float2 xr, float2 ym1,
+                                       float2 yp1, float2 ym2, float2 yp2, F2 z1, F2 z2)
+{
+    const F2 m0(-f0.x, -f0.y);
+    const float dx = f0.y - f0.x;
+    const F2 x1((xl.y - f0.x) + dx, (xr.x - f0.y) - dx);
+    const F2 d1 = (x1 + ((F2(ym1) + m0) + (F2(yp1) + m0))) + z1;
+    const F2 d2 = ((F2(xl) + m0) + (F2(xr) + m0)) + ((F2(ym2) + m0) + (F2(yp2) + m0)) + z2;
+    F2 l = fma(F2(a.wA), d1, F2(a.wB) * d2);
+    if constexpr (COMP) l = fma(F2(a.wA_lo), d1, fma(F2(a.wB_lo), d2, l));  // the weights' FP32 remainders
+    return l;
+}
+
+// the same with the row's taps r[0..5] = f(x-2 .. x+3) in an array and the z taps as they are
 template <bool COMP = false>
 __device__ __forceinline__ void lap_pair(const SweepArgs<float> &a, const float *r, float2 ym1, float2 yp1,
                                          float2 ym2, float2 yp2, float2 zm1, float2 zp1, float2 zm2, float2 zp2,
                                          float &l0, float &l1)
 {
     const F2 m0(-r[2], -r[3]);
-    const F2 d1 = ((F2(r[1], r[2]) + m0) + (F2(r[3], r[4]) + m0)) + ((F2(ym1) + m0) + (F2(yp1) + m0)) +
-                  ((F2(zm1) + m0) + (F2(zp1) + m0));
-    const F2 d2 = ((F2(r[0], r[1]) + m0) + (F2(r[4], r[5]) + m0)) + ((F2(ym2) + m0) + (F2(yp2) + m0)) +
-                  ((F2(zm2) + m0) + (F2(zp2) + m0));
-    F2 l = fma(F2(a.wA), d1, F2(a.wB) * d2);
-    if constexpr (COMP) l = fma(F2(a.wA_lo), d1, fma(F2(a.wB_lo), d2, l));  // the weights' FP32 remainders
+    const F2 l = lap_taps<COMP>(a, make_float2(r[0], r[1]), make_float2(r[2], r[3]), make_float2(r[4], r[5]), ym1,
+                                yp1, ym2, yp2, (F2(zm1) + m0) + (F2(zp1) + m0), (F2(zm2) + m0) + (F2(zp2) + m0));
     l0 = l.v.x;
     l1 = l.v.y;
 }

@@ -198,3 +198,26 @@ def test_compensated_fp32_step_vs_oracle_fp64(axs, orc):
     lv.advance(bg, 1.0, 0.0, dt, steps)
     lv.device_status()
     assert _rel_max(lv.get_state().double().cpu().numpy(), ref64) < 1e-5
+
+
+# extents around the fused tile (32 x 16): the smallest levels, a partial last tile
+# column, one row of tiles (wraps at both ends), tile rows that overlap by almost a
+# tile and by one row, row counts just below what the fused step takes, nz below the
+# stencil, and z-chunks of uneven length
+@pytest.mark.parametrize("shape", [(4, 16, 1), (8, 20, 2), (28, 16, 3), (36, 21, 5), (32, 19, 4), (60, 17, 6), (100, 33, 7),
+                                   (68, 31, 9), (132, 47, 61), (64, 128, 33)])
+@pytest.mark.parametrize("comp", [False, True], ids=["plain", "compensated"])
+def test_fused_step_at_the_edges_of_its_tiles(axs, shape, comp):
+    v = _state(shape, 3 * sum(shape)).cuda()
+    bg = axs.Background.expanding(1.5, 1.0, lambda0=2.0)
+    out = []
+    for name in ("f32 v2 32x8 ring8 l2", "f32 fused 32x16 columns"):
+        lv = axs.PeriodicLevel(shape, 0.5, dtype=torch.float32)
+        lv.tile_config = _config_id(lv, name)
+        lv.compensated = comp
+        lv.set_state(v)
+        lv.advance(bg, 1.0, 0.0, 0.1, 4)
+        lv.device_status()
+        out.append(lv.state)
+    # both the valid cells and the periodic padding and corners
+    assert torch.equal(out[0], out[1])
