@@ -199,12 +199,15 @@ __global__ void sum_partials_kernel(const double *__restrict__ part, int n, doub
 
 // ----------------------------------------------------------------------------
 // Adjoint tiling: one configuration per dtype (V = 1 keeps the 12 pointwise
-// components of sweep A in registers without spilling).
+// components of sweep A in registers without spilling; FP64 takes smaller
+// blocks, as the forward sweeps do, within kAdjMaxGridPerSm).
 constexpr int kAdjMaxGridPerSm = 4;
 
 template <typename T> struct AdjointRunner {
-    using LB = SweepLauncher<T, 1, 32, 8, 8, 2, AdjointB>;
-    using LA = SweepLauncher<T, 1, 32, 8, 8, 2, AdjointA>;
+    static constexpr bool kF64 = std::is_same<T, double>::value;
+    static constexpr int TY = kF64 ? 4 : 8, NS = kF64 ? 7 : 8, MINB = kF64 ? 3 : 2;
+    using LB = SweepLauncher<T, 1, 32, TY, NS, MINB, AdjointB>;
+    using LA = SweepLauncher<T, 1, 32, TY, NS, MINB, AdjointA>;
 
     static int run(const axs_level *lv, const LevelGeom &g, T *abar, T *adj, double *lam_part, int lam_slots,
                    const axs_background &bg, double tau_i, double t, double dt, double *lam_acc, cudaStream_t st)

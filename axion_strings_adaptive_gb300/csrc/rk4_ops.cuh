@@ -244,6 +244,8 @@ template <typename T> inline void fill_step_constants(SweepArgs<T> &a, double dx
     a.wA = T((4.0 / 3.0) * inv_dx2);
     a.wB = T((-1.0 / 12.0) * inv_dx2);
     a.wC = T(-7.5 * inv_dx2);
+    // lap_site scales wT by powers of two within 2^+-554
+    a.wT = T(inv_dx2 > 0x1p-400 && inv_dx2 < 0x1p400 ? inv_dx2 / 12.0 : 0.0);
     a.h = T(dt);
     a.h_half = T(0.5 * dt);
     a.h2_quarter = T(0.25 * dt * dt);

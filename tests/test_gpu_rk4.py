@@ -248,3 +248,50 @@ def test_eval_rhs_f32_wide_staging_equals_cell_staging(axs, shape):
         out.append(axs.valid(r, 0).clone())
     torch.cuda.synchronize()
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("kind", ["plain", "zeros", "wide", "edge28", "tiny", "large", "subnormal", "nonfinite"])
+def test_f64_step_on_fields_of_every_exponent_range(axs, orc, kind):
+    """One FP64 level step, whose Laplacians are summed as integers where every
+    tap's exponent lies within 28 of the largest, against the stage-by-stage
+    oracle: fields with exact zeros, exponents far apart, on both sides of the
+    28, near the ends of the double range, and infinities and NaN (the same
+    cells are finite). Tolerance: 1e-12 of the component's maximum, as for the
+    other FP64 steps (13 taps of weight up to 30 in ulp of 2^-53, times
+    h^2/dx^2 < 1)."""
+    nx, ny, nz = shape = (24, 10, 9)
+    rng = np.random.default_rng(11)
+    v = rng.standard_normal((4, nz, ny, nx))
+    if kind == "zeros":
+        v[:, :, :, ::3] = 0.0
+        v[3] = 0.0
+    elif kind == "wide":
+        v = np.ldexp(v, rng.integers(-70, 1, v.shape))
+    elif kind == "edge28":
+        v = np.ldexp(np.sign(v) * rng.uniform(1.0, 2.0, v.shape), -rng.integers(26, 31, v.shape) * (rng.random(v.shape) < 0.2))
+    elif kind == "tiny":
+        v *= 1e-160
+    elif kind == "large":
+        v *= 1e40
+    elif kind == "subnormal":
+        v *= 1e-308
+    elif kind == "nonfinite":
+        v[0, 2, 3, 4], v[1, 6, 7, 15], v[2, 4, 1, 20] = np.nan, np.inf, -np.inf
+    dx, dt = 0.5, 0.05
+    lam = 2.0 if kind != "large" else 1e-80
+    bg, bgo = axs.Background.expanding(2.0, 1.0, lambda0=lam), orc.background(a_inv=2.0, c0=1.0, lambda_scale=lam)
+    ref = orc.to_fab(v, 2)
+    with np.errstate(all="ignore"):
+        orc.rk4_advance(ref, 2, dx, bgo, 1.0, 0.0, dt, 1)
+    ref = orc.from_fab(ref, 2)
+    for cid, name in [(0, "default")] + axs.PeriodicLevel(shape, dx, dtype=torch.float64).tile_configs():
+        lv = axs.PeriodicLevel(shape, dx, dtype=torch.float64, tile_config=cid)
+        lv.set_state(_to_dev(v))
+        lv.advance(bg, 1.0, 0.0, dt, 1)
+        lv.device_status()
+        got = lv.get_state().cpu().numpy()
+        fin = np.isfinite(ref)
+        np.testing.assert_array_equal(np.isfinite(got), fin, err_msg=name)
+        for c in range(4):
+            scale = max(np.abs(ref[c][fin[c]]).max(), 1e-307)
+            assert np.abs(got[c] - ref[c])[fin[c]].max() <= 1e-12 * scale, (name, c)
