@@ -523,16 +523,18 @@ __global__ void __launch_bounds__(S::THREADS, 1)
 // rows are planes (z + nz c); within a plane, consecutive threads take
 // consecutive elements of a padding row, and each thread copies kPadUnroll
 // elements a grid-row stride apart, all loads before the stores (sources are
-// valid cells, destinations padding: no copy reads another's destination).
+// valid cells of `from`, destinations padding: no copy reads another's destination).
 constexpr int kPadUnroll = 4;
 template <typename T>
-__device__ __forceinline__ void pad_box(T *__restrict__ buf, int nx, int ny, int nz, int64_t js, int64_t ks, int64_t cs,
-                                        int ox, int oy)
+__device__ __forceinline__ void pad_box(T *buf, const T *from, int nx, int ny, int nz, int64_t js, int64_t ks,
+                                        int64_t cs, int ox, int oy)
 {
     const int xpad = 16 * (ny + 4), per_plane = xpad + 4 * nx;
     const int stride = gridDim.x * blockDim.x;
     for (int plane = blockIdx.y; plane < 4 * nz; plane += gridDim.y) {
-        T *p = buf + (int64_t)(plane / nz) * cs + (int64_t)(plane % nz) * ks + ox + (int64_t)oy * js;
+        const int64_t at = (int64_t)(plane / nz) * cs + (int64_t)(plane % nz) * ks + ox + (int64_t)oy * js;
+        T *p = buf + at;
+        const T *s = from + at;
         for (int r0 = blockIdx.x * blockDim.x + threadIdx.x; r0 < per_plane; r0 += kPadUnroll * stride) {
             int64_t dst[kPadUnroll], src[kPadUnroll];
             bool on[kPadUnroll];
@@ -558,7 +560,7 @@ __device__ __forceinline__ void pad_box(T *__restrict__ buf, int nx, int ny, int
             }
             T v[kPadUnroll];
 #pragma unroll
-            for (int u = 0; u < kPadUnroll; ++u) v[u] = p[src[u]];
+            for (int u = 0; u < kPadUnroll; ++u) v[u] = s[src[u]];
 #pragma unroll
             for (int u = 0; u < kPadUnroll; ++u)
                 if (on[u]) p[dst[u]] = v[u];
@@ -570,7 +572,45 @@ template <typename T>
 __global__ void level_pad_kernel(T *__restrict__ buf, int nx, int ny, int nz, int64_t js, int64_t ks, int64_t cs,
                                  int ox, int oy)
 {
-    pad_box(buf, nx, ny, nz, js, ks, cs, ox, oy);
+    pad_box(buf, buf, nx, ny, nz, js, ks, cs, ox, oy);
+}
+
+// The valid cells of a level-layout buffer with their periodic padding, from
+// another buffer's valid cells: the end of a run of an odd number of fused
+// steps, which leaves the result in the second buffer. Grid rows are planes;
+// within a plane the first nx ny / 4 tasks copy four cells each, the others
+// write the padding (pad_box, sources in src).
+template <typename T>
+__device__ __forceinline__ void copy_pad_box(T *__restrict__ dst, const T *__restrict__ src, int nx, int ny, int nz,
+                                             int64_t js, int64_t ks, int64_t cs, int ox, int oy)
+{
+    using V4 = typename VecN<T, 4>::type;
+    const int quads = nx / 4, units = quads * ny;
+    for (int plane = blockIdx.y; plane < 4 * nz; plane += gridDim.y) {
+        const int64_t at = (int64_t)(plane / nz) * cs + (int64_t)(plane % nz) * ks + ox + (int64_t)oy * js;
+        const int stride = gridDim.x * blockDim.x;
+        for (int r0 = blockIdx.x * blockDim.x + threadIdx.x; r0 < units; r0 += kPadUnroll * stride) {
+            V4 v[kPadUnroll];
+            int64_t o[kPadUnroll];
+#pragma unroll
+            for (int u = 0; u < kPadUnroll; ++u) {
+                const int r = min(r0 + u * stride, units - 1), y = r / quads;
+                o[u] = at + 4 * (r - y * quads) + (int64_t)y * js;
+                v[u] = *reinterpret_cast<const V4 *>(src + o[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < kPadUnroll; ++u)
+                if (r0 + u * stride < units) *reinterpret_cast<V4 *>(dst + o[u]) = v[u];
+        }
+    }
+    pad_box(dst, src, nx, ny, nz, js, ks, cs, ox, oy);
+}
+
+template <typename T>
+__global__ void level_copy_pad_kernel(T *__restrict__ dst, const T *__restrict__ src, int nx, int ny, int nz, int64_t js,
+                                      int64_t ks, int64_t cs, int ox, int oy)
+{
+    copy_pad_box(dst, src, nx, ny, nz, js, ks, cs, ox, oy);
 }
 
 // The same for every box of an ensemble buffer, one box per blockIdx.z.
@@ -578,7 +618,7 @@ template <typename T>
 __global__ void ens_pad_kernel(T *__restrict__ buf, const EnsBoxDesc *__restrict__ boxes, int64_t cs, int ox)
 {
     const EnsBoxDesc &d = boxes[blockIdx.z];
-    pad_box(buf + d.base, d.nx, d.ny, d.nz, d.js, d.ks, cs, ox, d.oy);
+    pad_box(buf + d.base, buf + d.base, d.nx, d.ny, d.nz, d.js, d.ks, cs, ox, d.oy);
 }
 
 }  // namespace axs

@@ -164,8 +164,9 @@ struct SweepConfig {
 // its tiles take; single sweeps and other levels run the two sweeps of the
 // fastest two-sweep tiling. Steps alternate between the level's state and
 // the first 4 component planes of its work buffer (same layout); each step is
-// the fused launch and the padding launch. An odd step count runs its first
-// step as the two sweeps, which step the state in place.
+// the fused launch and the padding launch. After an odd step count the last
+// step's padding launch brings the result back to the state as well: 341 us for
+// one step at 256^3, where the two sweeps in place took 391.
 template <int TX, int TY, bool COMP = false> struct FusedConfig {
     using S = LevelFusedShape<TX, TY, COMP>;
     using Fallback = SweepConfig<float, 2, 32, 8, 8, 3, true, COMP>;  // the fastest two-sweep tiling at 512^3
@@ -194,20 +195,6 @@ template <int TX, int TY, bool COMP = false> struct FusedConfig {
     {
         const axs_level *lv = r.lv;
         if (r.sweep_mask != 3 || !applies(lv)) return Fallback::run(r);
-        // An odd step count takes its first step as the two sweeps (in place; the
-        // results are the same bits), so the fused steps after it come in pairs
-        // and end in the state buffer. A step into another buffer is one fused
-        // launch from the state.
-        if ((r.nsteps & 1) && r.out_state == nullptr) {
-            SweepRunArgs one = r;
-            one.nsteps = 1;
-            const int rc1 = Fallback::run(one);
-            if (rc1 || r.nsteps == 1) return rc1;
-            SweepRunArgs rest = r;
-            rest.t0 = r.t0 + r.dt;
-            rest.nsteps = r.nsteps - 1;
-            return run(rest);
-        }
         const LevelGeom &g = *r.g;
         static int smem_set = 0;
         auto kern = level_fused_kernel<S, FusedLevel>;
@@ -250,6 +237,13 @@ template <int TX, int TY, bool COMP = false> struct FusedConfig {
             for (int c = 0; c < 4; ++c) as.out[c] = dst + c * g.cs;
             kern<<<grid, S::THREADS, S::SMEM, r.st>>>(maps[s & 1], as);
             if ((rc = launch_status("fused level step"))) return rc;
+            if (s + 1 == r.nsteps && (r.nsteps & 1) && r.out_state == nullptr) {
+                const int units = lv->nx / 4 * lv->ny;
+                const dim3 copy_grid((unsigned)std::max(1, std::min(64, units / (256 * kPadUnroll))), pad_grid.y);
+                level_copy_pad_kernel<float><<<copy_grid, 256, 0, r.st>>>(buf[0], dst, lv->nx, lv->ny, lv->nz, g.js,
+                                                                          g.ks, g.cs, g.ox, g.oy);
+                return launch_status("level copy");
+            }
             level_pad_kernel<float><<<pad_grid, 256, 0, r.st>>>(dst, lv->nx, lv->ny, lv->nz, g.js, g.ks, g.cs, g.ox, g.oy);
             if ((rc = launch_status("level padding"))) return rc;
         }
