@@ -81,11 +81,16 @@ class _StringCoreLoss(torch.autograd.Function):
         level = PeriodicLevel((nx, ny, nz), spec.dx, dtype=state0.dtype, device=state0.device, pierced_capacity=1)
         level.set_state(state0.detach())
         k = max(1, int(spec.checkpoint_every))
-        checkpoints = []
+        # Steps go from buffer to buffer (one fused launch each, where a step in place
+        # takes the two sweeps), so a checkpoint is a buffer kept, not a copy.
+        checkpoints, spare = [], None
         for s in range(spec.nsteps):
+            dst = torch.empty_like(level.state) if spare is None else spare
+            level.step_to(dst, bg, spec.tau_i, s * spec.dt, spec.dt)
+            spare = level.swap_state(dst)
             if s % k == 0:
-                checkpoints.append(level.state.clone())
-            level.advance(bg, spec.tau_i, s * spec.dt, spec.dt, 1)
+                checkpoints.append(spare)
+                spare = None
         buf = AdjointBuffers(level)
         tau_f = spec.tau_i + spec.nsteps * spec.dt
         loss = loss_and_seed(level, buf, bg.values(tau_f).R, spec.width)
@@ -103,11 +108,12 @@ class _StringCoreLoss(torch.autograd.Function):
             s0 = seg * k
             s1 = min(spec.nsteps, s0 + k)
             # re-run the segment forward, keeping the state at the start of each step
-            level.state.copy_(ctx.checkpoints[seg])
-            states = []
-            for s in range(s0, s1):
-                states.append(level.state.clone())
-                level.advance(bg, spec.tau_i, s * spec.dt, spec.dt, 1)
+            # (the last step's end is not needed)
+            states = [ctx.checkpoints[seg]]
+            for s in range(s0, s1 - 1):
+                states.append(torch.empty_like(states[0]))
+                level.swap_state(states[-2])
+                level.step_to(states[-1], bg, spec.tau_i, s * spec.dt, spec.dt)
             for s in reversed(range(s0, s1)):
                 adjoint_step(level, states[s - s0], buf, bg, spec.tau_i, s * spec.dt, spec.dt)
             del states
