@@ -198,16 +198,19 @@ __global__ void sum_partials_kernel(const double *__restrict__ part, int n, doub
 }
 
 // ----------------------------------------------------------------------------
-// Adjoint tiling: one configuration per dtype (V = 1 keeps the 12 pointwise
-// components of sweep A in registers without spilling; FP64 takes smaller
-// blocks, as the forward sweeps do, within kAdjMaxGridPerSm).
+// Adjoint tiling, one per dtype. FP32: two sites a thread, for the packed
+// Laplacians and half the index work (656 against 888 us a step at 256^3, 121
+// against 144 at 128^3, with one site on 256 threads; 32x16, 32x4 and 64x4
+// tiles and L2 policies lay between). FP64: one site (V = 1 keeps the 12
+// pointwise components of sweep A in registers) in smaller blocks, as the
+// forward sweeps.
 constexpr int kAdjMaxGridPerSm = 4;
 
 template <typename T> struct AdjointRunner {
     static constexpr bool kF64 = std::is_same<T, double>::value;
-    static constexpr int TY = kF64 ? 4 : 8, NS = kF64 ? 7 : 8, MINB = kF64 ? 3 : 2;
-    using LB = SweepLauncher<T, 1, 32, TY, NS, MINB, AdjointB>;
-    using LA = SweepLauncher<T, 1, 32, TY, NS, MINB, AdjointA>;
+    static constexpr int V = kF64 ? 1 : 2, TY = kF64 ? 4 : 8, NS = kF64 ? 7 : 8;
+    using LB = SweepLauncher<T, V, 32, TY, NS, 3, AdjointB>;
+    using LA = SweepLauncher<T, V, 32, TY, NS, 3, AdjointA>;
 
     static int run(const axs_level *lv, const LevelGeom &g, T *abar, T *adj, double *lam_part, int lam_slots,
                    const axs_background &bg, double tau_i, double t, double dt, double *lam_acc, cudaStream_t st)
