@@ -27,10 +27,12 @@
 // the coarse step -- cubic Hermite for psi (Pi = dpsi/dtau is its derivative)
 // and linear for Pi.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <vector>
 
+#include "level_fused.cuh"
 #include "rk4_ops.cuh"
 
 namespace axs {
@@ -133,26 +135,25 @@ template <typename T> struct PatchTilings {
 };
 
 // ---------------------------------------------------------------- the fused step
-// One RK4 step of a patch without the stage buffers: each CTA owns a TX x TY
+// One RK4 step of a patch without the stage buffers, its tiles a thread-block
+// cluster. FP32 patches run the level's one-pass kernel (level_fused.cuh) in
+// place, with FusedPatches as its source: 32 x 16 tiles, clusters that take
+// patches in turn. FP64 patches run the kernel below: each CTA owns a TX x TY
 // tile of the valid cells and marches in z. Per plane it runs sweep A on the
 // tile plus a 2-cell halo (the A region) from a TMA ring of (psi, Pi) planes
 // and keeps d3, d4 (A region, 5 planes) and E, Q (tile, 3 planes) in shared
 // memory; sweep B follows two planes behind and writes psi, Pi of the step's
-// end over the old values. The tiles of one patch form a thread-block cluster
-// that advances in lockstep: after every plane of sweep A a cluster barrier
-// makes sure no tile still reads (psi, Pi) of the plane sweep B is about to
-// overwrite (the A regions of neighbouring tiles overlap). The per-site
-// arithmetic is the two sweeps' own (star_laplacian, stage_a, stage_b), so the
-// result equals theirs bit for bit, at about a third of the DRAM traffic.
-template <typename T> struct Fused {
-    // FP32: two sites per thread on 32 x 16 tiles (174 KB of shared memory, one
-    // block per SM); 32 x 8 tiles with one site per thread fit two blocks per SM
-    // but ran 20 % slower on GB300. FP64: one site per thread on 32 x 8 tiles.
+// end over the old values. The tiles of one patch advance in lockstep: after
+// every plane of sweep A a cluster barrier makes sure no tile still reads
+// (psi, Pi) of the plane sweep B is about to overwrite (the A regions of
+// neighbouring tiles overlap). The per-site arithmetic is the two sweeps' own
+// (star_laplacian, stage_a, stage_b), so the result equals theirs bit for bit,
+// at about a third of the DRAM traffic.
+struct Fused {
+    using T = double;
     // NSW / NGP: d3, d4 and E, Q slots, one more than sweep B reads, so sweep A of
     // the next plane never overwrites what a slower thread's sweep B still reads
-    static constexpr int V = sizeof(T) == 4 ? 2 : 1;
-    static constexpr int TX = 32, TY = sizeof(T) == 4 ? 16 : 8, NS = sizeof(T) == 4 ? 6 : 5;
-    static constexpr int NSW = 6, NGP = 4;
+    static constexpr int V = 1, TX = 32, TY = 8, NS = 5, NSW = 6, NGP = 4;
     static constexpr int BX = TX + 8, BY = TY + 8;  // TMA box: the A region plus its stencil halo
     static constexpr int AX = TX + 4, AY = TY + 4;  // A region
     static constexpr int RING = 4 * BX * BY, SWIN = 4 * AX * AY, GPW = 4 * TX * TY;
@@ -160,23 +161,21 @@ template <typename T> struct Fused {
     static_assert(AX / V > 32 / V, "the A region is wider than one bank row");
     static constexpr size_t SMEM = sizeof(T) * ((size_t)NS * RING + NSW * (size_t)SWIN + NGP * (size_t)GPW);
     // 512 threads: sweep A's units run on threads 0 .., sweep B's (one per thread) on the
-    // last NB threads, so a plane's critical path is at most one A unit plus one B
-    // unit (256 threads: two A units plus one B). Running A and B side by side on
-    // separate threads, with B one plane further behind, saturated the shared-memory
-    // pipe and ran 10 % slower.
+    // last NB threads, so a plane's critical path is at most one A unit plus one B unit
     static constexpr int NB = TX * TY / V;  // sweep B units, one per thread of the last NB threads
     static constexpr int THREADS = 512;
     static_assert(NB <= THREADS, "one sweep B unit per thread");
     static_assert((BX * sizeof(T)) % 16 == 0 && (RING * sizeof(T)) % 128 == 0, "TMA box rows and slots");
     static_assert(SMEM <= 227 * 1024, "shared memory");
 };
+template <typename T> using PatchTile = std::conditional_t<std::is_same<T, float>::value, LevelFusedShape<32, 16>, Fused>;
 
 // tiles of a patch side n (the cluster), or 0 when the fused step does not apply
 template <typename T> static void fused_tiles(int n, int &cx, int &cy)
 {
     cx = cy = 0;
-    if (n % Fused<T>::TX != 0 || n % Fused<T>::TY != 0) return;
-    const int x = n / Fused<T>::TX, y = n / Fused<T>::TY;
+    if (n % PatchTile<T>::TX != 0 || n % PatchTile<T>::TY != 0) return;
+    const int x = n / PatchTile<T>::TX, y = n / PatchTile<T>::TY;
     if (x * y > 8) return;  // portable cluster size
     cx = x;
     cy = y;
@@ -207,11 +206,11 @@ struct FusedArgs {
     const CUtensorMap *maps;  // per patch q: map 2 q + 1 boxes BX x BY of the state
 };
 
-template <typename T>
-__global__ void __launch_bounds__(Fused<T>::THREADS, 1) patch_fused_kernel(T *__restrict__ st, const SweepArgs<T> a,
-                                                              const FusedArgs f)
+__global__ void __launch_bounds__(Fused::THREADS, 1) patch_fused_kernel(double *__restrict__ st,
+                                                                        const SweepArgs<double> a, const FusedArgs f)
 {
-    using F = Fused<T>;
+    using F = Fused;
+    using T = double;
     constexpr int V = F::V;
     extern __shared__ __align__(128) unsigned char fused_smem[];
     T *ring = reinterpret_cast<T *>(fused_smem);
@@ -404,7 +403,7 @@ template <typename T> static int build_patch_table(const axs_patches *p, const P
             return rc;
         if (fused) {  // the fused step's box over the state
             if ((rc = make_tensor_map_4d(&maps[1], sb, p->dtype, g.js, n + 2 * kPatchRY, n + 2 * kPatchRZ, 4,
-                                         g.js * es, g.ks * es, g.plane * es, Fused<T>::BX, Fused<T>::BY, 1, 4)))
+                                         g.js * es, g.ks * es, g.plane * es, PatchTile<T>::BX, PatchTile<T>::BY, 1, 4)))
                 return rc;
         } else if ((rc = make_tensor_map_4d(&maps[1], wb, p->dtype, g.js, n + 2 * kPatchRY, n + 2 * kPatchRZ, 4,
                                             g.js * es, g.ks * es, g.plane * es, PT::TXB + 8, PT::TYB + 4, 1, 4))) {
@@ -423,13 +422,13 @@ template <typename T> static int build_patch_table(const axs_patches *p, const P
     return AXS_OK;
 }
 
-template <typename T>
-static int patch_step_fused(const axs_patches *p, const PatchGeom &g, SweepArgs<T> a, int cx, int cy, cudaStream_t st)
+static int patch_step_fused(const axs_patches *p, const PatchGeom &g, SweepArgs<double> a, int cx, int cy,
+                            cudaStream_t st)
 {
-    using F = Fused<T>;
+    using F = Fused;
     static int attr_done = 0;
     if (!attr_done) {
-        AXS_CUDA_CHECK(cudaFuncSetAttribute(patch_fused_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        AXS_CUDA_CHECK(cudaFuncSetAttribute(patch_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)F::SMEM));
         attr_done = 1;
     }
@@ -450,8 +449,50 @@ static int patch_step_fused(const axs_patches *p, const PatchGeom &g, SweepArgs<
     for (int q0 = 0; q0 < p->npatches; q0 += 65535) {
         f.q0 = q0;
         cfg.gridDim = dim3((unsigned)cx, (unsigned)cy, (unsigned)std::min(65535, p->npatches - q0));
-        AXS_CUDA_CHECK(cudaLaunchKernelEx(&cfg, patch_fused_kernel<T>, static_cast<T *>(p->state), a, f));
+        AXS_CUDA_CHECK(cudaLaunchKernelEx(&cfg, patch_fused_kernel, static_cast<double *>(p->state), a, f));
     }
+    return launch_status("patch fused step");
+}
+
+// FP32: as many clusters as fit at once, each taking patches in turn.
+static int patch_step_fused(const axs_patches *p, const PatchGeom &g, SweepArgs<float> a, int cx, int cy,
+                            cudaStream_t st)
+{
+    using S = LevelFusedShape<32, 16>;
+    auto kern = level_fused_kernel<S, FusedPatches>;
+    const int tiles = cx * cy;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)tiles, 1, 1);
+    cfg.blockDim = dim3(S::THREADS, 1, 1);
+    cfg.dynamicSmemBytes = S::SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)tiles;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    static std::atomic<int> resident[9];  // clusters of each size that fit on the device (0: not asked yet)
+    int fit = resident[tiles].load();
+    if (fit == 0) {
+        AXS_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
+        AXS_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&fit, kern, &cfg));
+        AXS_REQUIRE(fit > 0, AXS_ERR_CUDA, "no cluster of %d blocks fits on the device", tiles);
+        resident[tiles].store(fit);
+    }
+    a.nx = g.n;
+    a.tiles_x = cx;
+    a.ntiles = tiles;
+    a.n_items = p->npatches;
+    a.js = g.js;
+    a.ks = g.ks;
+    a.cs = g.box;
+    for (int c = 0; c < 4; ++c) a.out[c] = static_cast<float *>(p->state) + c * g.plane;
+    LevelFusedMaps unused;  // FusedPatches reads each patch's map from the table
+    std::memset(&unused, 0, sizeof(unused));
+    cfg.gridDim.x = (unsigned)(std::min(fit, p->npatches) * tiles);
+    AXS_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, unused, a));
     return launch_status("patch fused step");
 }
 
@@ -473,7 +514,7 @@ static int patch_step(const axs_patches *p, const PatchGeom &g, const axs_patch_
         a.c1 = stage_coef<T>(bg, tau_i + t);
         a.c2 = stage_coef<T>(bg, tau_i + t + 0.5 * dt);
         a.c4 = stage_coef<T>(bg, tau_i + t + dt);
-        return patch_step_fused<T>(p, g, a, fcx, fcy, st);
+        return patch_step_fused(p, g, a, fcx, fcy, st);
     }
     a.boxes = reinterpret_cast<const EnsBoxDesc *>(table + kPatchHeader + 2 * sizeof(CUtensorMap) * np);
     const uint32_t *items = reinterpret_cast<const uint32_t *>(a.boxes + 2 * np);
@@ -555,6 +596,7 @@ struct FillArgs {
     int64_t js, ks, box, plane;
     double theta, hdt;      // time fraction in the coarse step, coarse dt
     int valid_too;          // 1: also the valid cells (initialisation)
+    int blend;              // theta != 0
     const int *patch_list;  // the patches to fill (NULL: all), one launch row of tiles each
     // time blend weights (host-computed): psi = h[0] psi0 + h[1] Pi0 + h[2] psi1 + h[3] Pi1,
     // Pi = h[4] Pi0 + h[5] Pi1 (h[1], h[3] include the coarse dt)
@@ -565,6 +607,7 @@ struct FillArgs {
 static void fill_time_weights(FillArgs &f)
 {
     const double s = f.theta, s2 = s * s, s3 = s2 * s;
+    f.blend = s != 0.0;
     f.hd[0] = 2 * s3 - 3 * s2 + 1;
     f.hd[1] = (s3 - 2 * s2 + s) * f.hdt;
     f.hd[2] = -2 * s3 + 3 * s2;
@@ -705,7 +748,7 @@ __global__ void __launch_bounds__(kFillThreads, sizeof(T) == 4 ? 4 : 2) patch_fi
     // time blend in the field precision with host-computed weights (FP64
     // issues at 1/64 of the FP32 rate on GB300, conversions included; the
     // blend is rounded to T when stored anyway)
-    const bool blend = f.theta != 0.0;
+    const bool blend = f.blend != 0;  // theta != 0 (compared here, in FP64, once a load: 10 % of the FP64 pipe)
     const T *hw;
     if constexpr (sizeof(T) == 4)
         hw = f.hf;
@@ -946,6 +989,7 @@ static int fill_args(const axs_patches *p, const PatchGeom &g, const axs_patch_m
     f.plane = g.plane;
     f.theta = 0.0;
     f.hdt = 0.0;
+    f.blend = 0;
     f.valid_too = 0;
     f.patch_list = nullptr;
     return AXS_OK;

@@ -319,6 +319,25 @@ __device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity)
     return ok != 0;
 }
 
+// Arrive at block `rank`'s barrier that sits where `bar` does in this block.
+// Relaxed: for waits that pass no data through memory (a release at cluster
+// scope fences the warp's earlier accesses each time).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, int rank)
+{
+    asm volatile(
+        "{\n\t.reg .b32 r;\n\t"
+        "mapa.shared::cluster.u32 r, %0, %1;\n\t"
+        "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar),
+        "r"(rank)
+        : "memory");
+}
+
+// All threads of the cluster (no warp convergence needed).
+__device__ __forceinline__ void cluster_meet()
+{
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
 __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3,
                                             uint64_t *bar)
 {
