@@ -54,6 +54,7 @@ struct DiagConst {
     // single-precision copies for the per_cell_fp32 variant
     float f_one_over_dx, f_R2, f_inv_R, f_inv_R2, f_inv_R4, f_lambda, f_RpR, f_threshold;
     float f_vel_a, f_vel_b, f_vel_c;
+    float f_k12h, f_k12l;  // 1/(12 dx) as a float and its remainder (diff1_pairs)
 };
 
 template <typename T>
@@ -87,7 +88,8 @@ __device__ __forceinline__ double diff1_vals(double m2, double m1, double p1, do
         r = __dsub_rn(r, __dmul_rn(wf, p2));
         return (double)(float)__dmul_rn(r, inv_dx);
     } else {
-        return (wf * m2 - wn * m1 + wn * p1 - wf * p2) * inv_dx;
+        // differences first: an FP64 operation less than the sum of four products
+        return fma(wn * inv_dx, p1 - m1, -(wf * inv_dx) * (p2 - m2));
     }
 }
 
@@ -128,6 +130,80 @@ __device__ __forceinline__ double diff1_f32(float m2, float m1, float p1, float 
     return f2d_exact(r32);
 }
 
+// The float that diff1_f32 rounds to, without FP64 operations (GB300 issues 2
+// of them per SM and clock against 128 FP32 ones; the six diff1 values were a
+// third of the pass). diff1 = K (8 (p1 - m1) + (m2 - p2)), K = 1/(12 dx), is
+// formed as an unevaluated sum p + q of floats with Knuth's and Dekker's exact
+// sums and products, to within bound = 2^-41 K (|m2| + |m1| + |p1| + |p2|) of
+// what diff1_f32 has before its rounding: 2^-42 for the roundings of the low
+// parts, 2^-46 for the double chain's own. Ziv's test: where p + q with the
+// bound added and taken away rounds to the same float, that is diff1_f32's;
+// otherwise (and near under- or overflow) the answer is false and diff1_f32
+// has to be asked.
+__device__ __forceinline__ bool diff1_pairs(float m2, float m1, float p1, float p2, float kh, float kl, float &r32)
+{
+    auto two_diff = [](float x, float y, float &e) {
+        const float s = __fsub_rn(x, y), v = __fsub_rn(s, x);
+        e = __fsub_rn(__fsub_rn(x, __fsub_rn(s, v)), __fadd_rn(y, v));
+        return s;
+    };
+    float e1, e2;
+    const float s1 = two_diff(p1, m1, e1), s2 = two_diff(m2, p2, e2);
+    const float u = 8.f * s1, t = __fadd_rn(u, s2), v = __fsub_rn(t, u);
+    const float e3 = __fadd_rn(__fsub_rn(u, __fsub_rn(t, v)), __fsub_rn(s2, v));
+    const float lo = __fadd_rn(__fmaf_rn(8.f, e1, e2), e3);
+    const float p = __fmul_rn(t, kh), pe = __fmaf_rn(t, kh, -p);
+    const float q = __fmaf_rn(t, kl, __fmaf_rn(lo, kh, pe));
+    const float r = __fadd_rn(p, q), rest = __fsub_rn(q, __fsub_rn(r, p));
+    const float size = (fabsf(m2) + fabsf(m1) + fabsf(p1) + fabsf(p2)) * kh, bound = size * 0x1p-41f;
+    r32 = r;
+    return size > 1e-20f && size < 1e30f && __fadd_rn(r, __fadd_rn(rest, bound)) == r &&
+           __fadd_rn(r, __fsub_rn(rest, bound)) == r;
+}
+
+// A positive double within float range cut to float, and a normal float
+// widened, both by integer operations.
+__device__ __forceinline__ bool float_sized(double d)
+{
+    const int h = __double2hiint(d);
+    return h > 0x39b00000 && h < 0x46300000;  // about 2^-100 to 2^100
+}
+__device__ __forceinline__ float cut_to_float(double d)
+{
+    return __int_as_float(__funnelshift_l(__double2loint(d), __double2hiint(d) - 0x38000000, 3));
+}
+__device__ __forceinline__ double widen_normal(float x)
+{
+    const int u = __float_as_int(x);
+    return __hiloint2double((u >> 3) + 0x38000000, u << 29);
+}
+
+// 1/d and sqrt(d) of d > 0 in FP64 from a float estimate, for the few FP64
+// operations they take (3 and 5): 1/d by one step of third order, r (1 + e + e^2)
+// with e = 1 - d r (the truncated geometric series; e^3 < 2^-60), sqrt(d) by two
+// Newton steps on the residual d - s^2.
+__device__ __forceinline__ double recip_pos(double d)
+{
+    if (!float_sized(d)) return 1.0 / d;
+    const double r = widen_normal(__fdividef(1.f, cut_to_float(d)));
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+__device__ __forceinline__ double sqrt_pos(double d)
+{
+    if (!float_sized(d)) return sqrt(d);
+    const float y = rsqrtf(cut_to_float(d));
+    const double h = widen_normal(0.5f * y);
+    double s = d * widen_normal(y);
+    s = fma(fma(-s, s, d), h, s);
+    return fma(fma(-s, s, d), h, s);
+}
+// d >= 0, or a NaN, by its bits (a comparison is an FP64 operation)
+__device__ __forceinline__ bool positive(double d)
+{
+    return (__double2hiint(d) | __double2loint(d)) != 0 && __double2hiint(d) <= 0x7ff00000;
+}
+
 // The seven per-cell energy terms (EnergyKernel.hpp:130-190) and the masking
 // weight (Masking.hpp:75-93) from psi, Pi and the six diff1 values, in math
 // type M: double as the reference computes them, or float for the
@@ -136,26 +212,16 @@ template <typename M> struct CellConst {
     M R2, inv_R, inv_R2, inv_R4, lambda, RpR, threshold;
 };
 
-// gt: the diff1 values in the field precision (the reference squares them there)
-template <typename M, typename T>
-__device__ __forceinline__ void cell_energy_g(const CellConst<M> &k, int scheme, M psi1, M psi2, M Pi1, M Pi2,
-                                              const M (&g)[2][3], const T (&gt)[2][3], M (&term)[6], M &wgt)
+__device__ __forceinline__ void cell_energy(const CellConst<float> &k, int scheme, float psi1, float psi2, float Pi1,
+                                            float Pi2, const float (&g)[2][3], float (&term)[6], float &wgt)
 {
+    using M = float;
     const M psi_sq = psi1 * psi1 + psi2 * psi2;
     M g1sq = 0, g2sq = 0, cross2 = 0;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        if constexpr (sizeof(M) == 8 && sizeof(T) == 4) {
-            // the reference squares the float diff1 values in float
-            g1sq += f2d_exact(gt[0][d] * gt[0][d]);
-            g2sq += f2d_exact(gt[1][d] * gt[1][d]);
-        } else if constexpr (sizeof(M) == 8) {
-            g1sq += (M)(gt[0][d] * gt[0][d]);
-            g2sq += (M)(gt[1][d] * gt[1][d]);
-        } else {
-            g1sq += g[0][d] * g[0][d];
-            g2sq += g[1][d] * g[1][d];
-        }
+        g1sq += g[0][d] * g[0][d];
+        g2sq += g[1][d] * g[1][d];
         const M cr = psi1 * g[1][d] - psi2 * g[0][d];
         cross2 += cr * cr;
     }
@@ -184,24 +250,55 @@ __device__ __forceinline__ void cell_energy_g(const CellConst<M> &k, int scheme,
     }
 }
 
-template <typename M, typename T>
-__device__ __forceinline__ void cell_energy(const CellConst<M> &k, int scheme, M psi1, M psi2, M Pi1, M Pi2,
-                                            const M (&g)[2][3], M (&term)[6], M &wgt)
+// In double, from the diff1 values g and the same in the field precision, gt
+// (the reference squares them there). RAW: without the powers of 1/R, which the
+// caller puts on the sums (six FP64 operations a cell).
+template <typename T, bool RAW>
+__device__ __forceinline__ void cell_energy(const CellConst<double> &k, int scheme, double psi1, double psi2,
+                                            double Pi1, double Pi2, const double (&g)[2][3], const T (&gt)[2][3],
+                                            double (&term)[6], double &wgt)
 {
-    T gt[2][3];
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) gt[c][d] = (T)g[c][d];
-    cell_energy_g<M, T>(k, scheme, psi1, psi2, Pi1, Pi2, g, gt, term, wgt);
+    const double psi_sq = psi1 * psi1 + psi2 * psi2;
+    auto square = [&](int c, int d) -> double {
+        // the reference squares the float diff1 values in float
+        if constexpr (sizeof(T) == 4)
+            return f2d_exact(gt[c][d] * gt[c][d]);
+        else
+            return gt[c][d] * gt[c][d];
+    };
+    auto cross = [&](int d) { return psi1 * g[1][d] - psi2 * g[0][d]; };
+    const double g1sq = square(0, 0) + square(0, 1) + square(0, 2), g2sq = square(1, 0) + square(1, 1) + square(1, 2);
+    const double cr0 = cross(0), cr1 = cross(1), cr2 = cross(2);
+    const double inv_psq = positive(psi_sq) ? recip_pos(psi_sq) : 0.0;
+    const double gtsq_psq = (cr0 * cr0 + cr1 * cr1 + cr2 * cr2) * inv_psq, gtsq = gtsq_psq * inv_psq;
+    const double c1 = Pi1 - k.RpR * psi1, c2 = Pi2 - k.RpR * psi2;
+    const double dsq = psi_sq - k.R2;
+    const double pot = 0.25 * k.lambda * dsq * dsq;
+    const double s4 = RAW ? 1.0 : k.inv_R4, s2 = RAW ? 1.0 : k.inv_R2;
+    term[0] = (c1 * c1 + c2 * c2 + (g1sq + g2sq) + pot) * s4;  // rho
+    const double thp = (psi1 * Pi2 - Pi1 * psi2) * inv_psq;
+    term[1] = thp * thp * s2;                                  // 1/2 (sqrt(2) theta'/R)^2
+    term[2] = gtsq * s2;                                       // 1/2 sqrt(2)^2 |grad theta|^2 / R^2
+    const double rdot = psi1 * c1 + psi2 * c2;
+    term[3] = rdot * rdot * inv_psq * s4;                      // radial kinetic
+    term[4] = (g1sq + g2sq - gtsq_psq) * s4;                   // radial gradient
+    term[5] = pot * s4;                                        // radial mass
+    wgt = 1.0;
+    if (scheme == AXS_MASK_B) {
+        wgt = (sqrt_pos(psi_sq) * k.inv_R >= k.threshold) ? 1.0 : 0.0;
+    } else if (scheme != AXS_MASK_NONE) {
+        // 1 + r / f_a, r = |psi| / R - 1
+        const double f = (1.0 - 0.70710678118654752440) + sqrt_pos(psi_sq) * (k.inv_R * 0.70710678118654752440);
+        wgt = f * f;
+    }
 }
 
 // Tiled diagnostics pass. A block owns a DTX x DTY tile of cells and marches
 // in z over a chunk. Shared memory holds psi1/psi2 of six planes (tile plus a
 // 2-cell halo: the five of the gradient stencil and one in flight), Pi1/Pi2 of
 // three vertex planes ((DTX+1) x (DTY+1) vertices: z, z+1 and one in flight),
-// and for the two vertex planes z and z+1 the single-precision phases and
-// gamma^2 v^2, each computed once per vertex. Planes arrive by element-wise
+// and for the two vertex planes z and z+1 the single-precision phases (and with
+// FP32 per-cell terms gamma^2 v^2), each computed once per vertex. Planes arrive by element-wise
 // cp.async one plane ahead of their use, so their latency overlaps the
 // current plane's work. Plane loads use element offsets precomputed per work
 // item, so the march needs no index division.
@@ -217,16 +314,25 @@ constexpr int kVtxPer = (kVtxPts + kDiagThreads - 1) / kDiagThreads;      // ver
 // past the plane that last read it (psi: the 5-plane stencil plus two;
 // Pi: read at its vertex plane and again at its cell plane, plus two).
 // Vertex planes are computed one plane ahead into a third slot.
+// With FP64 per-cell terms the pass is bound by the FP64 pipe (75 % busy with
+// about 86 operations a cell; 160 with the diff1 chains, gamma^2 v^2 at every
+// vertex, library division and root, and the powers of 1/R in every cell):
+// 256^3 on FP32 fields 5.36 -> 2.9 ms.
 constexpr int kPsiSlots = 7, kPiSlots = 5, kVtxSlots = 3;
 // pierced plaquettes buffered per block; flushed to the global list with one
 // atomic once a plane could overflow it (at most 3 entries per cell)
 constexpr int kListBuf = 1536, kListFlushAt = kListBuf - 3 * kDiagThreads;
+constexpr int kVelQueue = 7 + 3 * 32;  // fewer than 8 left over, and a plane's
 template <typename T, bool FAST> struct DiagSmem {
     long long lbuf[kListBuf];
     T ps[kPsiSlots][2][DHY][DHX];
     T pi[kPiSlots][2][DVY][DVX];
-    typename std::conditional<FAST, float, double>::type gv[kVtxSlots][DVY][DVX];
+    // FAST: gamma^2 v^2 of the vertices; else the pierced plaquettes whose corners'
+    // values a warp still has to add up (vel_corners)
+    typename std::conditional<FAST, float[kVtxSlots][DVY][DVX], unsigned[kDiagThreads / 32][kVelQueue]>::type gv;
     float th[kVtxSlots][DVY][DVX];
+    float tie_value[kDiagThreads / 32][6 * 32];  // of a warp's undecided diff1 values: the float, and which they are
+    unsigned char tie[kDiagThreads / 32][6 * 32];
     unsigned char ok[kVtxSlots][DVY][DVX];
 };
 
@@ -289,6 +395,9 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
         warp_end = 0;
     };
 
+    int vq_n = 0;  // entries of this warp's plaquette queue (lane-uniform)
+    int n_cells = 0;
+
     for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
         // boxes of one batch share the view's geometry and sit box_stride apart
         const long long qbox = item / items_per_box, box_item = item % items_per_box;
@@ -341,7 +450,7 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
             }
         };
         auto load_pi = [&](int z) {
-            if (!q.want_energy && !q.want_vel) return;  // the string finder alone reads psi only
+            if (!q.want_energy && !(FAST && q.want_vel)) return;  // the string finder alone reads psi only
             bool zin;
             const int64_t po = plane_off(z, zin);
             T *pdst = &sm.pi[(z - za) % kPiSlots][0][0][0];
@@ -371,7 +480,8 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
                     sm.ok[ts][vy][vx] = (m > 1e-30 && m < 1e30) ? 1 : 0;
                 }
                 sm.th[ts][vy][vx] = atan2f((float)b, (float)a);
-                if (q.want_vel && FAST) {
+                if constexpr (FAST) {
+                    if (!q.want_vel) continue;
                     const float psi1 = a, psi2 = b, Pi1 = sm.pi[ps_][0][vy][vx], Pi2 = sm.pi[ps_][1][vy][vx];
                     const float phi1 = psi1 * q.f_inv_R, phi2 = psi2 * q.f_inv_R;
                     const float pd1 = (Pi1 - q.f_RpR * psi1) * q.f_inv_R2, pd2 = (Pi2 - q.f_RpR * psi2) * q.f_inv_R2;
@@ -379,17 +489,42 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
                     const float pd_sq = pd1 * pd1 + pd2 * pd2;
                     const float re = phi1 * pd1 + phi2 * pd2;
                     sm.gv[ts][vy][vx] = pd_sq * q.f_vel_a * (1.f - q.f_vel_b * phi_sq) - q.f_vel_c * re * re;
-                } else if (q.want_vel) {
-                    const double psi1 = widen(a), psi2 = widen(b), Pi1 = widen(sm.pi[ps_][0][vy][vx]),
-                                 Pi2 = widen(sm.pi[ps_][1][vy][vx]);
+                }
+            }
+        };
+
+        // gamma^2 v^2 (Velocity.hpp:62-78, the constant prefactors folded on the host)
+        // of the corners of `take` queued plaquettes of this warp, a corner to a lane,
+        // from global memory: 17 FP64 operations for eight plaquettes instead of for
+        // every vertex of the grid (an eighth of the pass). Entries: plane in the
+        // chunk, orientation, lane of the cell (a warp is a row of cells).
+        auto vel_corners = [&](int take) {
+            if constexpr (!FAST) {
+                __syncwarp();
+                vq_n -= take;
+                const int k = (tid & 31) >> 2, j = tid & 3;
+                if (k < take) {
+                    const unsigned en = sm.gv[tid >> 5][vq_n + k];
+                    const int pl = (en >> 5) & 3;
+                    const int mid = j == 1 || j == 2, far = j >= 2;
+                    int x = x0 + (int)(en & 31) + (pl == 0 ? mid : pl == 2 ? far : 0);
+                    int y = y0 + ly + (pl == 0 ? far : pl == 1 ? mid : 0);
+                    int z = za + (int)(en >> 7) + (pl == 1 ? far : pl == 2 ? mid : 0);
+                    const bool on = (v.wx || x < v.nx + v.ox) && (v.wy || y < v.ny + v.oy) && (v.wz || z < v.nz + v.oz);
+                    if (v.wx && x == v.nx) x = 0;
+                    if (v.wy && y == v.ny) y = 0;
+                    if (v.wz && z == v.nz) z = 0;
+                    const T *at = base + (x + v.ox) + (int64_t)(y + v.oy) * v.js + (int64_t)(z + v.oz) * v.ks;
+                    auto val = [&](int c) { return on ? widen(at[c * v.cs]) : 0.0; };
+                    const double psi1 = val(0), psi2 = val(1), Pi1 = val(2), Pi2 = val(3);
                     const double phi1 = psi1 * q.inv_R, phi2 = psi2 * q.inv_R;
                     const double pd1 = (Pi1 - q.RpR * psi1) * q.inv_R2, pd2 = (Pi2 - q.RpR * psi2) * q.inv_R2;
                     const double phi_sq = phi1 * phi1 + phi2 * phi2;
                     const double pd_sq = pd1 * pd1 + pd2 * pd2;
                     const double re = phi1 * pd1 + phi2 * pd2;
-                    // Velocity.hpp:62-78 with the constant prefactors folded on the host
-                    sm.gv[ts][vy][vx] = pd_sq * q.vel_a * (1.0 - q.vel_b * phi_sq) - q.vel_c * re * re;
+                    vsum += pd_sq * q.vel_a * (1.0 - q.vel_b * phi_sq) - q.vel_c * re * re;
                 }
+                __syncwarp();
             }
         };
 
@@ -426,12 +561,57 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
             const int64_t cell = qbox * box_cells + (int64_t)x + (int64_t)v.nx * ((int64_t)y + (int64_t)v.ny * z);
             const bool in = x < v.nx && y < v.ny && (mask == nullptr || mask[cell] != 0);
             int w[3] = {0, 0, 0};
+            const int s0 = (m + 2) % kPsiSlots;
+            const int sm1 = (m + 1) % kPsiSlots, sp1 = (m + 3) % kPsiSlots, sm2 = m % kPsiSlots,
+                      sp2 = (m + 4) % kPsiSlots;
+            const int hx = lx + 2, hy = ly + 2;
+            // the four taps of diff1 of component c along axis d at the cell of lane l
+            auto taps = [&](int c, int d, int l, float (&f)[4]) {
+                const T(*pl)[DHX] = sm.ps[s0][c];
+                const int x_ = l + 2;
+                f[0] = d == 0 ? pl[hy][x_ - 2] : d == 1 ? pl[hy - 2][x_] : sm.ps[sm2][c][hy][x_];
+                f[1] = d == 0 ? pl[hy][x_ - 1] : d == 1 ? pl[hy - 1][x_] : sm.ps[sm1][c][hy][x_];
+                f[2] = d == 0 ? pl[hy][x_ + 1] : d == 1 ? pl[hy + 1][x_] : sm.ps[sp1][c][hy][x_];
+                f[3] = d == 0 ? pl[hy][x_ + 2] : d == 1 ? pl[hy + 2][x_] : sm.ps[sp2][c][hy][x_];
+            };
+            float gf[2][3] = {};
+            if constexpr (sizeof(T) == 4 && !FAST) {
+                if (q.want_energy) {
+                    // Exact ties are common (at dx = 1/2 the sum of taps is divided by 6, and
+                    // the double chain's own roundings decide them): the warp's undecided
+                    // values, a few per cent, go through the FP64 chain together, a value to a lane.
+                    int n = 0;
+                    unsigned undecided = 0;
+#pragma unroll
+                    for (int cd = 0; cd < 6; ++cd) {
+                        float f[4];
+                        taps(cd / 3, cd % 3, lx, f);
+                        const bool sure = diff1_pairs(f[0], f[1], f[2], f[3], q.f_k12h, q.f_k12l, gf[cd / 3][cd % 3]) || !in;
+                        const unsigned who = __ballot_sync(0xffffffffu, !sure);
+                        if (!sure) {
+                            sm.tie[ly][n + __popc(who & ((1u << lx) - 1u))] = (unsigned char)(cd * 32 + lx);
+                            undecided |= 1u << cd;
+                        }
+                        n += __popc(who);
+                    }
+                    if (n > 0) {
+                        __syncwarp();
+                        for (int k = lx; k < n; k += 32) {
+                            const int en = sm.tie[ly][k], cd = en >> 5;
+                            float f[4], r;
+                            taps(cd / 3, cd % 3, en & 31, f);
+                            diff1_f32(f[0], f[1], f[2], f[3], q.one_over_dx, r);
+                            sm.tie_value[ly][en] = r;
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int cd = 0; cd < 6; ++cd)
+                            if (undecided >> cd & 1u) gf[cd / 3][cd % 3] = sm.tie_value[ly][cd * 32 + lx];
+                    }
+                }
+            }
             if (in) {
-                const int s0 = (m + 2) % kPsiSlots;
-                const int sm1 = (m + 1) % kPsiSlots, sp1 = (m + 3) % kPsiSlots, sm2 = m % kPsiSlots,
-                          sp2 = (m + 4) % kPsiSlots;
                 const int t0 = m % kVtxSlots, t1 = (m + 1) % kVtxSlots, tp = m % kPiSlots;
-                const int hx = lx + 2, hy = ly + 2;
                 if (q.want_energy) {
                     const T p1 = sm.ps[s0][0][hy][hx], p2 = sm.ps[s0][1][hy][hx];
                     const T q1 = sm.pi[tp][0][ly][lx], q2 = sm.pi[tp][1][ly][lx];
@@ -452,7 +632,7 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
                                            wn * (sm.ps[sp1][c][hy][hx] - sm.ps[sm1][c][hy][hx])) * q.f_one_over_dx;
                             }
                             float term[6], wgt;
-                            cell_energy<float, T>(kf, q.scheme, p1, p2, q1, q2, g, term, wgt);
+                            cell_energy(kf, q.scheme, p1, p2, q1, q2, g, term, wgt);
 #pragma unroll
                             for (int k = 0; k < 6; ++k) {
                                 csum(ef[2 * k], ec[2 * k], term[k]);
@@ -467,20 +647,21 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
                         double g[2][3], term[6], wgt;
                         if constexpr (sizeof(T) == 4) {
                             // FP32 fields: taps widened by integer operations (f2d_exact)
-                            float gf[2][3];
+                            if constexpr (FAST) {
 #pragma unroll
-                            for (int c = 0; c < 2; ++c) {
-                                g[c][0] = diff1_f32(sm.ps[s0][c][hy][hx - 2], sm.ps[s0][c][hy][hx - 1],
-                                                    sm.ps[s0][c][hy][hx + 1], sm.ps[s0][c][hy][hx + 2], q.one_over_dx,
-                                                    gf[c][0]);
-                                g[c][1] = diff1_f32(sm.ps[s0][c][hy - 2][hx], sm.ps[s0][c][hy - 1][hx],
-                                                    sm.ps[s0][c][hy + 1][hx], sm.ps[s0][c][hy + 2][hx], q.one_over_dx,
-                                                    gf[c][1]);
-                                g[c][2] = diff1_f32(sm.ps[sm2][c][hy][hx], sm.ps[sm1][c][hy][hx],
-                                                    sm.ps[sp1][c][hy][hx], sm.ps[sp2][c][hy][hx], q.one_over_dx,
-                                                    gf[c][2]);
+                                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                                    for (int d = 0; d < 3; ++d) {
+                                        float f[4];
+                                        taps(c, d, lx, f);
+                                        diff1_f32(f[0], f[1], f[2], f[3], q.one_over_dx, gf[c][d]);
+                                    }
                             }
-                            cell_energy_g<double, float>(kd, q.scheme, f2d_exact(p1), f2d_exact(p2), f2d_exact(q1),
+#pragma unroll
+                            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                                for (int d = 0; d < 3; ++d) g[c][d] = f2d_exact(gf[c][d]);
+                            cell_energy<float, !FAST>(kd, q.scheme, f2d_exact(p1), f2d_exact(p2), f2d_exact(q1),
                                                          f2d_exact(q2), g, gf, term, wgt);
                         } else {
 #pragma unroll
@@ -494,7 +675,7 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
                                 g[c][2] = diff1_vals<T>(sm.ps[sm2][c][hy][hx], sm.ps[sm1][c][hy][hx],
                                                         sm.ps[sp1][c][hy][hx], sm.ps[sp2][c][hy][hx], q.one_over_dx);
                             }
-                            cell_energy<double, T>(kd, q.scheme, p1, p2, q1, q2, g, term, wgt);
+                            cell_energy<T, !FAST>(kd, q.scheme, p1, p2, q1, q2, g, g, term, wgt);
                         }
 #pragma unroll
                         for (int k = 0; k < 6; ++k) {
@@ -502,7 +683,7 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
                             e[2 * k + 1] += term[k] * wgt;
                         }
                         e[12] += wgt;
-                        e[13] += 1.0;
+                        ++n_cells;
                     }
                 }
                 if (q.want_plaq || q.want_vel) {
@@ -538,19 +719,32 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
                     if (tags != nullptr) tags[cell] = (w[0] | w[1] | w[2]) != 0;
                     cnt[0] += (w[0] != 0) + (w[1] != 0) + (w[2] != 0);
                     cnt[1] += abs(w[0]) + abs(w[1]) + abs(w[2]);
-                    if (q.want_vel && (w[0] | w[1] | w[2])) {
-                        const double g000 = sm.gv[t0][ly][lx], g100 = sm.gv[t0][ly][lx + 1];
-                        const double g110 = sm.gv[t0][ly + 1][lx + 1], g010 = sm.gv[t0][ly + 1][lx];
-                        const double g001 = sm.gv[t1][ly][lx], g101 = sm.gv[t1][ly][lx + 1];
-                        const double g011 = sm.gv[t1][ly + 1][lx];
-                        double s = 0.0;
-                        long long c = 0;
-                        if (w[0]) { s += g000 + g100 + g110 + g010; c += 4; }
-                        if (w[1]) { s += g000 + g010 + g011 + g001; c += 4; }
-                        if (w[2]) { s += g000 + g001 + g101 + g100; c += 4; }
-                        vsum += s;
-                        cnt[2] += c;
+                    if constexpr (FAST) {
+                        if (q.want_vel && (w[0] | w[1] | w[2])) {
+                            const double g000 = sm.gv[t0][ly][lx], g100 = sm.gv[t0][ly][lx + 1];
+                            const double g110 = sm.gv[t0][ly + 1][lx + 1], g010 = sm.gv[t0][ly + 1][lx];
+                            const double g001 = sm.gv[t1][ly][lx], g101 = sm.gv[t1][ly][lx + 1];
+                            const double g011 = sm.gv[t1][ly + 1][lx];
+                            double s = 0.0;
+                            if (w[0]) s += g000 + g100 + g110 + g010;
+                            if (w[1]) s += g000 + g010 + g011 + g001;
+                            if (w[2]) s += g000 + g001 + g101 + g100;
+                            vsum += s;
+                        }
                     }
+                    if (q.want_vel) cnt[2] += 4 * ((w[0] != 0) + (w[1] != 0) + (w[2] != 0));
+                }
+            }
+            if constexpr (!FAST) {
+                if (q.want_vel && __any_sync(0xffffffffu, (w[0] | w[1] | w[2]) != 0)) {
+#pragma unroll
+                    for (int pl = 0; pl < 3; ++pl) {
+                        const unsigned hit = __ballot_sync(0xffffffffu, w[pl] != 0);
+                        if (w[pl])
+                            sm.gv[tid >> 5][vq_n + __popc(hit & ((1u << lx) - 1u))] = (unsigned)m << 7 | pl << 5 | lx;
+                        vq_n += __popc(hit);
+                    }
+                    while (vq_n >= 8) vel_corners(8);
                 }
             }
             // ---- pierced plaquettes of this plane into the block's buffer: a warp
@@ -576,6 +770,7 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
                 }
             }
         }
+        if (vq_n > 0) vel_corners(vq_n);
         __syncthreads();  // the next item's prologue refills the rings
         if constexpr (FAST) {
 #pragma unroll
@@ -589,6 +784,11 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
     // the rest of the buffer (warp_end > 0: the warp appended since the last flush)
     if (q.want_plaq && list != nullptr && __syncthreads_or(warp_end > 0)) flush();
 
+    if constexpr (!FAST) {  // the terms' powers of 1/R
+#pragma unroll
+        for (int s = 0; s < 12; ++s) e[s] *= s >= 2 && s < 6 ? kd.inv_R2 : kd.inv_R4;
+    }
+    e[13] += (double)n_cells;
     // ---- block reduction (fixed order) ----
     __shared__ double red_d[kDiagThreads / 32][15];
     __shared__ long long red_l[kDiagThreads / 32][4];
@@ -1110,8 +1310,11 @@ __device__ __noinline__ CellTerms energy_cell_double(const DiagView v, const Dia
     }
     const CellConst<double> kd{q.R2, q.inv_R, q.inv_R2, q.inv_R4, q.lambda, q.RpR, q.threshold};
     double term[6], wgt;
-    cell_energy<double, float>(kd, q.scheme, at(0, x, y, z), at(1, x, y, z), at(2, x, y, z), at(3, x, y, z), g, term,
-                               wgt);
+    float gt[2][3];
+    for (int c = 0; c < 2; ++c)
+        for (int d = 0; d < 3; ++d) gt[c][d] = (float)g[c][d];
+    cell_energy<float, false>(kd, q.scheme, at(0, x, y, z), at(1, x, y, z), at(2, x, y, z), at(3, x, y, z), g, gt, term,
+                              wgt);
     CellTerms r;
     for (int k = 0; k < 6; ++k) {
         r.t[2 * k] = term[k];
@@ -1242,7 +1445,7 @@ __global__ void __launch_bounds__(kDiagThreads, 3)
                                wn * (sm.ps[sp1][c][hy][hx] - sm.ps[sm1][c][hy][hx])) * q.f_one_over_dx;
                 }
                 float term[6], wgt;
-                cell_energy<float, float>(kf, q.scheme, p1, p2, sm.pi[tp][0][cy][lx], sm.pi[tp][1][cy][lx], g,
+                cell_energy(kf, q.scheme, p1, p2, sm.pi[tp][0][cy][lx], sm.pi[tp][1][cy][lx], g,
                                           term, wgt);
 #pragma unroll
                 for (int k = 0; k < 6; ++k) {
@@ -1452,6 +1655,8 @@ static int run_diag(const DiagView &v, const axs_diag_params *p, const uint8_t *
     q.want_plaq = p->want_plaquettes != 0;
     q.want_vel = p->want_velocity != 0;
     q.f_one_over_dx = (float)q.one_over_dx;
+    q.f_k12h = (float)(q.one_over_dx / 12.0);
+    q.f_k12l = (float)(q.one_over_dx / 12.0 - (double)q.f_k12h);
     q.f_R2 = (float)q.R2;
     q.f_inv_R = (float)q.inv_R;
     q.f_inv_R2 = (float)q.inv_R2;

@@ -372,3 +372,44 @@ def test_network_scalars_row_matches_oracle(axs, orc, dtype):
     for q in (0, 1, 21):
         assert row[q] == ref[q], output.NETWORK_COLUMNS[q]
     np.testing.assert_allclose(row, ref, rtol=1e-12 if dtype == torch.float64 else 1e-6, atol=0)
+
+
+@pytest.mark.parametrize("dx", [0.5, 0.3, 1.0])
+@pytest.mark.parametrize("kind", ["waves", "steps", "decades", "tiny", "large"])
+def test_fp32_fields_in_double_terms_at_every_scale(axs, orc, kind, dx):
+    """The pass with FP64 per-cell terms on FP32 fields, whose diff1 values come
+    from FP32 pairs where their rounding is certain and from the double chain
+    where it is not: smooth fields (mostly certain), fields of few distinct
+    values (ties), taps decades apart, and fields near the ends of the pairs'
+    range, on a box that leaves partial tiles and z-chunks, against the FLOAT
+    build (which rounds every diff1 as the chain does): sums to 1e-12, as for
+    the other boxes."""
+    from oracle.oracle import energy_sums, velocity
+    nx, ny, nz = 37, 21, 13
+    dx = float(np.float32(dx))  # the FLOAT build receives it as a float
+    rng = np.random.default_rng(4)
+    z, y, x = np.meshgrid(np.arange(nz), np.arange(ny), np.arange(nx), indexing="ij")
+    v = np.stack([np.cos(0.31 * x + 0.2 * y * (c + 1) - 0.17 * z + c) + 0.2 * np.sin(0.9 * x - 0.7 * z + c) for c in range(4)])
+    if kind == "steps":
+        v = np.round(4 * v) / 4 + 0.125
+    elif kind == "decades":
+        v *= 10.0 ** rng.integers(-6, 1, v.shape)
+    elif kind == "tiny":
+        v *= 1e-12
+    elif kind == "large":
+        v *= 1e8
+    v = v.astype(np.float32)
+    R, lam, rpr, m_r = (float(np.float32(s)) for s in (1.3 * np.abs(v).max(), 0.7, 0.4, 1.1))
+    f = orc.to_fab(v, 2)
+    t = axs.new_fab((nx, ny, nz), 2, dtype=torch.float32)
+    axs.valid(t, 2).copy_(_dev(v))
+    axs.fill_periodic_ghosts(t, 2)
+    for scheme in range(3):
+        p = axs._lib.DiagParams(dx, R, lam, rpr, m_r, scheme, 0.8, axs._lib.BOUNDARY_GHOSTS, 1, 1, 1, 0)
+        r, _ = _run_diag(axs, t, 2, p)
+        np.testing.assert_allclose(list(r.energy_sums), energy_sums(f, 2, dx, R, lam, rpr, scheme, 0.8), rtol=1e-12,
+                                   atol=1e-300)
+    assert (r.n_p_plain, r.n_p_weighted) == orc.count_plaquettes(f, 2)
+    vs, vc = velocity(f, 2, R, rpr, m_r)
+    if vc == 4 * r.n_p_plain:  # float and double atan2 agree on every winding
+        assert r.vel_count == vc and r.vel_sum == pytest.approx(vs, rel=1e-12)
