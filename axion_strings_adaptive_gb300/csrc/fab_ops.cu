@@ -53,32 +53,52 @@ __device__ __forceinline__ double diff2_exact(const double *__restrict__ p, int6
     return __dmul_rn(r, one_over_dx2);
 }
 
-__global__ void eval_rhs_f64_kernel(const axs_fab s, const axs_fab r, double one_over_dx2, double kappa,
-                                    double lambda, double R2)
+// The cell of thread `tid` of a block whose first cell is number `first` of the
+// box (x fastest): 64-bit arithmetic once a block.
+struct CellIdx {
+    int i, j, k;
+};
+__device__ __forceinline__ CellIdx cell_index(int64_t first, int tid, int nx, int ny)
+{
+    const int64_t row0 = first / nx;
+    const unsigned x = (unsigned)(first - row0 * nx) + (unsigned)tid, up = x / (unsigned)nx;
+    const unsigned row = (unsigned)row0 + up;  // rows fit 31 bits (rows_fit)
+    CellIdx c;
+    c.i = (int)(x - up * (unsigned)nx);
+    c.k = (int)(row / (unsigned)ny);
+    c.j = (int)(row - (unsigned)c.k * (unsigned)ny);
+    return c;
+}
+
+// Bound by the FP64 pipe (76 operations a cell), which serves a warp of one
+// cell as long as a full one: cells are numbered through, so that rows of any
+// length fill the warps, in small blocks that even out over the SMs: 97x75x50
+// 54.8 us, 96^3 130 us (the pipe's own time: 44 and 107), where a warp a row
+// took 90 and 135.
+constexpr int kRhs64Threads = 128;
+__global__ void __launch_bounds__(kRhs64Threads) eval_rhs_f64_kernel(const axs_fab s, const axs_fab r,
+                                                                     double one_over_dx2, double kappa, double lambda,
+                                                                     double R2, int64_t cells)
 {
     const double *__restrict__ sp = static_cast<const double *>(s.data);
     double *__restrict__ rp = static_cast<double *>(r.data);
-    const int rows = s.ny * s.nz, lane = threadIdx.x & 31;
     const int64_t st[3] = {1, s.jstride, s.kstride};
-    for (int row = row_warp(); row < rows; row += row_warps()) {
-        const RowIdx q = row_index(row, s.ny, s.nz);
-        const int64_t o0 = fab_off(s, 0, q.j, q.k), r0 = fab_off(r, 0, q.j, q.k);
-        for (int i = lane; i < s.nx; i += 32) {
-            const int64_t o = o0 + i;
-            double lap1 = 0.0, lap2 = 0.0;
+    for (int64_t first = (int64_t)blockIdx.x * kRhs64Threads; first < cells; first += (int64_t)gridDim.x * kRhs64Threads) {
+        if (first + threadIdx.x >= cells) return;
+        const CellIdx q = cell_index(first, threadIdx.x, s.nx, s.ny);
+        const int64_t o = fab_off(s, q.i, q.j, q.k), ro = fab_off(r, q.i, q.j, q.k);
+        double lap1 = 0.0, lap2 = 0.0;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) lap1 = __dadd_rn(lap1, diff2_exact(sp + o, st[d], one_over_dx2));
+        for (int d = 0; d < 3; ++d) lap1 = __dadd_rn(lap1, diff2_exact(sp + o, st[d], one_over_dx2));
 #pragma unroll
-            for (int d = 0; d < 3; ++d) lap2 = __dadd_rn(lap2, diff2_exact(sp + s.cstride + o, st[d], one_over_dx2));
-            const double psi1 = sp[o], psi2 = sp[s.cstride + o];
-            const double dsq = __dsub_rn(__dadd_rn(__dmul_rn(psi1, psi1), __dmul_rn(psi2, psi2)), R2);
-            const double pc = __dmul_rn(__dmul_rn(0.5, lambda), dsq);
-            const int64_t ro = r0 + i;
-            rp[ro] = sp[2 * s.cstride + o];
-            rp[r.cstride + ro] = sp[3 * s.cstride + o];
-            rp[2 * r.cstride + ro] = __dsub_rn(__dadd_rn(lap1, __dmul_rn(kappa, psi1)), __dmul_rn(pc, psi1));
-            rp[3 * r.cstride + ro] = __dsub_rn(__dadd_rn(lap2, __dmul_rn(kappa, psi2)), __dmul_rn(pc, psi2));
-        }
+        for (int d = 0; d < 3; ++d) lap2 = __dadd_rn(lap2, diff2_exact(sp + s.cstride + o, st[d], one_over_dx2));
+        const double psi1 = sp[o], psi2 = sp[s.cstride + o];
+        const double dsq = __dsub_rn(__dadd_rn(__dmul_rn(psi1, psi1), __dmul_rn(psi2, psi2)), R2);
+        const double pc = __dmul_rn(__dmul_rn(0.5, lambda), dsq);
+        rp[ro] = sp[2 * s.cstride + o];
+        rp[r.cstride + ro] = sp[3 * s.cstride + o];
+        rp[2 * r.cstride + ro] = __dsub_rn(__dadd_rn(lap1, __dmul_rn(kappa, psi1)), __dmul_rn(pc, psi1));
+        rp[3 * r.cstride + ro] = __dsub_rn(__dadd_rn(lap2, __dmul_rn(kappa, psi2)), __dmul_rn(pc, psi2));
     }
 }
 
@@ -278,6 +298,33 @@ __device__ __forceinline__ float rn_sub(float a, float b) { return __fsub_rn(a, 
 __device__ __forceinline__ double rn_div(double a, double b) { return __ddiv_rn(a, b); }
 __device__ __forceinline__ float rn_div(float a, float b) { return __fdiv_rn(a, b); }
 
+// 2 x, exactly: a normal double's exponent one up (an FP64 operation is a
+// third of the combination's time), the rest by the multiplication.
+__device__ __forceinline__ double twice(double x)
+{
+    const int h = __double2hiint(x), e = h & 0x7ff00000;
+    if (e - 0x100000 < 0x7fd00000 && e != 0) return __hiloint2double(h + 0x100000, __double2loint(x));
+    return __dmul_rn(2.0, x);
+}
+
+// FP64 form of rk4_combine_kernel below: the same expressions, cells numbered
+// through (FP64-bound like the RHS; rows of any length fill the warps),
+// components on grid y. 97x75x50: 29.3 -> 21.9 us, 96^3: 53 -> 50.
+__global__ void __launch_bounds__(256) rk4_combine_f64_kernel(const axs_fab d, const axs_fab u, const axs_fab k1,
+                                                              const axs_fab k2, const axs_fab k3, const axs_fab k4,
+                                                              double h6, int64_t cells)
+{
+    const int c = blockIdx.y;
+    for (int64_t first = (int64_t)blockIdx.x * 256; first < cells; first += (int64_t)gridDim.x * 256) {
+        if (first + threadIdx.x >= cells) return;
+        const CellIdx q = cell_index(first, threadIdx.x, d.nx, d.ny);
+        auto at = [&](const axs_fab &f) { return static_cast<double *>(f.data) + c * f.cstride + fab_off(f, q.i, q.j, q.k); };
+        const double a = *at(k1), b = *at(k2), e = *at(k3), f = *at(k4), v = *at(u);
+        const double sum = rn_add(rn_add(rn_add(a, twice(b)), twice(e)), f);
+        *at(d) = rn_add(v, rn_mul(h6, sum));
+    }
+}
+
 template <typename T>
 __global__ void lincomb_kernel(const axs_fab d, const axs_fab x, T b, const axs_fab y, int ncomp)
 {
@@ -299,6 +346,7 @@ __global__ void lincomb_kernel(const axs_fab d, const axs_fab x, T b, const axs_
     }
 }
 
+// FP32; FP64 above
 template <typename T>
 __global__ void rk4_combine_kernel(const axs_fab d, const axs_fab u, const axs_fab k1, const axs_fab k2,
                                    const axs_fab k3, const axs_fab k4, T h6, int ncomp)
@@ -600,6 +648,21 @@ int axs_level_count_nonfinite(const axs_level *lv, int64_t *count_dev, void *str
                            (cudaStream_t)stream);
 }
 
+// Grids of the kernels that number the cells through.
+static int64_t cell_count(const axs_fab &f) { return (int64_t)f.nx * f.ny * f.nz; }
+static dim3 cell_grid(const axs_fab &f, int ncomp)
+{
+    return dim3((unsigned)std::min<int64_t>((cell_count(f) + 255) / 256, 1 << 20), (unsigned)ncomp);
+}
+
+static void launch_eval_rhs_f64(const axs_fab &s, const axs_fab &r, double one_over_dx2, const axs_rhs_coeffs &c,
+                                cudaStream_t st)
+{
+    const int64_t cells = (int64_t)s.nx * s.ny * s.nz;
+    const int64_t blocks = std::min<int64_t>((cells + kRhs64Threads - 1) / kRhs64Threads, 1 << 20);
+    eval_rhs_f64_kernel<<<(unsigned)blocks, kRhs64Threads, 0, st>>>(s, r, one_over_dx2, c.kappa, c.lambda, c.R2, cells);
+}
+
 int axs_eval_rhs(const axs_fab *soln, const axs_fab *rhs, double dx, const axs_rhs_coeffs *c, void *stream)
 {
     int rc = validate_fab(soln, "soln", 4, 2);
@@ -609,23 +672,29 @@ int axs_eval_rhs(const axs_fab *soln, const axs_fab *rhs, double dx, const axs_r
     AXS_REQUIRE(c != nullptr, AXS_ERR_INVALID_ARGUMENT, "null coefficients");
     AXS_REQUIRE(dx > 0.0, AXS_ERR_INVALID_ARGUMENT, "dx must be positive");
     if ((rc = rows_fit(soln, "eval_rhs"))) return rc;
-    const int g = grid_rows((int64_t)soln->ny * soln->nz);
     const double one_over_dx2 = 1.0 / (dx * dx);
     cudaStream_t st = (cudaStream_t)stream;
     if (soln->dtype == AXS_F64)
-        eval_rhs_f64_kernel<<<g, 256, 0, st>>>(*soln, *rhs, one_over_dx2, c->kappa, c->lambda, c->R2);
+        launch_eval_rhs_f64(*soln, *rhs, one_over_dx2, *c, st);
     else {
-        const dim3 grid((soln->nx + 31) / 32, (soln->ny + 7) / 8, (soln->nz + 63) / 64), block(32, 8);
+        // Planes a block marches: 64, or down to 8 where the box is too small to give
+        // every SM four blocks (a march loads 4 planes more than it computes): 128^3
+        // 32.5 -> 22.7 us with 16 planes, 64^3 22 -> 4.6 us with 8. At compile time:
+        // a run-time length cost 4 % at 256^3.
+        const int64_t cols = (int64_t)((soln->nx + 31) / 32) * ((soln->ny + 7) / 8);
+        const int sms = std::max(1, device_sm_count());
+        int zc = 64;
+        while (zc > 8 && cols * ((soln->nz + zc - 1) / zc) < 4 * (int64_t)sms) zc /= 2;
         const bool w16 = soln->ng % 4 == 2 && soln->jstride % 4 == 0 && soln->kstride % 4 == 0 &&
                          soln->cstride % 4 == 0 && (uintptr_t)soln->data % 16 == 0 && soln->nx % 32 == 0 &&
                          soln->ny % 8 == 0;
         const float k = (float)c->kappa, l = (float)c->lambda, r2 = (float)c->R2;
-        if (w16)
-            eval_rhs_f32_zmarch_kernel<8, 64, 2, true><<<grid, block, 0, st>>>(*soln, *rhs, (float)one_over_dx2, k, l,
-                                                                               r2);
-        else
-            eval_rhs_f32_zmarch_kernel<8, 64, 2, false><<<grid, block, 0, st>>>(*soln, *rhs, (float)one_over_dx2, k, l,
-                                                                                r2);
+        const dim3 grid((soln->nx + 31) / 32, (soln->ny + 7) / 8, (soln->nz + zc - 1) / zc), block(32, 8);
+        auto kern = zc == 64   ? (w16 ? eval_rhs_f32_zmarch_kernel<8, 64, 2, true> : eval_rhs_f32_zmarch_kernel<8, 64, 2, false>)
+                    : zc == 32 ? (w16 ? eval_rhs_f32_zmarch_kernel<8, 32, 2, true> : eval_rhs_f32_zmarch_kernel<8, 32, 2, false>)
+                    : zc == 16 ? (w16 ? eval_rhs_f32_zmarch_kernel<8, 16, 2, true> : eval_rhs_f32_zmarch_kernel<8, 16, 2, false>)
+                               : (w16 ? eval_rhs_f32_zmarch_kernel<8, 8, 2, true> : eval_rhs_f32_zmarch_kernel<8, 8, 2, false>);
+        kern<<<grid, block, 0, st>>>(*soln, *rhs, (float)one_over_dx2, k, l, r2);
     }
     return launch_status("eval_rhs");
 }
@@ -726,7 +795,8 @@ int axs_rk4_combine(const axs_fab *dst, const axs_fab *uold, const axs_fab *k1, 
     const int g = grid_rows((int64_t)dst->ny * dst->nz * 4);
     cudaStream_t st = (cudaStream_t)stream;
     if (dst->dtype == AXS_F64)
-        rk4_combine_kernel<double><<<g, 256, 0, st>>>(*dst, *uold, *k1, *k2, *k3, *k4, dt / 6.0, 4);
+        rk4_combine_f64_kernel<<<cell_grid(*dst, 4), 256, 0, st>>>(*dst, *uold, *k1, *k2, *k3, *k4, dt / 6.0,
+                                                                  cell_count(*dst));
     else
         rk4_combine_kernel<float><<<g, 256, 0, st>>>(*dst, *uold, *k1, *k2, *k3, *k4, (float)(dt / 6.0), 4);
     return launch_status("rk4_combine");

@@ -295,3 +295,46 @@ def test_f64_step_on_fields_of_every_exponent_range(axs, orc, kind):
         for c in range(4):
             scale = max(np.abs(ref[c][fin[c]]).max(), 1e-307)
             assert np.abs(got[c] - ref[c])[fin[c]].max() <= 1e-12 * scale, (name, c)
+
+
+@pytest.mark.parametrize("n", [(1, 1, 1), (2, 3, 1), (31, 5, 4), (33, 4, 9), (65, 3, 5), (127, 2, 3)])
+@pytest.mark.parametrize("ng", [2, 3])
+def test_f64_drop_in_kernels_on_rows_of_any_length(axs, orc, n, ng):
+    """The FP64 RHS and the RK4 combination number the cells of the box through:
+    rows shorter and longer than a warp, a box below a block, bit for bit."""
+    nx, ny, nz = n
+    rng = np.random.default_rng(sum(n) + ng)
+    v = rng.standard_normal((4, nz + 2 * ng, ny + 2 * ng, nx + 2 * ng))
+    soln = _to_dev(v)
+    rhs = axs.new_fab(n, 1, dtype=torch.float64)
+    axs.eval_rhs(soln, rhs, ng, 1, 0.3, axs._lib.RhsCoeffs(0.1, 1.3, 0.9))
+    np.testing.assert_array_equal(axs.valid(rhs, 1).cpu().numpy(),
+                                  orc.from_fab(orc.rhs(v, ng, 0.3, 0.1, 1.3, 0.9), ng))
+    ks = [rng.standard_normal((4, nz, ny, nx)) * 10.0 ** rng.integers(-300, 300, (4, nz, ny, nx)) for _ in range(4)]
+    ks[1][0], ks[2][1] = 0.0, 5e-324  # zeros and subnormals, which are doubled by another path
+    ks[1][2, 0, 0, 0], ks[2][2, 0, 0, 0] = np.inf, 1.5e308
+    u = rng.standard_normal((4, nz, ny, nx))
+    d = axs.new_fab(n, ng, dtype=torch.float64)
+    axs.rk4_combine(axs.valid(d, ng), _to_dev(u), *[_to_dev(k) for k in ks], 0, 0.6)
+    with np.errstate(all="ignore"):
+        ref = u + (0.6 / 6.0) * (((ks[0] + 2.0 * ks[1]) + 2.0 * ks[2]) + ks[3])
+    np.testing.assert_array_equal(axs.valid(d, ng).cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("ng", [2, 3])
+def test_f32_rhs_of_part_of_a_box_equals_the_boxs(axs, ng):
+    """The FP32 RHS marches 64 planes a block on a large box and down to 8 on a
+    small one: the same bits for the same cells."""
+    n = (256, 256, 192)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    soln = axs.new_fab(n, ng, dtype=torch.float32)
+    soln.normal_(generator=g)
+    c = axs._lib.RhsCoeffs(0.1, 1.3, 0.9)
+    big = axs.new_fab(n, 0, dtype=torch.float32)
+    axs.eval_rhs(soln, big, ng, 0, 0.5, c)
+    for (x, y, z), (nx, ny, nz) in [((0, 0, 0), (64, 64, 64)), ((32, 8, 5), (128, 128, 77)), ((3, 1, 7), (33, 17, 9)),
+                                    ((64, 0, 100), (160, 200, 92)), ((1, 2, 3), (5, 4, 1))]:
+        part = soln[:, z:z + nz + 2 * ng, y:y + ny + 2 * ng, x:x + nx + 2 * ng]
+        out = axs.new_fab((nx, ny, nz), 1, dtype=torch.float32)
+        axs.eval_rhs(part, out, ng, 1, 0.5, c)
+        assert torch.equal(axs.valid(out, 1), big[:, z:z + nz, y:y + ny, x:x + nx]), (x, y, z, nx, ny, nz)
