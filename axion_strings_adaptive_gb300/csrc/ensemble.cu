@@ -324,7 +324,7 @@ template <int TX, int TY> struct EnsFusedConfig {
         for (int b = 0; b < e->nboxes; ++b) {
             const int nx = e->dims[3 * b], ny = e->dims[3 * b + 1], nz = e->dims[3 * b + 2];
             max_nz = std::max(max_nz, nz);
-            max_row = std::max(max_row, 16 * (ny + 4) + 4 * nx);
+            max_row = std::max(max_row, pad_quads(nx, ny));
         }
         const dim3 pad_grid((unsigned)std::min(64, (max_row + 256 * kPadUnroll - 1) / (256 * kPadUnroll)),
                             (unsigned)std::min(4 * max_nz, 65535), (unsigned)e->nboxes);

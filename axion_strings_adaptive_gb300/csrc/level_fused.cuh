@@ -569,15 +569,19 @@ __global__ void __launch_bounds__(S::THREADS, 1)
 // x = -8 .. -1 and nx .. nx+7 of rows y = -2 .. ny+1, and rows y = -2, -1, ny,
 // ny+1 of columns 0 .. nx-1, each a copy of the valid cell it wraps to. Grid
 // rows are planes (z + nz c); within a plane, consecutive threads take
-// consecutive elements of a padding row, and each thread copies kPadUnroll
-// elements a grid-row stride apart, all loads before the stores (sources are
-// valid cells of `from`, destinations padding: no copy reads another's destination).
+// consecutive quads of a padding row (nx and the layout's offsets are multiples
+// of 4 cells), and each thread copies kPadUnroll quads a grid-row stride apart,
+// all loads before the stores (sources are valid cells of `from`, destinations
+// padding: no copy reads another's destination). Latency-bound: a cell at a
+// time took 1.9 us more of a 128^3 step (48.1 -> 46.2 us; 64^3 17.5 -> 16.5 us).
 constexpr int kPadUnroll = 4;
+__host__ __device__ constexpr int pad_quads(int nx, int ny) { return 4 * (ny + 4) + nx; }  // of a plane
 template <typename T>
 __device__ __forceinline__ void pad_box(T *buf, const T *from, int nx, int ny, int nz, int64_t js, int64_t ks,
                                         int64_t cs, int ox, int oy)
 {
-    const int xpad = 16 * (ny + 4), per_plane = xpad + 4 * nx;
+    using V4 = typename VecN<T, 4>::type;
+    const int xpad = 4 * (ny + 4), per_plane = pad_quads(nx, ny), quads = nx / 4;
     const int stride = gridDim.x * blockDim.x;
     for (int plane = blockIdx.y; plane < 4 * nz; plane += gridDim.y) {
         const int64_t at = (int64_t)(plane / nz) * cs + (int64_t)(plane % nz) * ks + ox + (int64_t)oy * js;
@@ -590,13 +594,13 @@ __device__ __forceinline__ void pad_box(T *buf, const T *from, int nx, int ny, i
             for (int u = 0; u < kPadUnroll; ++u) {
                 const int r = r0 + u * stride;
                 int x, y;
-                if (r < xpad) {  // x padding: 16 columns of every padded row
-                    const int k = r & 15;
-                    x = k < 8 ? k - 8 : nx + (k - 8);
-                    y = (r >> 4) - 2;
+                if (r < xpad) {  // x padding: 4 quads of every padded row
+                    const int k = r & 3;
+                    x = k < 2 ? 4 * k - 8 : nx + 4 * (k - 2);
+                    y = (r >> 2) - 2;
                 } else {  // y padding: 4 rows of the valid columns
-                    const int rr = r - xpad, k = rr / nx;
-                    x = rr - k * nx;
+                    const int rr = r - xpad, k = rr / quads;
+                    x = 4 * (rr - k * quads);
                     y = k < 2 ? k - 2 : ny + (k - 2);
                 }
                 int xs = x < 0 ? x + nx : (x >= nx ? x - nx : x);
@@ -606,12 +610,12 @@ __device__ __forceinline__ void pad_box(T *buf, const T *from, int nx, int ny, i
                 dst[u] = x + (int64_t)y * js;
                 src[u] = on[u] ? xs + (int64_t)ys * js : 0;
             }
-            T v[kPadUnroll];
+            V4 v[kPadUnroll];
 #pragma unroll
-            for (int u = 0; u < kPadUnroll; ++u) v[u] = s[src[u]];
+            for (int u = 0; u < kPadUnroll; ++u) v[u] = *reinterpret_cast<const V4 *>(s + src[u]);
 #pragma unroll
             for (int u = 0; u < kPadUnroll; ++u)
-                if (on[u]) p[dst[u]] = v[u];
+                if (on[u]) *reinterpret_cast<V4 *>(p + dst[u]) = v[u];
         }
     }
 }

@@ -218,7 +218,7 @@ template <int TX, int TY, bool COMP = false> struct FusedConfig {
         int grid = 0;
         plan_chunks(a.ntiles, lv->nz, sms, a.zchunk, a.n_items, grid);
         fill_level_constants(a, lv, g, r.dt);
-        const int pad_per_plane = 16 * (lv->ny + 4) + 4 * lv->nx;
+        const int pad_per_plane = pad_quads(lv->nx, lv->ny);
         const dim3 pad_grid((unsigned)std::min(64, (pad_per_plane + 256 * kPadUnroll - 1) / (256 * kPadUnroll)),
                             (unsigned)std::min(4 * lv->nz, 65535));
         float *buf[2] = {static_cast<float *>(lv->state),
