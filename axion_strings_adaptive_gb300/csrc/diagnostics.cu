@@ -22,6 +22,7 @@
 #include <type_traits>
 
 #include "axs_internal.cuh"
+#include "sweep.cuh"
 #include "winding.cuh"
 
 namespace axs {
@@ -826,40 +827,47 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
 }
 
 // ---------------------------------------------------------------- string finder
-// The string finder and the tagger's plaquette criterion alone (no energy, no
-// velocity). A block owns a FTX x FTY tile of cells, two cells per thread, and
-// marches in z. Each fold decision is made once per edge: the winding of a
-// plaquette is the signed sum of its four edges' folds, #(d < -pi) - #(d > pi)
-// of the edge's phase difference d, and a plaquette walks an edge backwards
-// with exactly -d, so it adds exactly minus the forward fold. That is the
-// single-precision fast path of the fused pass edge for edge, with the same
-// fall back to the reference's double arithmetic: a cell is redone in double
-// when one of its nine edges lies within 1e-5 of +-pi or ends at a vertex
-// outside float range. Those cells are queued in shared memory and redone
-// after the z-chunk, outside the plane loop, so the rare double path costs
-// the loop no registers; a chunk with more than the queue holds is searched
-// again for them. Per vertex plane, with one block barrier:
-//   B: the x and y edge codes of the plane before, from the neighbours' phases;
-//   A: the thread's vertices' phases, from psi loaded into registers two
-//      planes ahead, and their z edges to the plane below (phase kept in a
-//      register);
-//   C: the windings of the cells three planes back.
-// Four slots per vertex-plane array keep every write two barriers from the
-// last read of its slot.
-constexpr int FTX = 32, FTY = 16, FVX = FTX + 1, FVY = FTY + 1;
-constexpr int kFinderExtra = FTX + FTY + 1;  // vertices of the last row (x < FTX) and last column
-constexpr int kFinderListBuf = 3072, kFinderFlushAt = kFinderListBuf - 6 * kDiagThreads;
-constexpr int kFinderBadQ = 1024;  // cells queued for the double path per z-chunk
-static_assert(FTX * FTY == 2 * kDiagThreads && kFinderExtra <= kDiagThreads, "two cells, at most three vertices per thread");
-
+// The string finder and the tagger's plaquette criterion (no energy). A warp owns
+// a strip of kStripW cells in x by kStripRows in y and marches in z: lane l holds
+// the kStripRows + 1 vertices of column x0 + l in registers, the plane before too
+// and the plane after in flight, so there is no shared memory and no barrier in
+// the march. Only two things are asked of an edge a -> b:
+//   - does the short way round cross the negative real axis (the phase difference
+//     folds)? With the vertices' imaginary parts of opposite sign (the sign bit: a
+//     +-0 belongs to its side, as atan2 has it) it does exactly where cross(a, b) =
+//     a1 b2 - a2 b1 has a's sign bit. There the two products have one sign, or a
+//     and b lie within the next test's angle, so the sign is exact, underflow included;
+//   - is it within 1e-5 of antiparallel, |cross| + 1e-5 dot < 0? Then the lane's
+//     cells of that plane take the exact path, as with a vertex outside float range
+//     or not a number: per cell the folds of float phases, or, with an edge within
+//     1e-5 of +-pi, the reference's double arithmetic.
+// The four reduced differences of a plaquette stay below pi each, so its winding is
+// -1, 0 or 1, and it is pierced where an odd number of its edges fold: the folds
+// are bits, row r of the strip in bit r, and the three plaquettes of eight cells
+// come from a few XORs and one shuffle. Columns with pierced cells go to the warp's
+// queue; emptying it, with none of the march's registers live, writes the list entries
+// (one global atomic for 32 columns) and sums gamma^2 v^2 of the corners. Packed FP32
+// pairs are rows r and r + 4.
+// A sixth of the instructions of a phase and three edge codes per vertex in shared memory
+// (66 against 422 million at 320^3), so the march waits for its loads (16 warps an SM at
+// 128 registers; 4 rows a lane with 24 warps took 1.17x as long). 512^3, string finder
+// with its list 1.57 -> 0.60 ms, with velocities and no list 1.79 -> 0.63 ms; white
+// noise (70 % of the cells pierced), 320^3, list: 0.69 -> 0.60 ms.
+constexpr int FTX = 32, FTY = 16;  // energy32_kernel's tile
+static_assert(FTX * FTY == 2 * kDiagThreads, "two cells per thread");
+constexpr int kStripW = 31, kStripRows = 8, kStripPairs = kStripRows / 2;
+constexpr int kStripQueue = 512;  // a warp's queued columns
+constexpr int kFinderBlocks = 2;  // per SM
+static_assert(kStripQueue >= 3 * kStripW && kStripRows <= 8 && kStripRows % 2 == 0,
+              "an empty queue takes three planes' columns; rows are bits of a byte");
+// A lane's column of cells in a plane: pierced xy, yz, zx plaquettes, bit per row, in bits
+// 0-7, 8-15 and 16-23, the lane above; none pierced: to be taken through the exact path.
+struct StripColumn {
+    unsigned pierced;
+    int z;
+};
 struct FinderSmem {
-    long long lbuf[kFinderListBuf];
-    int badq[kFinderBadQ];           // tile-local x | y << 5 | (z - za) << 9
-    float th[4][FVY][FVX];           // phases of vertex plane p in slot p mod 4
-    unsigned char ok[4][FVY][FVX];   // the vertex lies inside float range
-    unsigned char inp[4][FVY][FVX];  // x edge code (bits 0-2), y edge code (bits 3-5)
-    unsigned char zc[4][FVY][FVX];   // z edge code to the plane above (bits 0-2)
-    float gv[4][FVY][FVX];           // gamma^2 v^2 of the vertex (velocity mode)
+    StripColumn queue[kDiagThreads / 32][kStripQueue];
 };
 
 // gamma^2 v^2 at a vertex (Velocity.hpp:62-78 with the prefactors folded on the
@@ -875,6 +883,15 @@ __device__ __forceinline__ float vertex_gv(float psi1, float psi2, float Pi1, fl
     const float re = __fadd_rn(__fmul_rn(phi1, pd1), __fmul_rn(phi2, pd2));
     return __fsub_rn(__fmul_rn(__fmul_rn(pd_sq, q.f_vel_a), __fsub_rn(1.f, __fmul_rn(q.f_vel_b, phi_sq))),
                      __fmul_rn(__fmul_rn(q.f_vel_c, re), re));
+}
+
+// the same at two vertices, to the same bits
+__device__ __forceinline__ F2 vertex_gv(F2 psi1, F2 psi2, F2 Pi1, F2 Pi2, const DiagConst &q)
+{
+    const F2 phi1 = psi1 * F2(q.f_inv_R), phi2 = psi2 * F2(q.f_inv_R);
+    const F2 pd1 = (Pi1 - F2(q.f_RpR) * psi1) * F2(q.f_inv_R2), pd2 = (Pi2 - F2(q.f_RpR) * psi2) * F2(q.f_inv_R2);
+    const F2 phi_sq = phi1 * phi1 + phi2 * phi2, pd_sq = pd1 * pd1 + pd2 * pd2, re = phi1 * pd1 + phi2 * pd2;
+    return (pd_sq * F2(q.f_vel_a)) * (F2(1.f) - F2(q.f_vel_b) * phi_sq) - (F2(q.f_vel_c) * re) * re;
 }
 
 struct CellWindings {
@@ -912,11 +929,10 @@ __device__ __noinline__ CellWindings finder_cell_double(const DiagView v, const 
     return r;
 }
 
-// Whether the finder sends a cell to the double path: one of its seven
-// vertices outside float range, or one of its nine edges inside the band
-// (edge_code's test on the same float phases).
+// A cell whose edges the bits cannot decide: the folds of its float phases or, with an
+// edge in the band of edge_code or a vertex outside float range, the double path.
 template <typename T>
-__device__ __noinline__ bool finder_cell_bad(const DiagView v, const T *base, int x, int y, int z)
+__device__ __noinline__ CellWindings finder_cell_exact(const DiagView &v, const T *base, int x, int y, int z)
 {
     float th[8];
     bool ok[8];
@@ -937,328 +953,396 @@ __device__ __noinline__ bool finder_cell_bad(const DiagView v, const T *base, in
     }
     // corners c = x + 2 y + 4 z; edges x: 0-1, 2-3, 4-5; y: 0-2, 1-3, 4-6; z: 0-4, 1-5, 2-6
     const int ea[9] = {0, 2, 4, 0, 1, 4, 0, 1, 2}, eb[9] = {1, 3, 5, 2, 3, 6, 4, 5, 6};
-    unsigned bad = 0;
+    unsigned code[9], bad = 0;
 #pragma unroll
-    for (int e = 0; e < 9; ++e) bad |= edge_code(th[ea[e]], th[eb[e]], ok[ea[e]] && ok[eb[e]]);
-    return (bad & 4u) != 0;
+    for (int e = 0; e < 9; ++e) bad |= code[e] = edge_code(th[ea[e]], th[eb[e]], ok[ea[e]] && ok[eb[e]]);
+    if (bad & 4u) return finder_cell_double<T>(v, base, x, y, z);
+    // StringFinder.hpp:45-68 order: xy (000 100 110 010), yz (000 010 011 001), zx (000 001 101 100)
+    CellWindings r;
+    r.w[0] = edge_fold(code[0]) + edge_fold(code[4]) - edge_fold(code[1]) - edge_fold(code[3]);
+    r.w[1] = edge_fold(code[3]) + edge_fold(code[8]) - edge_fold(code[5]) - edge_fold(code[6]);
+    r.w[2] = edge_fold(code[6]) + edge_fold(code[2]) - edge_fold(code[7]) - edge_fold(code[0]);
+    r.ties = 0;
+    return r;
 }
 
-// VEL (FP32 fields, beside energy32_kernel): also Pi at the vertices, gamma^2 v^2
-// per vertex and its sum over the corners of every pierced plaquette. Blocks from
-// e_from on clear their partial record's energy sums (energy32_kernel writes those
-// of the blocks below it).
+// Empty a warp's queue of n columns. Written are the list entries (one global atomic for
+// every 32 columns with pierced cells, one for each plaquette of the exact path) and the
+// exact path's tags; returned the lane's part of the exact path's counts and (VEL) of the
+// sum over the corners of every pierced plaquette.
+struct StripCounts {
+    double vsum;
+    int plain, weighted, ties;
+};
+template <typename T> struct StripJob {
+    const T *base;
+    const uint8_t *mask;
+    uint8_t *tags;
+    unsigned long long *list_counter;
+    long long *list;
+    long long capacity;
+    int64_t cell0;  // number of the strip's first cell in plane 0
+    int x0, y0;
+};
 template <typename T, bool VEL>
-__global__ void __launch_bounds__(kDiagThreads, (sizeof(T) == 4 && !VEL) ? 4 : 3)
-    finder_kernel(const DiagView v, const DiagConst q, const uint8_t *__restrict__ mask,
-                  DiagPartial *__restrict__ partials, unsigned long long *__restrict__ list_counter,
-                  long long *__restrict__ list, long long capacity, int tiles_x, int ntiles, int zchunk,
-                  long long n_items, long long items_per_box, int64_t box_stride, uint8_t *__restrict__ tags,
-                  int e_from)
+__device__ __noinline__ StripCounts strip_drain(const DiagView &v, const DiagConst &q, const StripJob<T> &job,
+                                                const StripColumn *queue, int n)
 {
-    extern __shared__ __align__(16) unsigned char finder_smem_raw[];
-    FinderSmem &sm = *reinterpret_cast<FinderSmem *>(finder_smem_raw);
-    __shared__ int lcount, flush_n, badn, bad_over;
-    __shared__ unsigned long long flush_base;
-    __shared__ long long red[kDiagThreads / 32][4];
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int lx = tid % FTX, ly = tid / FTX;  // cells (lx, ly) and (lx, ly + FTY / 2)
-    const int64_t box_cells = (int64_t)v.nx * v.ny * v.nz;
-    int cnt_p = 0, cnt_w = 0, cnt_tie = 0;  // per-thread counts fit 32 bits
-    // velocity mode: corner sums in FP32, a chunk's running sum compensated (Neumaier),
-    // FP64 across chunks (GB300 issues FP64 at 1/64 of the FP32 rate)
-    int cnt_v = 0;
-    double vsum = 0.0;
-    float vacc = 0.f, vcomp = 0.f;
-    auto vadd = [&](float x) {
-        const float t = vacc + x;
-        vcomp += fabsf(vacc) >= fabsf(x) ? (vacc - t) + x : (x - t) + vacc;
-        vacc = t;
-    };
-    if (tid == 0) lcount = badn = bad_over = 0;
-    int warp_end = 0;  // end of this warp's last append to lbuf (lane-uniform)
-    auto flush = [&]() {
-        if (tid == 0) {
-            const int nb = lcount;
-            flush_n = nb;
-            flush_base = nb ? atomicAdd(list_counter, (unsigned long long)nb) : 0ull;
-            lcount = 0;
-        }
-        __syncthreads();
-        const int nb = flush_n;
-        const unsigned long long b0 = flush_base;
-        for (int i = tid; i < nb; i += kDiagThreads)
-            if (b0 + i < (unsigned long long)capacity) list[b0 + i] = sm.lbuf[i];
-        __syncthreads();
-        warp_end = 0;
-    };
-    // a cell of the double path: windings, counts, tag and list entries (one
-    // global atomic each: these cells are rare)
-    auto redo_cell = [&](const T *base, long long qbox, int x, int y, int z) {
-        const CellWindings cw = finder_cell_double<T>(v, base, x, y, z);
-        const int64_t cell = qbox * box_cells + (int64_t)x + (int64_t)v.nx * ((int64_t)y + (int64_t)v.ny * z);
-        cnt_tie += cw.ties;
-        if (tags != nullptr) tags[cell] = (cw.w[0] | cw.w[1] | cw.w[2]) != 0;
-        if constexpr (VEL) {
-            if (cw.w[0] | cw.w[1] | cw.w[2]) {
-                // gamma^2 v^2 at the corners, from global memory (zero outside the ghost region)
-                auto gvat = [&](int dx_, int dy_, int dz_) -> float {
-                    const int xx = x + dx_, yy = y + dy_, zz = z + dz_;
-                    const bool on =
-                        (v.wx || xx < v.nx + v.ox) && (v.wy || yy < v.ny + v.oy) && (v.wz || zz < v.nz + v.oz);
-                    float c4[4];
-                    for (int c = 0; c < 4; ++c) c4[c] = on ? (float)base[view_off<T>(v, c, xx, yy, zz)] : 0.f;
-                    return vertex_gv(c4[0], c4[1], c4[2], c4[3], q);
-                };
-                const float g000 = gvat(0, 0, 0), g100 = gvat(1, 0, 0), g110 = gvat(1, 1, 0), g010 = gvat(0, 1, 0);
-                const float g001 = gvat(0, 0, 1), g101 = gvat(1, 0, 1), g011 = gvat(0, 1, 1);
-                float s_ = 0.f;
-                if (cw.w[0]) { s_ += g000 + g100 + g110 + g010; cnt_v += 4; }
-                if (cw.w[1]) { s_ += g000 + g010 + g011 + g001; cnt_v += 4; }
-                if (cw.w[2]) { s_ += g000 + g001 + g101 + g100; cnt_v += 4; }
-                vadd(s_);
+    const int lane = threadIdx.x & 31;
+    StripCounts r{0.0, 0, 0, 0};
+    // corner sums in FP32, compensated (Neumaier; GB300 issues FP64 at 1/64 of the FP32 rate)
+    float acc = 0.f, comp = 0.f;
+    // VelocityKernel.hpp:37-141: gamma^2 v^2 of the 4 corners of every pierced plaquette of
+    // a column (fields are zero outside the view's ghost region). The warp goes through the
+    // vertex rows that any lane needs together, so that its loads stay row segments.
+    auto velocity = [&](int x, int y0, int z, unsigned pierced) {
+        const int x1 = v.wx && x + 1 == v.nx ? 0 : x + 1, z1 = v.wz && z + 1 == v.nz ? 0 : z + 1;
+        const bool onx = v.wx || x + 1 < v.nx + v.ox, onz = v.wz || z + 1 < v.nz + v.oz;
+        const T *p0 = job.base + x + v.ox + (int64_t)(z + v.oz) * v.ks, *p1 = p0 + (int64_t)(z1 - z) * v.ks;
+        const int64_t right = x1 - x;
+        // vertices (x, y) and (x + 1, y) of plane z (up = 0) or z + 1
+        auto gv = [&](int y, int up) -> F2 {
+            const int yw = v.wy && y == v.ny ? 0 : y;
+            const bool on = (v.wy || y < v.ny + v.oy) && (!up || onz);
+            const T *c = (up ? p1 : p0) + (int64_t)(yw + v.oy) * v.js;
+            F2 f[4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                f[m].v.x = on ? (float)__ldg(c + m * v.cs) : 0.f;
+                f[m].v.y = on && onx ? (float)__ldg(c + m * v.cs + right) : 0.f;
             }
-        }
-#pragma unroll
-        for (int pl = 0; pl < 3; ++pl) {
-            if (!cw.w[pl]) continue;
-            ++cnt_p;
-            cnt_w += abs(cw.w[pl]);
-            if (list != nullptr) {
-                const unsigned long long pos = atomicAdd(list_counter, 1ull);
-                if (pos < (unsigned long long)capacity) list[pos] = 4LL * cell + pl;
-            }
-        }
-    };
-
-    // the thread's vertices: (lx, ly), (lx, ly + 8) and, for the first 49
-    // threads, one of the last row (y = FTY) or the last column (x = FTX)
-    const bool extra = tid < kFinderExtra;
-    const int vi[3] = {lx, lx, tid < FTX ? tid : FTX};
-    const int vj[3] = {ly, ly + FTY / 2, tid < FTX ? FTY : (extra ? tid - FTX : 0)};
-
-    for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
-        const long long qbox = item / items_per_box, box_item = item % items_per_box;
-        const T *__restrict__ base = static_cast<const T *>(v.data) + qbox * box_stride;
-        const int tile = (int)(box_item % ntiles), chunk = (int)(box_item / ntiles);
-        const int x0 = (tile % tiles_x) * FTX, y0 = (tile / tiles_x) * FTY;
-        const int za = chunk * zchunk, len = min(zchunk, v.nz - za);
-
-        // in-plane element offsets of the thread's vertices (the host checks that
-        // a plane's offsets fit 31 bits), -1 outside the ghost region: psi is zero there
-        int voff[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const int xx = x0 + vi[k], yy = y0 + vj[k];
-            const bool on = (k < 2 || extra) && xx <= v.nx && yy <= v.ny && (v.wx || xx < v.nx + v.ox) &&
-                            (v.wy || yy < v.ny + v.oy);
-            voff[k] = on ? (wrap_or_self(xx, v.nx, v.wx) + v.ox) + (wrap_or_self(yy, v.ny, v.wy) + v.oy) * (int)v.js
-                         : -1;
-        }
-        // psi of vertex planes za, za + 1, ... in order, into registers
-        int lz = za, lzw = wrap_or_self(za, v.nz, v.wz);
-        constexpr int NC = VEL ? 4 : 2;  // psi (and Pi) at the vertices
-        auto load_plane = [&](T(&buf)[3][NC]) {
-            const bool zin = v.wz || lz < v.nz + v.oz;
-            const T *pb = base + (int64_t)(lzw + v.oz) * v.ks;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const bool on = zin && voff[k] >= 0;
-#pragma unroll
-                for (int c = 0; c < NC; ++c) buf[k][c] = on ? __ldg(pb + voff[k] + c * v.cs) : T(0);
-            }
-            ++lz;
-            lzw = v.wz ? (lzw + 1 == v.nz ? 0 : lzw + 1) : lzw + 1;
+            return vertex_gv(f[0], f[1], f[2], f[3], q);
         };
-        float thp[3];  // phase and range flag of the vertex one plane down
-        bool okp[3];
-
-        // B: x and y edge codes of vertex plane za + j - 1
-        auto stage_b = [&](int j) {
-            const int s = (j - 1) & 3;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                if (k == 2 && !extra) break;
-                const int i = vi[k], jj = vj[k];
-                unsigned code = 0;
-                if (i < FTX) code = edge_code(thp[k], sm.th[s][jj][i + 1], okp[k] && sm.ok[s][jj][i + 1]);
-                if (jj < FTY) code |= edge_code(thp[k], sm.th[s][jj + 1][i], okp[k] && sm.ok[s][jj + 1][i]) << 3;
-                sm.inp[s][jj][i] = (unsigned char)code;
-            }
-        };
-        // A: phases of vertex plane za + j and the z edges from plane za + j - 1
-        auto stage_a = [&](int j, const T(&buf)[3][NC]) {
-            const int s = j & 3, sp = (j - 1) & 3;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                if (k == 2 && !extra) break;
-                const T a = buf[k][0], b = buf[k][1];
-                bool ok;
-                if constexpr (sizeof(T) == 4) {
-                    const float m = fmaxf(fabsf(a), fabsf(b));
-                    ok = m > 1e-30f && m < 1e30f;
-                } else {
-                    const double m = fmax(fabs(a), fabs(b));
-                    ok = m > 1e-30 && m < 1e30;
+        const unsigned mine = (pierced | pierced >> 8 | pierced >> 16) & 0xffu, vertices = mine | mine << 1;
+        F2 low(0.f), low1(0.f);  // rows k and k + 1, planes z and z + 1
+        for (unsigned rows = __reduce_or_sync(0xffffffffu, vertices); rows; rows &= rows - 1) {
+            const int y = __ffs(rows) - 1, k = y - 1;
+            if (vertices >> y & 1) {
+                const F2 high = gv(y0 + y, 0), high1 = gv(y0 + y, 1);
+                if ((mine << 1) >> y & 1) {
+                    float s = 0.f;  // corners 000 100 110 010, 000 010 011 001, 000 001 101 100
+                    if (pierced >> k & 1) s += low.v.x + low.v.y + high.v.y + high.v.x;
+                    if (pierced >> (8 + k) & 1) s += low.v.x + high.v.x + high1.v.x + low1.v.x;
+                    if (pierced >> (16 + k) & 1) s += low.v.x + low1.v.x + low1.v.y + low.v.y;
+                    const float t = acc + s;
+                    comp += fabsf(acc) >= fabsf(s) ? (acc - t) + s : (s - t) + acc;
+                    acc = t;
                 }
-                const float th = atan2f((float)b, (float)a);
-                sm.th[s][vj[k]][vi[k]] = th;
-                sm.ok[s][vj[k]][vi[k]] = ok;
-                if constexpr (VEL) sm.gv[s][vj[k]][vi[k]] = vertex_gv((float)a, (float)b, (float)buf[k][2], (float)buf[k][3], q);
-                if (j > 0) sm.zc[sp][vj[k]][vi[k]] = (unsigned char)edge_code(thp[k], th, okp[k] && ok);
-                thp[k] = th;
-                okp[k] = ok;
+                low = high;
+                low1 = high1;
             }
-        };
-        // C: windings of the cells of plane za + j - 3
-        auto stage_c = [&](int j) {
-            const int s0 = (j - 3) & 3, s1 = (j - 2) & 3, z = za + j - 3;
-            // cell index of (lx, ly) and the step to (lx, ly + FTY / 2)
-            const int64_t cell0 = qbox * box_cells + (int64_t)(x0 + lx) +
-                                  (int64_t)v.nx * ((int64_t)(y0 + ly) + (int64_t)v.ny * z);
-            const int64_t hstep = (int64_t)v.nx * (FTY / 2);
-            unsigned pm = 0;  // pierced plaquettes: bit 3 h + plane
+        }
+    };
+    for (int i0 = 0; i0 < n; i0 += 32) {
+        const StripColumn e = i0 + lane < n ? queue[i0 + lane] : StripColumn{0u, 0};
+        const unsigned pierced = e.pierced & 0xffffffu;
+        const int dx = e.pierced >> 24;
+        const int64_t plane = (int64_t)v.nx * v.ny;
+        if (job.list != nullptr) {
+            int incl = __popc(pierced);
+            unsigned long long pos = 0;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int cy = ly + h * (FTY / 2), x = x0 + lx, y = y0 + cy;
-                if (!(x < v.nx && y < v.ny)) continue;
-                const int64_t cell = cell0 + h * hstep;
-                if (mask != nullptr && mask[cell] == 0) continue;
-                const unsigned c000 = sm.inp[s0][cy][lx], c100 = sm.inp[s0][cy][lx + 1];
-                const unsigned c010 = sm.inp[s0][cy + 1][lx], c001 = sm.inp[s1][cy][lx];
-                const unsigned z000 = sm.zc[s0][cy][lx], z100 = sm.zc[s0][cy][lx + 1], z010 = sm.zc[s0][cy + 1][lx];
-                const unsigned bad =
-                    ((c000 | c001) & 0x24u) | (c100 & 0x20u) | (c010 & 0x04u) | ((z000 | z100 | z010) & 0x04u);
-                if (bad) {
-                    // the double path after the chunk
-                    const int slot = atomicAdd(&badn, 1);
-                    if (slot < kFinderBadQ)
-                        sm.badq[slot] = lx | (cy << 5) | ((z - za) << 9);
-                    else
-                        bad_over = 1;
-                    continue;
-                }
-                // StringFinder.hpp:45-68 order: xy (000 100 110 010), yz (000 010 011 001), zx (000 001 101 100)
-                const int wxy = edge_fold(c000) + edge_fold(c100 >> 3) - edge_fold(c010) - edge_fold(c000 >> 3);
-                const int wyz = edge_fold(c000 >> 3) + edge_fold(z010) - edge_fold(c001 >> 3) - edge_fold(z000);
-                const int wzx = edge_fold(z000) + edge_fold(c001) - edge_fold(z100) - edge_fold(c000);
-                const unsigned cm = (wxy != 0) | (wyz != 0) << 1 | (wzx != 0) << 2;
-                // StringTagger.hpp:117-151: a cell is tagged when a plaquette at its low corner is pierced
-                if (tags != nullptr) tags[cell] = cm != 0;
-                if constexpr (VEL) {
-                    // VelocityKernel.hpp:37-141: gamma^2 v^2 of the 4 corners of every pierced plaquette
-                    if (cm) {
-                        const float g000 = sm.gv[s0][cy][lx], g100 = sm.gv[s0][cy][lx + 1];
-                        const float g110 = sm.gv[s0][cy + 1][lx + 1], g010 = sm.gv[s0][cy + 1][lx];
-                        const float g001 = sm.gv[s1][cy][lx], g101 = sm.gv[s1][cy][lx + 1];
-                        const float g011 = sm.gv[s1][cy + 1][lx];
-                        float s_ = 0.f;
-                        if (wxy) { s_ += g000 + g100 + g110 + g010; cnt_v += 4; }
-                        if (wyz) { s_ += g000 + g010 + g011 + g001; cnt_v += 4; }
-                        if (wzx) { s_ += g000 + g001 + g101 + g100; cnt_v += 4; }
-                        vadd(s_);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += up;
+            }
+            if (lane == 31 && incl) pos = atomicAdd(job.list_counter, (unsigned long long)incl);
+            pos = __shfl_sync(0xffffffffu, pos, 31) + incl - __popc(pierced);
+            const int64_t cell = job.cell0 + dx + plane * e.z;
+            for (unsigned p = pierced; p; p &= p - 1) {
+                const int b = __ffs(p) - 1;
+                if (pos < (unsigned long long)job.capacity) job.list[pos] = 4 * (cell + (int64_t)v.nx * (b & 7)) + (b >> 3);
+                ++pos;
+            }
+        }
+        // the pierced cells, then the exact path, four columns at a time, a row a lane
+        unsigned exact = __ballot_sync(0xffffffffu, i0 + lane < n && !pierced), some = pierced;
+        int x = job.x0 + dx, y = job.y0, z = e.z;
+        while (true) {
+            if constexpr (VEL) velocity(x, y, z, some);
+            if (!exact) break;
+            unsigned m = exact;
+            for (int i = 0; i < lane / 8; ++i) m &= m - 1;
+            const int src = m ? __ffs(m) - 1 : 0;
+            x = job.x0 + __shfl_sync(0xffffffffu, dx, src);
+            y = job.y0 + (lane & 7);
+            z = __shfl_sync(0xffffffffu, e.z, src);
+            some = 0;
+            const int64_t c = job.cell0 + (x - job.x0) + (int64_t)v.nx * (lane & 7) + plane * z;
+            if (m && y < min(job.y0 + kStripRows, v.ny) && (job.mask == nullptr || job.mask[c] != 0)) {
+                const CellWindings cw = finder_cell_exact<T>(v, job.base, x, y, z);
+                r.ties += cw.ties;
+                for (int pl = 0; pl < 3; ++pl) {
+                    if (cw.w[pl] == 0) continue;
+                    some |= 1u << (8 * pl);
+                    ++r.plain;
+                    r.weighted += abs(cw.w[pl]);
+                    if (job.list != nullptr) {
+                        const unsigned long long at = atomicAdd(job.list_counter, 1ull);
+                        if (at < (unsigned long long)job.capacity) job.list[at] = 4 * c + pl;
                     }
                 }
-                cnt_w += abs(wxy) + abs(wyz) + abs(wzx);
-                pm |= cm << (3 * h);
+                if (job.tags != nullptr) job.tags[c] = some != 0;
             }
-            const int mine = __popc(pm);
-            cnt_p += mine;
-            // pierced plaquettes into the block's buffer: a warp scan and one
-            // shared-memory atomic per warp that has any
-            if (list != nullptr && __any_sync(0xffffffffu, mine != 0)) {
-                int incl = mine;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int yv = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += yv;
-                }
-                const int wtot = __shfl_sync(0xffffffffu, incl, 31);
-                int wbase = 0;
-                if (lane == 31) wbase = atomicAdd(&lcount, wtot);
-                wbase = __shfl_sync(0xffffffffu, wbase, 31);
-                warp_end = wbase + wtot;
-                int pos = wbase + incl - mine;
-                const long long e0 = 4LL * cell0, eh = 4LL * hstep - 3;
-                while (pm) {
-                    const int b = __ffs(pm) - 1;
-                    pm &= pm - 1;
-                    sm.lbuf[pos++] = e0 + b + (b >= 3 ? eh : 0);  // 4 cell + plane
-                }
-            }
-        };
-        // iteration j: B (plane za + j - 1), A (plane za + j, then the load of
-        // plane za + j + 2 into the registers A just read), C (cells of plane
-        // za + j - 3); the loop is unrolled by two so each register buffer has
-        // a fixed name
-        auto step = [&](int j, T(&buf)[3][NC]) {
-            // the plane's one barrier; the block also learns whether the pierced
-            // buffer could overflow during this plane
-            if (__syncthreads_or(warp_end > kFinderFlushAt)) flush();
-            if (j >= 1 && j <= len + 1) stage_b(j);
-            if (j <= len) {
-                stage_a(j, buf);
-                if (j + 2 <= len) load_plane(buf);
-            }
-            if (j >= 3) stage_c(j);
-        };
-        T bufa[3][NC], bufb[3][NC];
-        load_plane(bufa);  // vertex plane za
-        load_plane(bufb);  // za + 1 (len >= 1)
-        for (int j = 0; j < len + 3; j += 2) {
-            step(j, bufa);
-            if (j + 1 < len + 3) step(j + 1, bufb);
-        }
-        // the chunk's double-path cells: from the queue, or, when it overflowed,
-        // by testing every cell of the chunk again
-        __syncthreads();
-        const int nbad = badn;
-        if (!bad_over) {
-            for (int i = tid; i < nbad; i += kDiagThreads) {
-                const int e = sm.badq[i];
-                redo_cell(base, qbox, x0 + (e & 31), y0 + ((e >> 5) & 15), za + (e >> 9));
-            }
-        } else {
-            for (int c = tid; c < FTX * FTY * len; c += kDiagThreads) {
-                const int x = x0 + c % FTX, y = y0 + (c / FTX) % FTY, z = za + c / (FTX * FTY);
-                if (x >= v.nx || y >= v.ny) continue;
-                if (mask != nullptr &&
-                    mask[qbox * box_cells + x + (int64_t)v.nx * ((int64_t)y + (int64_t)v.ny * z)] == 0)
-                    continue;
-                if (finder_cell_bad<T>(v, base, x, y, z)) redo_cell(base, qbox, x, y, z);
-            }
-        }
-        __syncthreads();
-        if (tid == 0) badn = bad_over = 0;  // published by the next chunk's first barrier
-        if constexpr (VEL) {
-            vsum += (double)vacc + (double)vcomp;
-            vacc = vcomp = 0.f;
+            for (int i = 0; i < 4; ++i) exact &= exact - 1;
         }
     }
-    if (list != nullptr && __syncthreads_or(warp_end > 0)) flush();
+    if (VEL) r.vsum = (double)acc + (double)comp;
+    return r;
+}
+
+// psi at the vertices of a lane's column in one plane
+struct StripPlane {
+    F2 a1[kStripPairs], a2[kStripPairs];  // rows k, k + kStripPairs
+    float b1, b2;                         // row kStripRows
+};
+
+// One edge (two, packed): cross and dot products, the antiparallel test into `bad`'s
+// sign bit; the value returned has the sign bit of cross.
+__device__ __forceinline__ float strip_edge(float a1, float n2, float a2, float b1, float b2, unsigned &bad)
+{
+    const float cr = fmaf(a1, b2, n2 * b1), dot = fmaf(a1, b1, a2 * b2);
+    bad |= __float_as_uint(fmaf(1e-5f, dot, fabsf(cr)));
+    return cr;
+}
+__device__ __forceinline__ F2 strip_edge(F2 a1, F2 n2, F2 a2, F2 b1, F2 b2, unsigned &bad)
+{
+    const F2 cr = fma(a1, b2, n2 * b1), e = F2(1e-5f) * fma(a1, b1, a2 * b2);
+    bad |= __float_as_uint(fabsf(cr.v.x) + e.v.x) | __float_as_uint(fabsf(cr.v.y) + e.v.y);
+    return cr;
+}
+// append to `bits` whether an edge folds: imaginary parts of opposite sign, cross of a2's
+__device__ __forceinline__ void strip_fold(unsigned &bits, float a2, float b2, float cr)
+{
+    const unsigned a = __float_as_uint(a2);
+    bits = __funnelshift_l((a ^ __float_as_uint(b2)) & ~(a ^ __float_as_uint(cr)), bits, 1);
+}
+
+// VEL (FP32 fields, beside energy32_kernel): also the sum of gamma^2 v^2 over the
+// corners of every pierced plaquette. Blocks from e_from on clear their partial
+// record's energy sums (energy32_kernel writes those of the blocks below it).
+template <typename T, bool VEL>
+__global__ void __launch_bounds__(kDiagThreads, kFinderBlocks)
+    finder_kernel(const __grid_constant__ DiagView v, const __grid_constant__ DiagConst q,
+                  const uint8_t *__restrict__ mask, DiagPartial *__restrict__ partials,
+                  unsigned long long *__restrict__ list_counter, long long *__restrict__ list, long long capacity,
+                  int strips_x, int strips, int zchunk, long long n_items, long long items_per_box, int64_t box_stride,
+                  uint8_t *__restrict__ tags, int e_from)
+{
+    constexpr int W = kDiagThreads / 32;
+    extern __shared__ __align__(16) unsigned char finder_smem_raw[];
+    __shared__ StripJob<T> jobs[W];
+    __shared__ long long red[W][3];
+    __shared__ double redv[W];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    StripColumn *queue = reinterpret_cast<FinderSmem *>(finder_smem_raw)->queue[warp];
+    int cnt_p = 0, cnt_w = 0, cnt_tie = 0;  // per-thread counts fit 32 bits
+    double vsum = 0.0;
+
+    for (long long item = (long long)blockIdx.x * W + warp; item < n_items; item += (long long)gridDim.x * W) {
+        const long long qbox = item / items_per_box, box_item = item % items_per_box;
+        const T *__restrict__ base = static_cast<const T *>(v.data) + qbox * box_stride;
+        const int strip = (int)(box_item % strips), chunk = (int)(box_item / strips);
+        const int x0 = (strip % strips_x) * kStripW, y0 = (strip / strips_x) * kStripRows;
+        const int za = chunk * zchunk, zend = min(za + zchunk, v.nz);
+        const int64_t cell0 = qbox * v.nx * v.ny * v.nz + x0 + (int64_t)v.nx * y0;
+        const int x = x0 + lane;
+        if (lane == 0) jobs[warp] = StripJob<T>{base, mask, tags, list_counter, list, capacity, cell0, x0, y0};
+        __syncwarp();
+
+        const unsigned valid = lane < kStripW && x < v.nx ? (1u << min(kStripRows, v.ny - y0)) - 1 : 0u;
+
+        // march until the chunk is done or the queue could overflow, then empty the queue with
+        // none of the march's registers live, and go on from there
+        for (int zs = za; zs < zend;) {
+        const int len = zend - zs;
+        // in-plane element offsets of the lane's vertices (the host checks that a plane's
+        // offsets fit 31 bits). Vertices no cell of the strip has repeat the last one;
+        // outside the ghost region psi is zero.
+        int off[kStripRows + 1];
+        unsigned on = 0;  // bit per row
+        const int xv = min(x, v.nx), xw = v.wx && xv == v.nx ? 0 : xv;
+#pragma unroll
+        for (int r = 0; r <= kStripRows; ++r) {
+            const int yv = min(y0 + r, v.ny), yw = v.wy && yv == v.ny ? 0 : yv;
+            const bool in = (v.wx || xv < v.nx + v.ox) && (v.wy || yv < v.ny + v.oy);
+            on |= (unsigned)in << r;
+            off[r] = in ? (xw + v.ox) + (yw + v.oy) * (int)v.js : 0;
+        }
+        const bool all_on = __all_sync(0xffffffffu, on == (2u << kStripRows) - 1);
+        int lz = zs, lzw = zs;  // (zs < nz)
+        auto load = [&](StripPlane &p) {
+            const bool zin = v.wz || lz < v.nz + v.oz;
+            const T *c1 = base + (int64_t)(lzw + v.oz) * v.ks, *c2 = c1 + v.cs;
+            if (all_on && zin) {
+#pragma unroll
+                for (int k = 0; k < kStripPairs; ++k) {
+                    p.a1[k] = F2((float)__ldg(c1 + off[k]), (float)__ldg(c1 + off[k + kStripPairs]));
+                    p.a2[k] = F2((float)__ldg(c2 + off[k]), (float)__ldg(c2 + off[k + kStripPairs]));
+                }
+                p.b1 = (float)__ldg(c1 + off[kStripRows]);
+                p.b2 = (float)__ldg(c2 + off[kStripRows]);
+            } else {
+                auto get = [&](const T *c, int r) { return zin && (on >> r & 1) ? (float)__ldg(c + off[r]) : 0.f; };
+#pragma unroll
+                for (int k = 0; k < kStripPairs; ++k) {
+                    p.a1[k] = F2(get(c1, k), get(c1, k + kStripPairs));
+                    p.a2[k] = F2(get(c2, k), get(c2, k + kStripPairs));
+                }
+                p.b1 = get(c1, kStripRows);
+                p.b2 = get(c2, kStripRows);
+            }
+            ++lz;
+            lzw = v.wz && lz == v.nz ? 0 : lz;
+        };
+
+        int queued = 0;  // warp-uniform
+        unsigned X0 = 0, Y0 = 0, bad0 = 0;  // the plane before: x and y edges that fold; bad: sign bit
+        // plane zs + j in `cur`, the one before in `prev`; the one after is loaded into `next`
+        auto step = [&](int j, const StripPlane &prev, const StripPlane &cur, StripPlane &next) {
+            if (j < len) load(next);
+            F2 n2[kStripPairs];
+            const float nb2 = -cur.b2;
+            int least = INT_MAX, most = 0;  // of |psi|^2's bits: NaN lies above, negative below
+            unsigned bad1 = 0, bz = 0;
+#pragma unroll
+            for (int k = 0; k < kStripPairs; ++k) {
+                n2[k] = F2(-1.f) * cur.a2[k];
+                const F2 s = fma(cur.a1[k], cur.a1[k], cur.a2[k] * cur.a2[k]);
+                least = __vimin3_s32(least, __float_as_int(s.v.x), __float_as_int(s.v.y));
+                most = __vimax3_s32(most, __float_as_int(s.v.x), __float_as_int(s.v.y));
+            }
+            {
+                const int s = __float_as_int(fmaf(cur.b1, cur.b1, cur.b2 * cur.b2));
+                least = min(least, s);
+                most = max(most, s);
+            }
+            const bool outside = least < __float_as_int(1e-36f) || most > __float_as_int(1e36f);
+            // x edges (rows 0 .. 8) and y edges (rows 0 .. 7), row 0 appended last
+            unsigned xl = 0, xh = 0, yl = 0, yh = 0;
+            {
+                const float r1 = __shfl_down_sync(0xffffffffu, cur.b1, 1), r2 = __shfl_down_sync(0xffffffffu, cur.b2, 1);
+                strip_fold(xh, cur.b2, r2, strip_edge(cur.b1, nb2, cur.b2, r1, r2, bad1));
+            }
+#pragma unroll
+            for (int k = kStripPairs - 1; k >= 0; --k) {
+                const F2 a1 = cur.a1[k], a2 = cur.a2[k];
+                F2 r1, r2;
+                r1.v.x = __shfl_down_sync(0xffffffffu, a1.v.x, 1);
+                r1.v.y = __shfl_down_sync(0xffffffffu, a1.v.y, 1);
+                r2.v.x = __shfl_down_sync(0xffffffffu, a2.v.x, 1);
+                r2.v.y = __shfl_down_sync(0xffffffffu, a2.v.y, 1);
+                const F2 cx = strip_edge(a1, n2[k], a2, r1, r2, bad1);
+                strip_fold(xl, a2.v.x, r2.v.x, cx.v.x);
+                strip_fold(xh, a2.v.y, r2.v.y, cx.v.y);
+                const F2 u1 = k + 1 < kStripPairs ? cur.a1[(k + 1) % kStripPairs] : F2(cur.a1[0].v.y, cur.b1);
+                const F2 u2 = k + 1 < kStripPairs ? cur.a2[(k + 1) % kStripPairs] : F2(cur.a2[0].v.y, cur.b2);
+                const F2 cy = strip_edge(a1, n2[k], a2, u1, u2, bad1);
+                strip_fold(yl, a2.v.x, u2.v.x, cy.v.x);
+                strip_fold(yh, a2.v.y, u2.v.y, cy.v.y);
+            }
+            const unsigned X1 = xl | xh << kStripPairs, Y1 = yl | yh << kStripPairs;
+            bad1 |= outside ? 0x80000000u : 0u;
+            if (j > 0) {
+                // z edges to the plane before (rows 0 .. 8)
+                unsigned zl = 0, zh = 0;
+                strip_fold(zh, cur.b2, prev.b2, strip_edge(cur.b1, nb2, cur.b2, prev.b1, prev.b2, bz));
+#pragma unroll
+                for (int k = kStripPairs - 1; k >= 0; --k) {
+                    const F2 cz = strip_edge(cur.a1[k], n2[k], cur.a2[k], prev.a1[k], prev.a2[k], bz);
+                    strip_fold(zl, cur.a2[k].v.x, prev.a2[k].v.x, cz.v.x);
+                    strip_fold(zh, cur.a2[k].v.y, prev.a2[k].v.y, cz.v.y);
+                }
+                const unsigned Z = zl | zh << kStripPairs;
+                // the cells of plane zs + j - 1: this column's bits and the next one's
+                const unsigned mine = Y0 | Z << 8 | ((bad0 | bz | bad1) >> 31) << 17;
+                const unsigned right = __shfl_down_sync(0xffffffffu, mine, 1);
+                unsigned pxy = (X0 ^ X0 >> 1 ^ Y0 ^ right) & valid;
+                unsigned pyz = (Y0 ^ Y1 ^ Z ^ Z >> 1) & valid;
+                unsigned pzx = (Z ^ right >> 8 ^ X0 ^ X1) & valid;
+                const bool inexact = valid != 0 && ((mine | right) >> 17 & 1);
+                if (inexact) pxy = pyz = pzx = 0;
+                unsigned any = pxy | pyz | pzx;
+                if (mask != nullptr || tags != nullptr) {
+                    const int64_t cell = cell0 + lane + (int64_t)v.nx * v.ny * (zs + j - 1);
+                    unsigned keep = 0;
+                    for (int k = 0; k < kStripRows; ++k)
+                        if (valid >> k & 1) keep |= (unsigned)(mask == nullptr || mask[cell + (int64_t)v.nx * k] != 0) << k;
+                    any &= keep;
+                    pxy &= keep;
+                    pyz &= keep;
+                    pzx &= keep;
+                    // StringTagger.hpp:117-151: a cell is tagged when a plaquette at its low corner is pierced
+                    if (tags != nullptr && !inexact)
+                        for (int k = 0; k < kStripRows; ++k)
+                            if (keep >> k & 1) tags[cell + (int64_t)v.nx * k] = any >> k & 1;
+                }
+                cnt_p += __popc(pxy | pyz << 8 | pzx << 16);
+                // queue the pierced cells (where anyone asks which they are), and the column of an inexact lane
+                // queue the lane's column if it is inexact, or pierced where anyone asks which cells are
+                const bool put = inexact || ((VEL || list != nullptr) && any != 0);
+                const unsigned with = __ballot_sync(0xffffffffu, put);
+                if (put)
+                    queue[queued + __popc(with & ((1u << lane) - 1))] =
+                        StripColumn{pxy | pyz << 8 | pzx << 16 | (unsigned)lane << 24, zs + j - 1};
+                queued += __popc(with);
+            }
+            X0 = X1;
+            Y0 = Y1;
+            bad0 = bad1;
+        };
+        StripPlane p0, p1, p2;
+        load(p0);
+        int j = 0;
+        do {
+            step(j, p2, p0, p1);
+            if (j + 1 <= len) step(j + 1, p0, p1, p2);
+            if (j + 2 <= len) step(j + 2, p1, p2, p0);
+            j += 3;
+        } while (j <= len && queued <= kStripQueue - 3 * kStripW);
+        zs += min(j - 1, len);  // the last vertex plane's cells are still to do
+        if (queued) {
+            __syncwarp();
+            const StripCounts c = strip_drain<T, VEL>(v, q, jobs[warp], queue, queued);
+            __syncwarp();
+            vsum += c.vsum;
+            cnt_p += c.plain;
+            cnt_w += c.weighted - c.plain;
+            cnt_tie += c.ties;
+        }
+        }
+        __syncwarp();  // the job record is free
+    }
 
     // ---- block reduction (fixed order) into the fused pass's partial record ----
-    __shared__ double redv[kDiagThreads / 32];
-    long long c4[4] = {cnt_p, cnt_w, VEL ? cnt_v : 0, cnt_tie};
+    long long c3[3] = {cnt_p, cnt_w, cnt_tie};
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        for (int o = 16; o > 0; o >>= 1) c4[s] += __shfl_down_sync(0xffffffffu, c4[s], o);
-        if (lane == 0) red[tid >> 5][s] = c4[s];
+    for (int s = 0; s < 3; ++s) {
+        for (int o = 16; o > 0; o >>= 1) c3[s] += __shfl_down_sync(0xffffffffu, c3[s], o);
+        if (lane == 0) red[warp][s] = c3[s];
     }
     if constexpr (VEL)
         for (int o = 16; o > 0; o >>= 1) vsum += __shfl_down_sync(0xffffffffu, vsum, o);
-    if (lane == 0) redv[tid >> 5] = VEL ? vsum : 0.0;
+    if (lane == 0) redv[warp] = VEL ? vsum : 0.0;
     __syncthreads();
     if (tid < 14) {
         if ((int)blockIdx.x >= e_from) partials[blockIdx.x].e[tid] = 0.0;
     } else if (tid == 14) {
         double xv = 0.0;
-        for (int ww = 0; ww < kDiagThreads / 32; ++ww) xv += redv[ww];
+        for (int ww = 0; ww < W; ++ww) xv += redv[ww];
         partials[blockIdx.x].vsum = xv;
-    } else if (tid >= 32 && tid < 36) {
-        const int f = tid - 32;  // n_p_plain, n_p_weighted, vel_count, near_tie
-        long long xv = 0;
-        for (int ww = 0; ww < kDiagThreads / 32; ++ww) xv += red[ww][f];
-        partials[blockIdx.x].cnt[f] = xv;
+    } else if (tid == 32) {
+        long long np = 0, extra = 0, ties = 0;
+        for (int ww = 0; ww < W; ++ww) {
+            np += red[ww][0];
+            extra += red[ww][1];
+            ties += red[ww][2];
+        }
+        DiagPartial &r = partials[blockIdx.x];
+        r.cnt[0] = np;                   // n_p_plain
+        r.cnt[1] = np + extra;           // n_p_weighted
+        r.cnt[2] = VEL ? 4 * np : 0;     // vel_count: the corners of every pierced plaquette
+        r.cnt[3] = ties;                 // near_tie
     }
 }
 
@@ -1328,7 +1412,7 @@ __device__ __noinline__ CellTerms energy_cell_double(const DiagView v, const Dia
 __global__ void __launch_bounds__(kDiagThreads, 3)
     energy32_kernel(const DiagView v, const DiagConst q, const uint8_t *__restrict__ mask,
                     DiagPartial *__restrict__ partials, int tiles_x, int ntiles, int zchunk, long long n_items,
-                    long long items_per_box, int64_t box_stride, int zero_counts)
+                    long long items_per_box, int64_t box_stride, int cnt_from)
 {
     extern __shared__ __align__(16) unsigned char energy_smem_raw[];
     EnergySmem &sm = *reinterpret_cast<EnergySmem *>(energy_smem_raw);
@@ -1524,9 +1608,9 @@ __global__ void __launch_bounds__(kDiagThreads, 3)
         double xv = 0.0;
         for (int ww = 0; ww < kDiagThreads / 32; ++ww) xv += sm.ew[ww][tid];
         partials[blockIdx.x].e[tid] = xv;
-    } else if (zero_counts && tid == 14) {
+    } else if ((int)blockIdx.x >= cnt_from && tid == 14) {
         partials[blockIdx.x].vsum = 0.0;
-    } else if (zero_counts && tid >= 32 && tid < 36) {
+    } else if ((int)blockIdx.x >= cnt_from && tid >= 32 && tid < 36) {
         partials[blockIdx.x].cnt[tid - 32] = 0;
     }
 }
@@ -1612,6 +1696,37 @@ static void diag_plan(const DiagView &v, int nboxes, int max_grid, int tx, int t
     grid = (int)std::min<long long>(std::min<long long>(items, resident), max_grid);
 }
 
+// The string finder's work items (strip, z-chunk), strip fastest, one warp each: as many
+// chunks as make the fullest warp's planes fewest (a chunk reads one plane more
+// than it has cells, and starts with an empty pipeline).
+struct FinderPlan {
+    int strips_x, strips, zchunk, grid;
+    long long items_per_box, items;
+};
+static FinderPlan finder_plan(const DiagView &v, int nboxes, int max_grid)
+{
+    constexpr int W = kDiagThreads / 32;
+    FinderPlan f;
+    f.strips_x = (v.nx + kStripW - 1) / kStripW;
+    f.strips = f.strips_x * ((v.ny + kStripRows - 1) / kStripRows);
+    const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
+    const long long warps = (long long)std::min(kFinderBlocks * sms, max_grid) * W, all = (long long)f.strips * nboxes;
+    long long best = LLONG_MAX;
+    f.zchunk = v.nz;
+    for (int n = 1; n == 1 || (n <= 64 && v.nz / n >= 4); ++n) {
+        const int len = (v.nz + n - 1) / n, chunks = (v.nz + len - 1) / len;
+        const long long cost = (all * chunks + warps - 1) / warps * (len + 3);
+        if (cost < best) {
+            best = cost;
+            f.zchunk = len;
+        }
+    }
+    f.items_per_box = (long long)f.strips * ((v.nz + f.zchunk - 1) / f.zchunk);
+    f.items = f.items_per_box * nboxes;
+    f.grid = (int)std::min<long long>((f.items + W - 1) / W, std::min(kFinderBlocks * sms, max_grid));
+    return f;
+}
+
 static int64_t diag_scratch_bytes(int64_t ncell) { return 256 + (int64_t)diag_grid(ncell) * sizeof(DiagPartial); }
 
 static int run_diag(const DiagView &v, const axs_diag_params *p, const uint8_t *mask, axs_diag_result *out,
@@ -1675,44 +1790,41 @@ static int run_diag(const DiagView &v, const axs_diag_params *p, const uint8_t *
     long long *lst = (q.want_plaq && capacity > 0) ? reinterpret_cast<long long *>(list) : nullptr;
     int rc0 = AXS_OK;
     const bool offs31 = (int64_t)(v.ny + 2 * v.oy + 2) * v.js < INT_MAX;  // in-plane offsets in 31 bits
+    const FinderPlan f = finder_plan(v, nboxes, diag_grid(ncell));
     auto launch_finder = [&](auto kern, int e_from) -> int {
         AXS_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FinderSmem)));
-        kern<<<grid, kDiagThreads, sizeof(FinderSmem), st>>>(v, q, mask, partials, counter, lst, capacity, tiles_x,
-                                                              ntiles, zchunk, items, items_per_box, box_stride, tags,
-                                                              e_from);
+        kern<<<f.grid, kDiagThreads, sizeof(FinderSmem), st>>>(v, q, mask, partials, counter, lst, capacity, f.strips_x,
+                                                               f.strips, f.zchunk, f.items, f.items_per_box, box_stride,
+                                                               tags, e_from);
         return launch_status("string finder");
     };
     if (q.want_plaq && !q.want_energy && !q.want_vel && offs31) {
-        // windings only: the edge-code finder
-        const bool f32 = v.dtype != AXS_F64;
-        diag_plan(v, nboxes, diag_grid(ncell), FTX, FTY, f32 ? 4 : 3, tiles_x, ntiles, zchunk, items_per_box, items,
-                  grid);
-        rc0 = f32 ? launch_finder(finder_kernel<float, false>, 0) : launch_finder(finder_kernel<double, false>, 0);
+        // windings only
+        rc0 = v.dtype != AXS_F64 ? launch_finder(finder_kernel<float, false>, 0)
+                                 : launch_finder(finder_kernel<double, false>, 0);
         if (rc0) return rc0;
-        diag_finalize_kernel<<<1, 256, 0, st>>>(partials, grid, counter, capacity, lst != nullptr, out);
+        diag_finalize_kernel<<<1, 256, 0, st>>>(partials, f.grid, counter, capacity, lst != nullptr, out);
         return launch_status("diagnostics finalize");
     }
     if (q.want_energy && v.dtype == AXS_F32 && p->per_cell_fp32 && offs31) {
-        // per-cell FP32 terms: the energy sums (3 blocks per SM) and, over the same work
-        // items, the windings, the list and the velocity (4 per SM). Each kernel fills
-        // its own fields of the partial records; the finder clears the energy sums of
-        // the records the energy kernel has no block for.
+        // per-cell FP32 terms: the energy sums (3 blocks per SM) and the windings, the
+        // list and the velocity. Each kernel fills its own fields of the partial records
+        // and clears the other's in those that the other has no block for.
         const bool strings = q.want_plaq || q.want_vel;
-        diag_plan(v, nboxes, diag_grid(ncell), FTX, FTY, q.want_vel ? 3 : 4, tiles_x, ntiles, zchunk, items_per_box,
-                  items, grid);
-        const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
-        const int egrid = strings ? std::min(grid, 3 * sms) : grid;
+        diag_plan(v, nboxes, diag_grid(ncell), FTX, FTY, 3, tiles_x, ntiles, zchunk, items_per_box, items, grid);
         AXS_CUDA_CHECK(
             cudaFuncSetAttribute(energy32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EnergySmem)));
-        energy32_kernel<<<egrid, kDiagThreads, sizeof(EnergySmem), st>>>(v, q, mask, partials, tiles_x, ntiles, zchunk,
-                                                                          items, items_per_box, box_stride, !strings);
+        energy32_kernel<<<grid, kDiagThreads, sizeof(EnergySmem), st>>>(v, q, mask, partials, tiles_x, ntiles, zchunk,
+                                                                         items, items_per_box, box_stride,
+                                                                         strings ? f.grid : 0);
         if ((rc0 = launch_status("energy sums"))) return rc0;
         if (strings) {
-            rc0 = q.want_vel ? launch_finder(finder_kernel<float, true>, egrid)
-                             : launch_finder(finder_kernel<float, false>, egrid);
+            rc0 = q.want_vel ? launch_finder(finder_kernel<float, true>, grid)
+                             : launch_finder(finder_kernel<float, false>, grid);
             if (rc0) return rc0;
         }
-        diag_finalize_kernel<<<1, 256, 0, st>>>(partials, grid, counter, capacity, lst != nullptr, out);
+        diag_finalize_kernel<<<1, 256, 0, st>>>(partials, strings ? std::max(grid, f.grid) : grid, counter, capacity,
+                                                lst != nullptr, out);
         return launch_status("diagnostics finalize");
     }
     diag_plan(v, nboxes, diag_grid(ncell), DTX, DTY, 2, tiles_x, ntiles, zchunk, items_per_box, items, grid);

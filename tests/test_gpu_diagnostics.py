@@ -413,3 +413,36 @@ def test_fp32_fields_in_double_terms_at_every_scale(axs, orc, kind, dx):
     vs, vc = velocity(f, 2, R, rpr, m_r)
     if vc == 4 * r.n_p_plain:  # float and double atan2 agree on every winding
         assert r.vel_count == vc and r.vel_sum == pytest.approx(vs, rel=1e-12)
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(31, 8, 1), (32, 9, 5), (30, 7, 64), (62, 16, 37), (63, 17, 3), (5, 2, 200)])
+@pytest.mark.parametrize("ng", [0, 2])
+def test_finder_strips_of_every_remainder(axs, nx, ny, nz, ng):
+    """The string finder on boxes that leave a cell, a row, a plane or none over
+    from its strips, on white noise and on a smooth field, with and without a
+    mask: the fused pass's counts, near-ties and pierced set; the velocities
+    beside the FP32 energy terms to the rounding of their sums (1e-6)."""
+    rng = np.random.default_rng(nx + ny + nz)
+    x = np.arange(nx) / nx * 2 * np.pi
+    y, z = np.arange(ny) / ny * 2 * np.pi, np.arange(nz) / nz * 2 * np.pi
+    smooth = np.stack(np.broadcast_arrays(np.cos(x)[None, None] + 0.3 * np.sin(z)[:, None, None],
+                                          np.sin(2 * y)[None, :, None] + 0.2 * np.cos(z)[:, None, None],
+                                          np.ones((nz, ny, nx)), np.sin(x)[None, None] * np.ones((nz, ny, 1))))
+    bmode = axs._lib.BOUNDARY_GHOSTS if ng else axs._lib.BOUNDARY_PERIODIC
+    for field in (rng.standard_normal((4, nz, ny, nx)), smooth + 1e-3 * rng.standard_normal((4, nz, ny, nx))):
+        for mask in (None, rng.random((nz, ny, nx)) < 0.5):
+            for dtype in (torch.float32, torch.float64):
+                t = axs.new_fab((nx, ny, nz), ng, dtype=dtype)
+                t.copy_(_dev(np.pad(field, ((0, 0),) + ((ng, ng),) * 3, mode="wrap"), dtype))
+                par = lambda e, s, v, f32: axs._lib.DiagParams(0.5, 1.3, 2.0, 0.4, 1.0, 1, 0.8, bmode, e, s, v, f32)
+                full, pierced = _run_diag(axs, t, ng, par(1, 1, 1, 0), mask)
+                runs = [par(0, 1, 0, 0)] + ([par(1, 1, 1, 1)] if dtype == torch.float32 else [])
+                for p in runs:
+                    got, lst = _run_diag(axs, t, ng, p, mask)
+                    assert got.status == 0
+                    assert (got.n_p_plain, got.n_p_weighted, got.n_near_tie) == \
+                        (full.n_p_plain, full.n_p_weighted, full.n_near_tie)
+                    np.testing.assert_array_equal(np.sort(lst), np.sort(pierced))
+                if len(runs) == 2:
+                    assert got.vel_count == full.vel_count
+                    assert got.vel_sum == pytest.approx(full.vel_sum, rel=1e-6, abs=1e-6 * max(1, full.vel_count))
