@@ -251,6 +251,54 @@ __device__ __forceinline__ void cell_energy(const CellConst<float> &k, int schem
     }
 }
 
+// The float version for two cells at once, to the same bits: the scalar one's roundings,
+// with its sums of products fused as the compiler fuses them.
+__device__ __forceinline__ F2 neg(F2 a) { return F2(-a.v.x, -a.v.y); }
+__device__ __forceinline__ F2 diff1_pair(F2 m2, F2 p2, F2 p1, F2 m1, float inv_dx)
+{
+    const float wf = 0.0833333333f, wn = 0.666666667f;
+    return fma(F2(wf), m2 - p2, F2(wn) * (p1 - m1)) * F2(inv_dx);
+}
+__device__ __forceinline__ void cell_energy(const CellConst<float> &k, int scheme, F2 psi1, F2 psi2, F2 Pi1, F2 Pi2,
+                                            const F2 (&g)[2][3], F2 (&term)[6], F2 &wgt)
+{
+    const F2 psi_sq = fma(psi1, psi1, psi2 * psi2);
+    F2 g1sq = g[0][0] * g[0][0], g2sq = g[1][0] * g[1][0], cross2;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        if (d) {
+            g1sq = fma(g[0][d], g[0][d], g1sq);
+            g2sq = fma(g[1][d], g[1][d], g2sq);
+        }
+        const F2 cr = fma(psi1, g[1][d], neg(psi2 * g[0][d]));
+        cross2 = d ? fma(cr, cr, cross2) : cr * cr;
+    }
+    const F2 inv_psq(psi_sq.v.x > 0.f ? 1.f / psi_sq.v.x : 0.f, psi_sq.v.y > 0.f ? 1.f / psi_sq.v.y : 0.f);
+    const F2 gtsq = (cross2 * inv_psq) * inv_psq;
+    const F2 c1 = fma(F2(-k.RpR), psi1, Pi1), c2 = fma(F2(-k.RpR), psi2, Pi2);
+    const F2 dsq = psi_sq - F2(k.R2);
+    const F2 pot = (F2(0.25f * k.lambda) * dsq) * dsq;
+    const F2 gsq = g1sq + g2sq;
+    term[0] = ((fma(c1, c1, c2 * c2) + gsq) + pot) * F2(k.inv_R4);
+    const F2 thp = fma(psi1, Pi2, neg(Pi1 * psi2)) * inv_psq;
+    term[1] = (thp * thp) * F2(k.inv_R2);
+    term[2] = gtsq * F2(k.inv_R2);
+    const F2 rdot = fma(psi1, c1, psi2 * c2);
+    term[3] = ((rdot * rdot) * inv_psq) * F2(k.inv_R4);
+    term[4] = fma(neg(psi_sq), gtsq, gsq) * F2(k.inv_R4);
+    term[5] = pot * F2(k.inv_R4);
+    wgt = F2(1.f);
+    if (scheme != AXS_MASK_NONE) {
+        const F2 mod = F2(sqrtf(psi_sq.v.x), sqrtf(psi_sq.v.y)) * F2(k.inv_R);
+        if (scheme == AXS_MASK_B) {
+            wgt = F2(mod.v.x >= k.threshold ? 1.f : 0.f, mod.v.y >= k.threshold ? 1.f : 0.f);
+        } else {
+            const F2 f = fma(mod + F2(-1.f), F2(0.70710678118654752440f), F2(1.f));
+            wgt = f * f;
+        }
+    }
+}
+
 // In double, from the diff1 values g and the same in the field precision, gt
 // (the reference squares them there). RAW: without the powers of 1/R, which the
 // caller puts on the sums (six FP64 operations a cell).
@@ -1348,24 +1396,27 @@ __global__ void __launch_bounds__(kDiagThreads, kFinderBlocks)
 
 // ---------------------------------------------------------------- FP32 per-cell energy sums
 // The per_cell_fp32 energy sums on FP32 fields, run beside finder_kernel<float, VEL>
-// (windings, the pierced list and the velocity), each kernel with few registers.
-// A block owns a FTX x FTY tile, two cells per thread, and marches in z. psi of the
-// tile plus a 2-cell halo arrives by cp.async in a ring of seven planes (the
-// gradient stencil's five plus two, so one block barrier per plane suffices), Pi
-// of the tile in a ring of three. Per plane each warp adds up its cells' 13 terms
-// in FP32 with a butterfly over the lanes, and lane k adds sum k to a compensated
-// (Neumaier) FP32 accumulator, lane 13 the cell count. After each z-chunk the
-// accumulators go to per-warp FP64 slots. Cells where FP32 cannot hold 1/|psi|^4
-// (|psi|^2 outside (1e-15, 1e15): the cores' exact zeros) are queued and take the
-// reference's double arithmetic after the chunk, as the fused pass does.
-constexpr int EHX = FTX + 4, EHY = FTY + 4, kEnergySlots = 7, kEnergyPiSlots = 3, kEnergyBadQ = 1024;
-constexpr int kEnergyPts = 2 * EHX * EHY, kEnergyPer = (kEnergyPts + kDiagThreads - 1) / kDiagThreads;
-constexpr int kEnergyPiPts = 2 * FTX * FTY, kEnergyPiPer = kEnergyPiPts / kDiagThreads;
-static_assert(kEnergyPiPts % kDiagThreads == 0, "Pi loads per thread");
+// (windings, the pierced list and the velocity). A block owns a FTX x FTY tile, two
+// cells per thread FTY / 2 rows apart, packed, and marches in z. psi of the tile
+// plus a 2-cell halo arrives by cp.async in a ring of five planes: the current one, whose
+// rows the x and y stencils read, the one two above, whose centre goes to the
+// thread's column of five planes in registers, the two on the way, and one that a
+// slower warp may still read (one block barrier per plane). Pi comes to registers a plane
+// ahead. Per plane the warp's sums of its cells' 13 terms and of their count end on a
+// lane each (15 exchanges that halve what a lane holds), which adds them to a
+// compensated (Neumaier) FP32 accumulator. After each z-chunk the accumulators go to per-warp FP64 slots. Cells
+// where FP32 cannot hold 1/|psi|^4 (|psi|^2 outside (1e-15, 1e15): the cores' exact
+// zeros) are queued and take the reference's double arithmetic after the chunk, as the
+// fused pass does. VEC: rows, strides and the tile's origin allow 8-byte copies.
+// Bound by instruction issue. 512^3: 1.68 -> 0.93 ms (scalar cells, z taps from shared
+// memory, 4-byte copies, a full butterfly of each of the 14 sums: 380 instructions a
+// cell). Two cells next to each other in x, their sums over five planes first, took
+// 0.77 ms, but FP32 partial sums in another order move small boxes' sums by 5e-9.
+constexpr int EHX = FTX + 4, EHY = FTY + 4, kEnergySlots = 5, kEnergyBadQ = 1024;
+constexpr int kEnergyPts = 2 * EHX * EHY;
 struct EnergySmem {
     double ew[kDiagThreads / 32][14];
     float ps[kEnergySlots][2][EHY][EHX];
-    float pi[kEnergyPiSlots][2][FTY][FTX];
     int badq[kEnergyBadQ];  // tile-local x | y << 5 | (z - za) << 9
 };
 
@@ -1409,21 +1460,44 @@ __device__ __noinline__ CellTerms energy_cell_double(const DiagView v, const Dia
     return r;
 }
 
-__global__ void __launch_bounds__(kDiagThreads, 3)
-    energy32_kernel(const DiagView v, const DiagConst q, const uint8_t *__restrict__ mask,
-                    DiagPartial *__restrict__ partials, int tiles_x, int ntiles, int zchunk, long long n_items,
-                    long long items_per_box, int64_t box_stride, int cnt_from)
+// The warp's sums of v[0 .. 13]: lane l returns that of k = 7 b4 + 4 b3 + 2 b2 + b1 of its
+// bits (b3 b2 b1 = 7: none), added up in the order of a butterfly from 16 down.
+__device__ __forceinline__ float warp_sums14(const float (&v)[14], int lane)
 {
-    extern __shared__ __align__(16) unsigned char energy_smem_raw[];
-    EnergySmem &sm = *reinterpret_cast<EnergySmem *>(energy_smem_raw);
+    auto fold = [&](float lo, float hi, int o) {
+        const bool up = lane & o;
+        return (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, o);
+    };
+    float a[7], b[4];
+#pragma unroll
+    for (int i = 0; i < 7; ++i) a[i] = fold(v[i], v[i + 7], 16);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) b[i] = fold(a[i], i < 3 ? a[i + 4] : 0.f, 8);
+    const float c0 = fold(b[0], b[2], 4), c1 = fold(b[1], b[3], 4), d = fold(c0, c1, 2);
+    return d + __shfl_xor_sync(0xffffffffu, d, 1);
+}
+
+constexpr int kEnergyBlocks = 3;  // per SM: 80 registers (64 and 128 took 1.10x as long)
+template <bool VEC>
+__global__ void __launch_bounds__(kDiagThreads, kEnergyBlocks)
+    energy32_kernel(const __grid_constant__ DiagView v, const __grid_constant__ DiagConst q,
+                    const uint8_t *__restrict__ mask, DiagPartial *__restrict__ partials, int tiles_x, int ntiles,
+                    int zchunk, long long n_items, long long items_per_box, int64_t box_stride, int cnt_from)
+{
+    __shared__ __align__(16) EnergySmem sm;
     __shared__ int badn, bad_over;
+    constexpr int EN = VEC ? 2 : 1;  // elements per copy
+    constexpr int PER = (kEnergyPts / EN + kDiagThreads - 1) / kDiagThreads;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int lx = tid % FTX, ly = tid / FTX;  // cells (lx, ly) and (lx, ly + FTY / 2)
+    constexpr int HALF = FTY / 2;
+    const int lx = tid % FTX, ly = tid / FTX;                // cells (lx, ly) and (lx, ly + HALF)
+    const int sum_of = 7 * (lane >> 4) + ((lane >> 1) & 7);  // the sum the lane keeps
+    const bool keeps = (lane & 1) == 0 && (lane & 14) != 14;
     const int64_t box_cells = (int64_t)v.nx * v.ny * v.nz;
     const CellConst<float> kf{q.f_R2, q.f_inv_R, q.f_inv_R2, q.f_inv_R4, q.f_lambda, q.f_RpR, q.f_threshold};
     for (int i = tid; i < (kDiagThreads / 32) * 14; i += kDiagThreads) sm.ew[i / 14][i % 14] = 0.0;
     if (tid == 0) badn = bad_over = 0;
-    float acc = 0.f, comp = 0.f;  // lane k < 13: running sum k of the chunk; lane 13: its cell count
+    float acc = 0.f, comp = 0.f;  // running sum of the chunk (13: its cell count, exact)
 
     for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
         const long long qbox = item / items_per_box, box_item = item % items_per_box;
@@ -1431,136 +1505,151 @@ __global__ void __launch_bounds__(kDiagThreads, 3)
         const int tile = (int)(box_item % ntiles), chunk = (int)(box_item / ntiles);
         const int x0 = (tile % tiles_x) * FTX, y0 = (tile / tiles_x) * FTY;
         const int za = chunk * zchunk, len = min(zchunk, v.nz - za);
+        const int x = x0 + lx, y = y0 + ly;
 
-        // load plans (in-plane offsets in 31 bits, checked on the host; -1: zero fill)
-        int poff[kEnergyPer];
+        // load plan: offsets in a plane of both components; elements outside the view's
+        // ghost region, and those no cell needs, are zero
+        int64_t poff[PER];
+        unsigned on = 0;
 #pragma unroll
-        for (int u = 0; u < kEnergyPer; ++u) {
-            const int idx = tid + u * kDiagThreads, r = idx % (EHX * EHY);
+        for (int u = 0; u < PER; ++u) {
+            const int e = (tid + u * kDiagThreads) * EN, r = e % (EHX * EHY);
             const int xx = x0 - 2 + r % EHX, yy = y0 - 2 + r / EHX;
-            const bool on = idx < kEnergyPts && xx < v.nx + 2 && yy < v.ny + 2 &&
+            const bool in = e < kEnergyPts && xx < v.nx + 2 && yy < v.ny + 2 &&
                             (v.wx || (xx >= -v.ox && xx < v.nx + v.ox)) && (v.wy || (yy >= -v.oy && yy < v.ny + v.oy));
-            poff[u] = on ? (wrap_or_self(xx, v.nx, v.wx) + v.ox) + (wrap_or_self(yy, v.ny, v.wy) + v.oy) * (int)v.js
-                         : -1;
+            on |= (unsigned)in << u;
+            poff[u] = in ? (wrap_or_self(xx, v.nx, v.wx) + v.ox) + (wrap_or_self(yy, v.ny, v.wy) + v.oy) * v.js +
+                               (e >= EHX * EHY ? v.cs : 0)
+                         : 0;
         }
-        int qoff[kEnergyPiPer];
-#pragma unroll
-        for (int u = 0; u < kEnergyPiPer; ++u) {
-            const int idx = tid + u * kDiagThreads, r = idx % (FTX * FTY);
-            const int xx = x0 + r % FTX, yy = y0 + r / FTX;
-            qoff[u] = xx < v.nx && yy < v.ny ? (xx + v.ox) + (yy + v.oy) * (int)v.js : -1;
-        }
-        // psi planes za - 2 .. za + len + 1 (plane p in slot (p - za + 2) mod 7), Pi planes
-        // za .. za + len - 1 (slot (p - za) mod 3), each loaded in order
+        // psi planes za - 2, ... in order (plane p in slot (p - za + 2) mod 5)
         int lz = za - 2, lzw = wrap_or_self(za - 2, v.nz, v.wz);
-        auto load_psi_next = [&]() {
+        auto load_psi_next = [&](int slot) {
             const bool zin = v.wz || (lz >= -v.oz && lz < v.nz + v.oz);
-            const float *pb = base + (int64_t)(lzw + v.oz) * v.ks;
-            float *dst = &sm.ps[(lz - za + 2) % kEnergySlots][0][0][0];
+            const float *pb = zin ? base + (int64_t)(lzw + v.oz) * v.ks : base;
+            float *dst = &sm.ps[slot][0][0][0];
 #pragma unroll
-            for (int u = 0; u < kEnergyPer; ++u) {
-                const int idx = tid + u * kDiagThreads;
-                if (idx < kEnergyPts)
-                    cp_async_elem(dst + idx, pb + (idx >= EHX * EHY ? v.cs : 0) + poff[u], zin && poff[u] >= 0, base);
+            for (int u = 0; u < PER; ++u) {
+                const int e = (tid + u * kDiagThreads) * EN;
+                const float *src = pb + poff[u];
+                const bool in = zin && (on >> u & 1);
+                if (e < kEnergyPts) {
+                    if constexpr (VEC)
+                        cp_async_elem(reinterpret_cast<float2 *>(dst + e), reinterpret_cast<const float2 *>(src), in,
+                                      reinterpret_cast<const float2 *>(src));
+                    else
+                        cp_async_elem(dst + e, src, in, src);
+                }
             }
             ++lz;
             lzw = v.wz ? (lzw + 1 == v.nz ? 0 : lzw + 1) : lzw + 1;
         };
-        int pz = za, pzw = wrap_or_self(za, v.nz, v.wz);
+        // Pi of the thread's cells, plane za on
+        const unsigned valid = x < v.nx ? (unsigned)(y < v.ny) | (unsigned)(y + HALF < v.ny) << 1 : 0u;
+        const float *pi_at = base + (valid ? (x + v.ox) + (int64_t)(y + v.oy) * v.js : 0) + (int64_t)(za + v.oz) * v.ks +
+                             2 * v.cs;
+        F2 pi_next[2];
         auto load_pi_next = [&]() {
-            const float *pb = base + (int64_t)(pzw + v.oz) * v.ks + 2 * v.cs;
-            float *dst = &sm.pi[(pz - za) % kEnergyPiSlots][0][0][0];
 #pragma unroll
-            for (int u = 0; u < kEnergyPiPer; ++u) {
-                const int idx = tid + u * kDiagThreads;
-                cp_async_elem(dst + idx, pb + (idx >= FTX * FTY ? v.cs : 0) + qoff[u], qoff[u] >= 0, base);
-            }
-            ++pz;
-            pzw = v.wz ? (pzw + 1 == v.nz ? 0 : pzw + 1) : pzw + 1;
+            for (int c = 0; c < 2; ++c)
+                pi_next[c] = F2(valid & 1 ? __ldg(pi_at + c * v.cs) : 0.f,
+                                valid & 2 ? __ldg(pi_at + c * v.cs + HALF * v.js) : 0.f);
+            pi_at += v.ks;
         };
-        for (int p = 0; p < 5; ++p) load_psi_next();  // za - 2 .. za + 2
-        load_pi_next();                               // za
+        auto pair_at = [&](int slot, int c, int yy, int xx) {
+            return F2(sm.ps[slot][c][yy][xx], sm.ps[slot][c][yy + HALF][xx]);
+        };
+        for (int p = 0; p < 5; ++p) load_psi_next(p);  // za - 2 .. za + 2
         cp_async_commit();
+        load_pi_next();  // za
+        cp_async_wait<0>();
+        __syncthreads();
+        const int hx = lx + 2, hy = ly + 2;
+        F2 col[2][5];  // psi of planes z - 2 .. z + 2, by slot
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int p = 0; p < 4; ++p) col[c][p] = pair_at(p, c, hy, hx);
+        __syncthreads();  // slot 0 is loaded again
 
-        for (int m = 0; m < len; ++m) {
-            const int z = za + m;
-            // one plane ahead: psi(z + 3), Pi(z + 1); their slots were last read two planes back
+        // plane za + m, m mod 5 = I
+        auto step = [&](auto I, int m) {
+            constexpr int i = decltype(I)::value, s0 = (i + 2) % 5, m2 = i, m1 = (i + 1) % 5, p1 = (i + 3) % 5,
+                          p2 = (i + 4) % 5;
+            const F2 pi1 = pi_next[0], pi2 = pi_next[1];
+            // one plane ahead: psi(z + 3), Pi(z + 1)
             if (m + 1 < len) {
-                load_psi_next();
+                load_psi_next(i);
                 load_pi_next();
             }
             cp_async_commit();
-            cp_async_wait<1>();  // psi(z + 2), Pi(z)
+            cp_async_wait<1>();  // psi(z + 2)
             __syncthreads();
-            const int s0 = (m + 2) % kEnergySlots, sm1 = (m + 1) % kEnergySlots, sp1 = (m + 3) % kEnergySlots,
-                      sm2 = m % kEnergySlots, sp2 = (m + 4) % kEnergySlots, tp = m % kEnergyPiSlots;
-            float ts[13];
+            F2 g[2][3];
 #pragma unroll
-            for (int k = 0; k < 13; ++k) ts[k] = 0.f;
-            int ncell = 0;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int cy = ly + h * (FTY / 2), x = x0 + lx, y = y0 + cy;
-                if (!(x < v.nx && y < v.ny)) continue;
-                if (mask != nullptr &&
-                    mask[qbox * box_cells + (int64_t)x + (int64_t)v.nx * ((int64_t)y + (int64_t)v.ny * z)] == 0)
-                    continue;
-                const int hx = lx + 2, hy = cy + 2;
-                const float p1 = sm.ps[s0][0][hy][hx], p2 = sm.ps[s0][1][hy][hx];
-                const float psq = p1 * p1 + p2 * p2;
-                if (!(psq > 1e-15f && psq < 1e15f)) {
-                    // the double path after the chunk
-                    const int slot = atomicAdd(&badn, 1);
-                    if (slot < kEnergyBadQ)
-                        sm.badq[slot] = lx | (cy << 5) | ((z - za) << 9);
-                    else
-                        bad_over = 1;
-                    continue;
-                }
-                float g[2][3];
-                const float wf = 0.0833333333f, wn = 0.666666667f;
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    g[c][0] = (wf * (sm.ps[s0][c][hy][hx - 2] - sm.ps[s0][c][hy][hx + 2]) +
-                               wn * (sm.ps[s0][c][hy][hx + 1] - sm.ps[s0][c][hy][hx - 1])) * q.f_one_over_dx;
-                    g[c][1] = (wf * (sm.ps[s0][c][hy - 2][hx] - sm.ps[s0][c][hy + 2][hx]) +
-                               wn * (sm.ps[s0][c][hy + 1][hx] - sm.ps[s0][c][hy - 1][hx])) * q.f_one_over_dx;
-                    g[c][2] = (wf * (sm.ps[sm2][c][hy][hx] - sm.ps[sp2][c][hy][hx]) +
-                               wn * (sm.ps[sp1][c][hy][hx] - sm.ps[sm1][c][hy][hx])) * q.f_one_over_dx;
-                }
-                float term[6], wgt;
-                cell_energy(kf, q.scheme, p1, p2, sm.pi[tp][0][cy][lx], sm.pi[tp][1][cy][lx], g,
-                                          term, wgt);
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    ts[2 * k] += term[k];
-                    ts[2 * k + 1] += term[k] * wgt;
-                }
-                ts[12] += wgt;
-                ++ncell;
+            for (int c = 0; c < 2; ++c) {
+                col[c][p2] = pair_at(p2, c, hy, hx);
+                g[c][0] = diff1_pair(pair_at(s0, c, hy, hx - 2), pair_at(s0, c, hy, hx + 2),
+                                     pair_at(s0, c, hy, hx + 1), pair_at(s0, c, hy, hx - 1), q.f_one_over_dx);
+                g[c][1] = diff1_pair(pair_at(s0, c, hy - 2, hx), pair_at(s0, c, hy + 2, hx),
+                                     pair_at(s0, c, hy + 1, hx), pair_at(s0, c, hy - 1, hx), q.f_one_over_dx);
+                g[c][2] = diff1_pair(col[c][m2], col[c][p2], col[c][p1], col[c][m1], q.f_one_over_dx);
             }
-            // the warp's sums of this plane (butterfly), then lane k's compensated accumulator
+            const F2 f1 = col[0][s0], f2 = col[1][s0], psq = fma(f1, f1, f2 * f2);
+            const bool in0 = psq.v.x > 1e-15f && psq.v.x < 1e15f, in1 = psq.v.y > 1e-15f && psq.v.y < 1e15f;
+            F2 term[6], wgt;
+            cell_energy(kf, q.scheme, f1, f2, pi1, pi2, g, term, wgt);
+            float cells = 2.f;
+            if (!__all_sync(0xffffffffu, valid == 3u && in0 && in1 && mask == nullptr)) {
+                unsigned take = valid;
+                if (mask != nullptr) {
+                    const uint8_t *mc = mask + qbox * box_cells + x + (int64_t)v.nx * ((int64_t)y + (int64_t)v.ny * (za + m));
+                    if ((take & 1) && mc[0] == 0) take &= ~1u;
+                    if ((take & 2) && mc[(int64_t)HALF * v.nx] == 0) take &= ~2u;
+                }
 #pragma unroll
-            for (int k = 0; k < 13; ++k)
+                for (int h = 0; h < 2; ++h)
+                    if ((take >> h & 1) && !(h ? in1 : in0)) {
+                        // the double path after the chunk
+                        take &= ~(1u << h);
+                        const int slot = atomicAdd(&badn, 1);
+                        if (slot < kEnergyBadQ)
+                            sm.badq[slot] = lx | ((ly + h * HALF) << 5) | (m << 9);
+                        else
+                            bad_over = 1;
+                    }
+                auto drop = [&](F2 &f) {
+                    if (!(take & 1)) f.v.x = 0.f;
+                    if (!(take & 2)) f.v.y = 0.f;
+                };
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) ts[k] += __shfl_xor_sync(0xffffffffu, ts[k], o);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ncell += __shfl_xor_sync(0xffffffffu, ncell, o);
-            float mine = (float)ncell;
-#pragma unroll
-            for (int k = 0; k < 13; ++k)
-                if (lane == k) mine = ts[k];
-            if (lane < 13) {
-                const float t = acc + mine;
-                comp += fabsf(acc) >= fabsf(mine) ? (acc - t) + mine : (mine - t) + acc;
-                acc = t;
-            } else if (lane == 13) {
-                acc += mine;  // cell counts stay exact in float: at most 512 per plane, 2^24 per chunk
+                for (int k = 0; k < 6; ++k) drop(term[k]);
+                drop(wgt);
+                cells = (float)__popc(take);
             }
+            float ts[14];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                ts[2 * k] = term[k].v.x + term[k].v.y;
+                ts[2 * k + 1] = fmaf(term[k].v.y, wgt.v.y, term[k].v.x * wgt.v.x);
+            }
+            ts[12] = wgt.v.x + wgt.v.y;
+            ts[13] = cells;
+            const float mine = warp_sums14(ts, lane), t = acc + mine;
+            comp += fabsf(acc) >= fabsf(mine) ? (acc - t) + mine : (mine - t) + acc;
+            acc = t;
+        };
+        for (int m = 0; m < len; m += 5) {
+            step(std::integral_constant<int, 0>(), m);
+            if (m + 1 < len) step(std::integral_constant<int, 1>(), m + 1);
+            if (m + 2 < len) step(std::integral_constant<int, 2>(), m + 2);
+            if (m + 3 < len) step(std::integral_constant<int, 3>(), m + 3);
+            if (m + 4 < len) step(std::integral_constant<int, 4>(), m + 4);
         }
         __syncthreads();  // the queue is complete; the rings are free for the next chunk
-        if (lane < 14) sm.ew[warp][lane] += (double)acc + (double)comp;
+        if (keeps) sm.ew[warp][sum_of] += (double)acc + (double)comp;
         acc = comp = 0.f;
+        __syncwarp();  // the double path adds to the same sums
         // the chunk's double-path cells: from the queue or, when it overflowed, by testing
         // every cell again; each warp sums its cells' terms and lane k adds sum k
         const int nbad = badn;
@@ -1811,12 +1900,10 @@ static int run_diag(const DiagView &v, const axs_diag_params *p, const uint8_t *
         // list and the velocity. Each kernel fills its own fields of the partial records
         // and clears the other's in those that the other has no block for.
         const bool strings = q.want_plaq || q.want_vel;
-        diag_plan(v, nboxes, diag_grid(ncell), FTX, FTY, 3, tiles_x, ntiles, zchunk, items_per_box, items, grid);
-        AXS_CUDA_CHECK(
-            cudaFuncSetAttribute(energy32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EnergySmem)));
-        energy32_kernel<<<grid, kDiagThreads, sizeof(EnergySmem), st>>>(v, q, mask, partials, tiles_x, ntiles, zchunk,
-                                                                         items, items_per_box, box_stride,
-                                                                         strings ? f.grid : 0);
+        diag_plan(v, nboxes, diag_grid(ncell), FTX, FTY, kEnergyBlocks, tiles_x, ntiles, zchunk, items_per_box, items, grid);
+        const bool vec = (uintptr_t)v.data % 8 == 0 && (v.nx | v.ox | v.js | v.ks | v.cs | box_stride) % 2 == 0;
+        (vec ? energy32_kernel<true> : energy32_kernel<false>)<<<grid, kDiagThreads, 0, st>>>(
+            v, q, mask, partials, tiles_x, ntiles, zchunk, items, items_per_box, box_stride, strings ? f.grid : 0);
         if ((rc0 = launch_status("energy sums"))) return rc0;
         if (strings) {
             rc0 = q.want_vel ? launch_finder(finder_kernel<float, true>, grid)

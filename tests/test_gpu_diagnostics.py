@@ -446,3 +446,28 @@ def test_finder_strips_of_every_remainder(axs, nx, ny, nz, ng):
                 if len(runs) == 2:
                     assert got.vel_count == full.vel_count
                     assert got.vel_sum == pytest.approx(full.vel_sum, rel=1e-6, abs=1e-6 * max(1, full.vel_count))
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(32, 16, 5), (34, 17, 6), (33, 15, 11), (31, 3, 1), (6, 40, 64)])
+@pytest.mark.parametrize("ng", [0, 2, 3])
+def test_per_cell_fp32_energy_tiles_of_every_remainder(axs, nx, ny, nz, ng):
+    """The FP32-term energy sums on boxes that leave cells, rows or planes over
+    from the kernel's tiles and its five-plane turns, with 8-byte rows and without,
+    with and without a mask: against FP64 terms on the same fields. A term is a
+    few tens of FP32 roundings of parts no larger than the largest sum: 2e-6 of it."""
+    rng = np.random.default_rng(nx * ny + nz)
+    x = np.arange(nx) / nx * 2 * np.pi
+    field = 0.3 * rng.standard_normal((4, nz, ny, nx)) + np.cos(x)
+    field[0] += 3.0
+    bmode = axs._lib.BOUNDARY_GHOSTS if ng else axs._lib.BOUNDARY_PERIODIC
+    t = axs.new_fab((nx, ny, nz), ng, dtype=torch.float32)
+    t.copy_(_dev(np.pad(field, ((0, 0),) + ((ng, ng),) * 3, mode="wrap"), torch.float32))
+    for scheme in (0, 1, 2):
+        for mask in (None, rng.random((nz, ny, nx)) < 0.5):
+            par = lambda f32: axs._lib.DiagParams(0.5, 1.3, 2.0, 0.4, 1.0, scheme, 0.8, bmode, 1, 0, 0, f32)
+            ref, _ = _run_diag(axs, t, ng, par(0), mask)
+            got, _ = _run_diag(axs, t, ng, par(1), mask)
+            assert got.energy_sums[13] == ref.energy_sums[13] == (nx * ny * nz if mask is None else mask.sum())
+            np.testing.assert_allclose(list(got.energy_sums), list(ref.energy_sums), rtol=0,
+                                       atol=2e-6 * max(abs(e) for e in list(ref.energy_sums)[:12]))
+            np.testing.assert_allclose(got.energy_sums[12], ref.energy_sums[12], rtol=2e-6)
