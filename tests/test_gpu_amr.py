@@ -395,3 +395,51 @@ def test_patch_counts_past_the_grid_and_two_sweep_limits(axs):
     assert float((valid[0] - 1.1).abs().max()) < 2e-6
     assert float((valid[2] - 1.0).abs().max()) < 2e-6
     assert float(valid[1].abs().max()) < 1e-6 and float(valid[3].abs().max()) < 1e-6
+
+
+@pytest.mark.parametrize("block", [4, 8, 16, 32])
+@pytest.mark.parametrize("theta", [0.0, 0.37])
+@pytest.mark.parametrize("whole", [False, True])
+def test_fp32_fill_equals_fp64_fill(axs, block, theta, whole):
+    """The FP32 fill (rows of parents) against the FP64 one (tiles, pinned above) on
+    the same FP32 fields: patch sides whose rows take one segment or two, an axis
+    that is one block (a patch its own neighbour), the ring alone and the whole
+    patch. Copies are exact and valid cells stay; an interpolated cell is 20 FP32
+    roundings of values up to 3 times the field: 4e-6 of its largest."""
+    import ctypes as C
+    from axion_strings_adaptive_gb300 import _lib as L
+    from axion_strings_adaptive_gb300.amr import TwoLevel
+    dims = (2 * block, block, 3 * block)
+    rng = np.random.default_rng(block)
+    shape = (4, dims[2], dims[1], dims[0])
+    old, new = (rng.standard_normal(shape).astype(np.float32) for _ in range(2))
+    blocks = np.array([[0, 0, 0], [1, 0, 2], [1, 0, 1]])
+    valid = rng.standard_normal((3, 4) + (2 * block,) * 3).astype(np.float32)
+    got = {}
+    for dtype in (torch.float32, torch.float64):
+        coarse, start = (axs.PeriodicLevel(dims, 0.5, dtype=dtype) for _ in range(2))
+        coarse.set_state(torch.from_numpy(new).cuda().to(dtype))
+        start.set_state(torch.from_numpy(old).cuda().to(dtype))
+        two = TwoLevel(coarse, block)
+        two.old_state.copy_(start.state)
+        two.set_blocks(blocks)
+        p = two.patches
+        for q in range(3):
+            p.valid(q).copy_(torch.from_numpy(valid[q]).cuda().to(dtype))
+        L.call("axs_patches_fill", C.byref(p.c), C.byref(two._map()), C.byref(two.old_c), C.byref(coarse.c), theta, 0.1,
+               int(whole), None)
+        torch.cuda.synchronize()
+        n, lay = p.n, p.layout
+        got[dtype] = [p.box(q)[:, lay.z_offset - 4:lay.z_offset + n + 4, lay.y_offset - 4:lay.y_offset + n + 4,
+                               lay.x_offset - 6:lay.x_offset + n + 6].double().cpu().numpy() for q in range(3)]
+    order = [tuple(b) for b in two.blocks]
+    for q in range(3):
+        a, b = got[torch.float32][q], got[torch.float64][q]
+        np.testing.assert_allclose(a, b, rtol=0, atol=4e-6 * max(np.abs(old).max(), np.abs(new).max()))
+        if not whole:
+            np.testing.assert_array_equal(a[:, 4:-4, 4:-4, 6:-6], valid[q])
+            # the y ring of a level one block wide in y: the patch's own valid cells
+            np.testing.assert_array_equal(a[:, 4:-4, :4, 6:-6], valid[q][:, :, -4:])
+            # blocks (1, 0, 1) and (1, 0, 2) are neighbours in z
+            if order[q] == (1, 0, 1):
+                np.testing.assert_array_equal(a[:, -4:, 4:-4, 6:-6], valid[order.index((1, 0, 2))][:, :4])
