@@ -1038,7 +1038,7 @@ __global__ void __launch_bounds__(kFillThreads)
                           ((dz < 0 ? -kRingYZ : (dz > 0 ? n : 0)) + kPatchRZ) * f.ks;
     float *const d = st + (int64_t)pq * f.box + first;
     const float *const s = st + (int64_t)owner * f.box + first - (int64_t)n * (dx + dy * f.js + dz * f.ks);
-    for (int i = threadIdx.x; i < wx * wy * wz; i += 2 * kFillThreads) {
+    for (int i = 2 * kFillThreads * blockIdx.y + threadIdx.x; i < wx * wy * wz; i += 2 * kFillThreads * gridDim.y) {
         float4 w[2][4];
         int64_t o[2];
         bool on[2];
@@ -1362,7 +1362,10 @@ int axs_patches_fill_list(const axs_patches *p, const axs_patch_map *m, const ax
     AXS_REQUIRE(blocks < (int64_t)INT32_MAX, AXS_ERR_UNSUPPORTED, "too many patches for one fill launch");
     if (p->dtype == AXS_F32) {
         float *state = static_cast<float *>(p->state);
-        if (!f.valid_too) patch_copy_ring_kernel<<<26u * (unsigned)count, kFillThreads, 0, st>>>(state, f);
+        if (!f.valid_too) {
+            const dim3 grid(26u * (unsigned)count, (unsigned)std::max(1, g.n * g.n / 1024));  // a slab of n = 32 a block
+            patch_copy_ring_kernel<<<grid, kFillThreads, 0, st>>>(state, f);
+        }
         (f.blend ? patch_fill_kernel<true> : patch_fill_kernel<false>)
             <<<(unsigned)((items + kFillThreads / 32 - 1) / (kFillThreads / 32)), kFillThreads, 0, st>>>(state, cv, f, q,
                                                                                                     units, items);
