@@ -287,10 +287,11 @@ static const TileConfigEntry kF32Configs[] = {
 };
 static const TileConfigEntry kF64Configs[] = {
     // The default. FP64 sweeps alternate between the integer Laplacian sums and the
-    // FP64 stage arithmetic; 8 blocks of two warps a SM are rarely in the same phase,
-    // which two blocks of eight are: 3.03 against 3.74 ms a step at 256^3, 70 against
-    // 71 us at 64^3 (32x4: 3.07 ms, 74 us).
-    {"f64 v1 16x4 ring6", &SweepConfig<double, 1, 16, 4, 6, 8>::run, nullptr},
+    // FP64 stage arithmetic; 4 blocks of four warps a SM are rarely in the same phase,
+    // which two blocks of eight are (32x8: 3.51 ms a step at 256^3, this 2.79). 16x4, 6
+    // or 7 blocks of two warps with half as many rows of halo again, took 1.04x as long
+    // at 256^3, 1.06-1.09x at 96^3 to 224^3, 0.95-1.07x at 128^3 and below 96^3.
+    {"f64 v1 16x8 ring6", &SweepConfig<double, 1, 16, 8, 6, 4>::run, nullptr},
     {"f64 v1 32x8 ring6", &SweepConfig<double, 1, 32, 8, 6, 2>::run, nullptr},
     {"f64 v2 32x8 ring6", &SweepConfig<double, 2, 32, 8, 6, 2>::run, nullptr},
     {"f64 v2 32x16 ring6", &SweepConfig<double, 2, 32, 16, 6, 1>::run, nullptr},
