@@ -305,11 +305,25 @@ static int config_count(int32_t dtype)
                             : (int)(sizeof(kF32Configs) / sizeof(kF32Configs[0]));
 }
 
+// The default of small FP32 levels: the fused step's march (12 planes to start, 20
+// warps in turn) and its padding launch take longer there than two short launches.
+// One step, fused / two sweeps: 48^3 13.4 / 10.1 us, 64x35x70 14.8 / 11.5, 64^3 15.0 / 14.0,
+// 80^3 22.8 / 23.8; two steps 24.1 / 19.8, 27.0 / 22.6, 27.3 / 28.0, 39.8 / 47.0.
+constexpr int64_t kFusedLeastSites = 300000;
+static const TileConfigEntry kSmallF32Config = {"", &FusedConfig<32, 16>::Fallback::run,
+                                                &FusedConfig<32, 16, true>::Fallback::run};
+
 static const TileConfigEntry *config_for(int32_t dtype, int32_t id)
 {
     const TileConfigEntry *tab = dtype == AXS_F64 ? kF64Configs : kF32Configs;
     if (id < 0 || id > config_count(dtype)) return nullptr;
     return &tab[id == 0 ? 0 : id - 1];
+}
+static const TileConfigEntry *config_for(const axs_level *lv)
+{
+    if (lv->tile_config == 0 && lv->dtype == AXS_F32 && (int64_t)lv->nx * lv->ny * lv->nz < kFusedLeastSites)
+        return &kSmallF32Config;
+    return config_for(lv->dtype, lv->tile_config);
 }
 
 // The level's runner: its tiling, or the compensated FP32 step when the level
@@ -325,7 +339,7 @@ static Runner runner_for(const axs_level *lv, const TileConfigEntry *cfg)
 static int run_sweeps(const axs_level *lv, const LevelGeom &g, const axs_background *bg, double tau_i, double t0,
                       double dt, int nsteps, int mask, cudaStream_t st)
 {
-    const TileConfigEntry *cfg = config_for(lv->dtype, lv->tile_config);
+    const TileConfigEntry *cfg = config_for(lv);
     AXS_REQUIRE(cfg != nullptr, AXS_ERR_INVALID_ARGUMENT, "tile_config %d out of range (0..%d)", lv->tile_config,
                 config_count(lv->dtype));
     SweepRunArgs r{lv, &g, bg, tau_i, t0, dt, nsteps, mask, st, nullptr};
@@ -483,7 +497,7 @@ int axs_level_rk4_step_to(const axs_level *lv, void *dst_state, const axs_backgr
         AXS_REQUIRE(bg->a_inv > 1.0, AXS_ERR_INVALID_ARGUMENT, "a_inv must exceed 1");
         AXS_REQUIRE(tau_i + t > 0.0, AXS_ERR_INVALID_ARGUMENT, "conformal time must stay positive");
     }
-    const TileConfigEntry *cfg = config_for(lv->dtype, lv->tile_config);
+    const TileConfigEntry *cfg = config_for(lv);
     AXS_REQUIRE(cfg != nullptr, AXS_ERR_INVALID_ARGUMENT, "tile_config %d out of range (0..%d)", lv->tile_config,
                 config_count(lv->dtype));
     SweepRunArgs r{lv, &g, bg, tau_i, t, dt, 1, 3, (cudaStream_t)stream, dst_state};

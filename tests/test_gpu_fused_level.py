@@ -221,3 +221,27 @@ def test_fused_step_at_the_edges_of_its_tiles(axs, shape, comp):
         out.append(lv.state)
     # both the valid cells and the periodic padding and corners
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("nz", [73, 74])
+@pytest.mark.parametrize("compensated", [False, True])
+def test_default_of_small_levels_is_the_same_step(axs, nz, compensated):
+    """The default tiling just below and above the size from which it is the fused
+    step, in place and into another buffer, against the fused step asked for: the
+    same bits."""
+    bg = axs.Background.expanding(2.0, 1.0, lambda0=2.0)
+    st = torch.randn((4, nz, 64, 64), generator=torch.Generator().manual_seed(3)).cuda()
+    got = []
+    for name in (None, "f32 fused 32x16 columns"):
+        lv = axs.PeriodicLevel((64, 64, nz), 0.5, dtype=torch.float32)
+        lv.compensated = compensated
+        if name is not None:
+            lv.tile_config = _config_id(lv, name)
+        lv.set_state(st)
+        lv.advance(bg, 1.0, 0.0, 0.05, 3)
+        dst = torch.zeros_like(lv.state)
+        lv.step_to(dst, bg, 1.0, 0.15, 0.05)
+        lv.device_status()
+        ox, oy = lv.layout.x_offset, lv.layout.y_offset
+        got.append((lv.valid_view().clone(), dst[:, :, oy:oy + 64, ox:ox + 64].clone()))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
