@@ -17,8 +17,8 @@
 //   - the one-pass fused step (level_fused.cuh, FusedBoxes item source): ONE
 //     persistent launch per RK4 step plus one launch for the boxes' periodic
 //     padding, 8 words per site; steps alternate between the state arena and
-//     the work arena's first four planes. Boxes need ny a multiple of the
-//     tile height and an even nx (a last, partial tile column is masked);
+//     the work arena's first four planes. Boxes need ny = 16 or ny >= 20 (tile
+//     rows are spread evenly and overlap; a last, partial tile column is masked);
 //   - the two sweeps (sweep.cuh, BoxTable item source): one persistent launch
 //     per sweep, 28 words per site, any box shape.
 //
@@ -277,8 +277,9 @@ template <typename T, int V, int TX, int TY, int NS, int MINB, bool HINT = false
 // The one-pass fused step over every box: per RK4 step one launch of
 // level_fused_kernel<S, FusedBoxes> from one state buffer into the other and
 // one ens_pad_kernel for the periodic padding of the buffer written. An odd
-// step count first copies the state arena (padding included) to the work
-// arena, so that the last step writes the state arena.
+// step count ends with a copy back to the state arena that writes the padding
+// too (8 boxes of 36x28x40, one step: 34.7 us with the state copied to the work
+// arena first, 33.5 so).
 template <int TX, int TY> struct EnsFusedConfig {
     using S = LevelFusedShape<TX, TY>;
 
@@ -320,23 +321,18 @@ template <int TX, int TY> struct EnsFusedConfig {
         float *buf[2] = {static_cast<float *>(e->state), static_cast<float *>(e->work)};
         LevelFusedMaps unused;  // FusedBoxes reads each box's maps from the table
         std::memset(&unused, 0, sizeof(unused));
-        int max_nz = 1, max_row = 1;
+        int max_nz = 1, max_row = 1, max_units = 1;
         for (int b = 0; b < e->nboxes; ++b) {
             const int nx = e->dims[3 * b], ny = e->dims[3 * b + 1], nz = e->dims[3 * b + 2];
             max_nz = std::max(max_nz, nz);
             max_row = std::max(max_row, pad_quads(nx, ny));
+            max_units = std::max(max_units, nx / 4 * ny);
         }
         const dim3 pad_grid((unsigned)std::min(64, (max_row + 256 * kPadUnroll - 1) / (256 * kPadUnroll)),
                             (unsigned)std::min(4 * max_nz, 65535), (unsigned)e->nboxes);
-        int first = 0;
-        if (r.nsteps & 1) {
-            AXS_CUDA_CHECK(cudaMemcpyAsync(buf[1], buf[0], (size_t)(4 * P) * sizeof(float), cudaMemcpyDeviceToDevice,
-                                           r.st));
-            first = 1;
-        }
         for (int s = 0; s < r.nsteps; ++s) {
             const double t = r.t0 + s * r.dt;
-            const int src = (s + first) & 1;
+            const int src = s & 1;
             SweepArgs<float> as = a;
             as.map_sel = src;
             as.c1 = stage_coef<float>(*r.bg, r.tau_i + t);
@@ -346,6 +342,12 @@ template <int TX, int TY> struct EnsFusedConfig {
             for (int c = 0; c < 4; ++c) as.out[c] = dst + c * P;
             level_fused_kernel<S, FusedBoxes><<<r.plan->grid_a, S::THREADS, S::SMEM, r.st>>>(unused, as);
             if ((rc = launch_status("fused ensemble step"))) return rc;
+            if (s + 1 == r.nsteps && src == 0) {
+                const dim3 copy_grid((unsigned)std::max(1, std::min(64, max_units / (256 * kPadUnroll))), pad_grid.y,
+                                     pad_grid.z);
+                ens_copy_pad_kernel<float><<<copy_grid, 256, 0, r.st>>>(buf[0], dst, a.boxes, P, a.ox);
+                return launch_status("ensemble copy");
+            }
             ens_pad_kernel<float><<<pad_grid, 256, 0, r.st>>>(dst, a.boxes, P, a.ox);
             if ((rc = launch_status("ensemble padding"))) return rc;
         }
@@ -367,7 +369,7 @@ static bool fused_fits(const int32_t *dims, int nboxes, int ty)
 }
 
 // The default (tile_config 0) is the first entry of its table that suits
-// every box: the fused step (0.91 ms per step on a mixed 32^3..128^3
+// every box: the fused step (0.58 ms per step on a mixed 32^3..128^3
 // ensemble on GB300), else the fastest two-sweep tiling there (1.01 ms). The
 // 16-wide tiles leave no idle columns on boxes whose width is a multiple of
 // 16 but read 96-byte rows.

@@ -673,4 +673,12 @@ __global__ void ens_pad_kernel(T *__restrict__ buf, const EnsBoxDesc *__restrict
     pad_box(buf + d.base, buf + d.base, d.nx, d.ny, d.nz, d.js, d.ks, cs, ox, d.oy);
 }
 
+template <typename T>
+__global__ void ens_copy_pad_kernel(T *__restrict__ dst, const T *__restrict__ src,
+                                    const EnsBoxDesc *__restrict__ boxes, int64_t cs, int ox)
+{
+    const EnsBoxDesc &d = boxes[blockIdx.z];
+    copy_pad_box(dst + d.base, src + d.base, d.nx, d.ny, d.nz, d.js, d.ks, cs, ox, d.oy);
+}
+
 }  // namespace axs
