@@ -82,7 +82,7 @@ class _StringCoreLoss(torch.autograd.Function):
         level.set_state(state0.detach())
         k = max(1, int(spec.checkpoint_every))
         # Steps go from buffer to buffer (one fused launch each, where a step in place
-        # takes the two sweeps), so a checkpoint is a buffer kept, not a copy.
+        # copies its result back), so a checkpoint is a buffer kept, not a copy.
         checkpoints, spare = [], None
         for s in range(spec.nsteps):
             dst = torch.empty_like(level.state) if spare is None else spare

@@ -4,8 +4,8 @@
 stage-buffer arena (the ``axs_ensemble`` layout of include/axs.h), builds the
 device table for one tiling, and advances every box together: with the
 one-pass fused step (one persistent launch per RK4 step plus one for the
-periodic padding; the default for boxes with ny a multiple of 16 and an even
-nx) or with two persistent sweep launches per step (any box shape).
+periodic padding; the default where every box has ny = 16 or ny >= 20) or with
+two persistent sweep launches per step (any box shape).
 ``capture(...)`` records a whole run -- the steps plus
 per-box diagnostics -- as one CUDA graph; :meth:`Ensemble.autotune` times the
 compiled tilings and z-chunk targets (the work each block takes from a box) on

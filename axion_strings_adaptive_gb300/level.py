@@ -215,8 +215,8 @@ class PeriodicLevel:
                  stream=None) -> dict:
         """Time every compiled tiling on this level (the two-sweep tilings and
         the one-pass fused step; full RK4 steps, CUDA events) and keep the
-        fastest. An even step count times the fused step alone (an odd count
-        runs its first step as the two sweeps). The state is saved and restored, so the
+        fastest. An even step count times the fused step alone (an odd one ends
+        with a copy back to the state). The state is saved and restored, so the
         level's contents are unchanged. Returns {name: ms_per_step}."""
         saved = self.state.clone()
         timings = {}
@@ -255,7 +255,7 @@ class PeriodicLevel:
         L.call("axs_level_export_fab", C.byref(self.c), C.byref(fab(t, ng)), _stream_ptr(stream))
 
     def advance(self, bg: Background, tau_i: float, t0: float, dt: float, nsteps: int, stream=None) -> None:
-        """nsteps classic-RK4 steps (two fused sweeps each); asynchronous."""
+        """nsteps classic-RK4 steps (the tiling's one-pass launch or two sweeps each); asynchronous."""
         L.call("axs_level_rk4_advance", C.byref(self.c), C.byref(bg.to_c()), float(tau_i), float(t0), float(dt),
                int(nsteps), _stream_ptr(stream))
 

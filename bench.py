@@ -553,8 +553,8 @@ def run_native(args):
         """K RK4 steps of `level`, CUDA events on the launching stream around every
         kernel launch. Two-sweep tilings: sweep A and sweep B each step. The fused
         step (the fused launch and the padding launch), timed in pairs of steps:
-        a pair returns the state to the level's state buffer; a single step runs
-        as the two sweeps, so an odd K ends with one of those. Returns (total ms,
+        a pair returns the state to the level's state buffer; a single step
+        copies it back, so an odd K ends with one of those. Returns (total ms,
         {kernel: mean ms per launch}, clocks)."""
         fused = "fused" in level_config_name(level)
         for w in range(warmup):

@@ -188,8 +188,8 @@ int axs_rk4_combine(const axs_fab *dst, const axs_fab *uold, const axs_fab *k1, 
  * cache line; the 8 columns left of x = 0 and right of x = nx-1 (the stencils
  * read 4; 8 fill whole 32-byte sectors) and the 2 rows outside y hold periodic
  * copies that the kernels keep current (padding corners excepted). `state` holds psi1, psi2, Pi1, Pi2; `work` holds 8
- * components of the same layout used between the two sweeps of a step, plus
- * a 256-byte status block. Both must be 128-byte aligned. */
+ * components of the same layout used between the two sweeps of a step (the
+ * fused step's second state buffer is its first 4), plus a 256-byte status block. Both must be 128-byte aligned. */
 typedef struct axs_level_layout {
     int64_t jstride, kstride, cstride; /* elements */
     int32_t x_offset, y_offset;       /* elements */
@@ -246,8 +246,8 @@ int axs_level_download(const axs_level *lv, void *host_state, void *stream);
 /* Replaces GRTeclyn's RK4 level advance (docs/conventions.md:239-245, driver
  * absent from the reference tree) together with nsteps x 4 calls of
  * specific_eval_rhs: advances the state by nsteps classic-RK4 steps of size
- * dt from t0, coefficients from `bg` at tau = tau_i + t_stage. Two sweeps
- * per step; async on `stream`. */
+ * dt from t0, coefficients from `bg` at tau = tau_i + t_stage. One fused launch
+ * and one for the padding per step, or two sweeps; async on `stream`. */
 int axs_level_rk4_advance(const axs_level *lv, const axs_background *bg, double tau_i, double t0,
                           double dt, int32_t nsteps, void *stream);
 
