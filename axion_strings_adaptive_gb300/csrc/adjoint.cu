@@ -28,6 +28,7 @@
 
 namespace axs {
 
+int level_stages(const axs_level *lv, const axs_background *bg, double tau_i, double t, double dt, cudaStream_t st);
 int level_fill_ghosts(void *data, int32_t dtype, int nx, int ny, int nz, const LevelGeom &g, int ncomp,
                       cudaStream_t st);
 int make_level_map(CUtensorMap *map, const void *base, int32_t dtype, const LevelGeom &g, int ny, int nz,
@@ -199,8 +200,8 @@ __global__ void sum_partials_kernel(const double *__restrict__ part, int n, doub
 
 // ----------------------------------------------------------------------------
 // Adjoint tiling, one per dtype. FP32: two sites a thread, for the packed
-// Laplacians and half the index work (656 against 888 us a step at 256^3, 121
-// against 144 at 128^3, with one site on 256 threads; 32x16, 32x4 and 64x4
+// Laplacians and half the index work (613 against 845 us a step at 256^3, 111
+// against 134 at 128^3, with one site on 256 threads; 32x16, 32x4 and 64x4
 // tiles and L2 policies lay between). FP64: one site (V = 1 keeps the 12
 // pointwise components of sweep A in registers) in smaller blocks, as the
 // forward sweeps.
@@ -306,7 +307,7 @@ int axs_level_rk4_adjoint_step(const axs_level *lv, void *abar, void *adj_work, 
                 (long long)adj_work_bytes, (long long)need);
     cudaStream_t st = (cudaStream_t)stream;
     // recompute the stage fields u3, u4 of this step into lv->work
-    rc = axs_level_rk4_sweep(lv, bg, tau_i, t, dt, 0, stream);
+    rc = level_stages(lv, bg, tau_i, t, dt, st);
     if (rc) return rc;
     const size_t es = dtype_size(lv->dtype);
     double *lam_part = reinterpret_cast<double *>(static_cast<char *>(adj_work) + 8 * g.cs * es);

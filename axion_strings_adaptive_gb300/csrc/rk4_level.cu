@@ -117,6 +117,25 @@ struct SweepConfig {
     using LA = SweepLauncher<T, V, TX, TY, NS, MINB, ForwardAT<COMP>, SingleLevel, HINT>;
     using LB = SweepLauncher<T, V, TX, TY, NS, MINB, ForwardBT<COMP>, SingleLevel, HINT>;
 
+    // d3, d4 of one step into the work buffer's first four planes
+    static int run_stages(const SweepRunArgs &r)
+    {
+        using LS = SweepLauncher<T, V, TX, TY, NS, MINB, ForwardStagesT<COMP>, SingleLevel, HINT>;
+        const axs_level *lv = r.lv;
+        const LevelGeom &g = *r.g;
+        SweepArgs<T> a{};
+        int grid = 0;
+        int rc = LS::plan(a, lv->nx, lv->ny, lv->nz, grid);
+        if (rc) return rc;
+        fill_level_constants(a, lv, g, r.dt);
+        CUtensorMap map;
+        if ((rc = make_level_map(&map, lv->state, lv->dtype, g, lv->ny, lv->nz, LS::box_x(), LS::box_y()))) return rc;
+        a.c1 = stage_coef<T>(*r.bg, r.tau_i + r.t0);
+        a.c2 = stage_coef<T>(*r.bg, r.tau_i + r.t0 + 0.5 * r.dt);
+        for (int c = 0; c < 4; ++c) a.out[c] = static_cast<T *>(lv->work) + c * g.cs;
+        return LS::launch(map, a, grid, r.st);
+    }
+
     static int run(const SweepRunArgs &r)
     {
         const axs_level *lv = r.lv;
@@ -336,6 +355,7 @@ static Runner runner_for(const axs_level *lv, const TileConfigEntry *cfg)
     return cfg->run;
 }
 
+constexpr int kStagesOnly = 4;  // sweep mask: run_stages, in the default tilings of the two sweeps
 static int run_sweeps(const axs_level *lv, const LevelGeom &g, const axs_background *bg, double tau_i, double t0,
                       double dt, int nsteps, int mask, cudaStream_t st)
 {
@@ -343,7 +363,23 @@ static int run_sweeps(const axs_level *lv, const LevelGeom &g, const axs_backgro
     AXS_REQUIRE(cfg != nullptr, AXS_ERR_INVALID_ARGUMENT, "tile_config %d out of range (0..%d)", lv->tile_config,
                 config_count(lv->dtype));
     SweepRunArgs r{lv, &g, bg, tau_i, t0, dt, nsteps, mask, st, nullptr};
+    if (mask == kStagesOnly) {
+        if (lv->dtype == AXS_F64) return SweepConfig<double, 1, 16, 8, 6, 4>::run_stages(r);
+        return lv->flags & AXS_LEVEL_COMPENSATED_FP32 ? FusedConfig<32, 16, true>::Fallback::run_stages(r)
+                                                      : FusedConfig<32, 16>::Fallback::run_stages(r);
+    }
     return runner_for(lv, cfg)(r);
+}
+
+// The stage increments of the step from time t, for the adjoint step.
+int level_stages(const axs_level *lv, const axs_background *bg, double tau_i, double t, double dt, cudaStream_t st)
+{
+    LevelGeom g;
+    int rc = validate_level(lv, g);
+    if (rc) return rc;
+    AXS_REQUIRE(bg != nullptr, AXS_ERR_INVALID_ARGUMENT, "null background");
+    AXS_REQUIRE(std::isfinite(dt) && dt > 0.0, AXS_ERR_INVALID_ARGUMENT, "dt must be positive and finite");
+    return run_sweeps(lv, g, bg, tau_i, t, dt, 1, kStagesOnly, st);
 }
 
 }  // namespace axs

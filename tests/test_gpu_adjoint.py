@@ -2,6 +2,8 @@
 the C ABI: directional derivatives against central finite differences, the
 lambda0 gradient, checkpoint-interval invariance, and FP32 against the FP64
 adjoint (the differentiation configuration at reduced size)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -97,3 +99,29 @@ def test_differentiation_config_reduced(axs):
         fd = (float(_loss(axs, s64 + eps * d, lam, spec)) - float(_loss(axs, s64 - eps * d, lam, spec))) / (2 * eps)
         ad = float((g32 * d).sum())
         assert ad == pytest.approx(fd, rel=1e-2, abs=1e-3 * float(g64.norm())), (ad, fd)
+
+
+@pytest.mark.parametrize("shape", [(4, 2, 1), (36, 9, 5), (68, 33, 20)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("compensated", [False, True])
+def test_recomputed_stages_are_sweep_as(axs, shape, dtype, compensated):
+    """The stage increments that the adjoint step recomputes are the ones sweep A
+    writes, bit for bit, at sizes that leave sites over from its tiles."""
+    from axion_strings_adaptive_gb300 import adjoint
+    nx, ny, nz = shape
+    bg = axs.Background.expanding(2.0, 1.0, lambda0=2.0)
+    lv = axs.PeriodicLevel(shape, 0.5, dtype=dtype, pierced_capacity=1)
+    lv.compensated = compensated
+    lv.set_state(torch.randn((4, nz, ny, nx), generator=torch.Generator().manual_seed(1)).cuda().to(dtype))
+    n = lv.state.numel()
+    ox, oy = lv.layout.x_offset, lv.layout.y_offset
+    stages = lambda: lv.work.view(dtype)[:n].view(lv.state.shape)[:, :, oy:oy + ny, ox:ox + nx].clone()
+    lv.sweep(bg, 1.0, 0.0, 0.05, 0)
+    want = stages()
+    lv.work.zero_()
+    buf = adjoint.AdjointBuffers(lv)  # (adjoint.adjoint_step passes no level flags)
+    axs._lib.call("axs_level_rk4_adjoint_step", C.byref(lv.c), buf.abar.data_ptr(), buf.work.data_ptr(),
+                  buf.work.numel(), C.byref(bg.to_c()), 1.0, 0.0, 0.05, buf.lambda_bar.data_ptr(),
+                  torch.cuda.current_stream().cuda_stream)
+    lv.device_status()
+    assert torch.equal(stages(), want)
