@@ -17,8 +17,8 @@
 // with J_s(u)^T a = lap a + kappa_s a - lambda_s/2 [(|u|^2 - R_s^2) a + 2 u (u . a)]
 // (the periodic centred Laplacian is symmetric), and the lambda0 gradient
 //   lambda0bar += sum_s sum_sites -(lambda_s/2)/lambda0 (|u_s|^2 - R_s^2) (u_s . F_sbar).
-// u3 and u4 are recomputed by re-running forward sweep A on psi_n, Pi_n
-// (it stores d3 = u3 - psi_n, d4 = u4 - psi_n).
+// u3 and u4 are recomputed by forward sweep A's stencil on psi_n, Pi_n
+// (ForwardStagesT stores d3 = u3 - psi_n, d4 = u4 - psi_n).
 // Each adjoint sweep is the same TMA-staged stencil pipeline as the forward
 // sweeps (sweep.cuh); sweep B reads 4+6 and writes 8 components per site,
 // sweep A reads 4+12 and writes 4.
