@@ -275,7 +275,9 @@ __global__ void __launch_bounds__(S::THREADS, 1)
 
     // A wait is a test whose answer is looked at a step later, and a bounded wait
     // where it said no: the latency of a wait at its point of use would lie on the
-    // warp's path. An expired wait ends the block: every other wait sees `failed`.
+    // warp's path. A warp whose wait expired leaves the march there and then: it hands
+    // nothing on, so what waits for it expires as well (at once: the waits see
+    // `failed`), and sweep B stores nothing that was made from data still to come.
     uint32_t bar0 = smem_addr(bars);
     asm volatile("" : "+r"(bar0));  // kept, not recomputed
     auto landed = [&](int k) { return bar0 + 8u * k; };
@@ -293,10 +295,9 @@ __global__ void __launch_bounds__(S::THREADS, 1)
         *(volatile int *)&failed = 1;
         return false;
     };
-    auto ended = [&]() -> bool { return __any_sync(0xffffffffu, *(volatile int *)&failed != 0) != 0; };
-
-    auto need = [&](bool ready, uint32_t bar, uint32_t phase) {
-        if (__any_sync(0xffffffffu, !ready)) slow_wait(bar, phase);
+    auto need = [&](bool ready, uint32_t bar, uint32_t phase) -> bool {  // the whole warp's
+        if (__all_sync(0xffffffffu, ready)) return true;
+        return __all_sync(0xffffffffu, slow_wait(bar, phase)) != 0;
     };
 
     // March of an item. Planes are numbered from z0 - 4. Step i = 0 .. len + 3: sweep A
@@ -394,80 +395,84 @@ __global__ void __launch_bounds__(S::THREADS, 1)
             off += SLOT;
             if (off >= NS * SLOT) off -= NS * SLOT;
         };
-        auto take_plane = [&](bool ready) {
-            need(ready, landed(slot), landed_phase);
+        auto take_plane = [&](bool ready) -> bool {
+            if (!need(ready, landed(slot), landed_phase)) return false;
             if constexpr (Src::kPatches)
                 if (tid < a.ntiles) mbar_arrive_cluster(peers(slot), tid);  // tid: the tile told
             if (++slot == NS) {
                 slot = 0;
                 landed_phase ^= 1;
             }
+            return true;
         };
         FusedColumn col;
-        for (FusedCursor cur = Src::begin(a); Src::valid(cur); Src::next(cur, a)) {
-            const int n = Src::template item<TX, TY>(a, maps, cur).len + 4;
-            {
-                F2 first[4][4];
+        auto march = [&]() {  // returns when it is done or a wait expired
+            for (FusedCursor cur = Src::begin(a); Src::valid(cur); Src::next(cur, a)) {
+                const int n = Src::template item<TX, TY>(a, maps, cur).len + 4;
+                {
+                    F2 first[4][4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    take_plane(false);
-                    if (k == 2) off_mid = off_new;
+                    for (int k = 0; k < 4; ++k) {
+                        if (!take_plane(false)) return;
+                        if (k == 2) off_mid = off_new;
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) first[k][c] = F2(lds2(lf_smem + off_new + c * RC));
+                        for (int c = 0; c < 4; ++c) first[k][c] = F2(lds2(lf_smem + off_new + c * RC));
+                        next_off(off_new);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        col.f[0][c] = first[2][c];
+                        col.f[1][c] = first[3][c];
+                        col.u1[c] = first[2][c] - first[1][c];
+                        col.u2[1][c] = first[3][c] - first[1][c];
+                        col.u2[0][c] = first[2][c] - first[0][c];
+                    }
+                }
+                bool ready = false;
+                auto step = [&](auto ph) -> bool {
+                    constexpr int P = decltype(ph)::value;
+                    if (!take_plane(ready)) return false;
+                    ready = mbar_test_at(landed(slot), landed_phase);
+                    const bool free = mbar_test_at(win_read(ws), read_phase);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) col.in<P>(c) = F2(lds2(lf_smem + off_new + c * RC));
                     next_off(off_new);
-                }
+                    F2 lap[4];
+                    star4_column<P, RB, RC, S::COMP>(a, lf_smem + off_mid, col, lap);
+                    next_off(off_mid);
+                    const StageAPair sa = stage_a_pair<S::COMP>(a, col.mid<P>(0), col.mid<P>(1), col.mid<P>(2),
+                                                                col.mid<P>(3), lap[0], lap[1], lap[2], lap[3]);
+                    if (!need(free, win_read(ws), read_phase)) return false;
+                    unsigned char *const wz = wsite + ws * WSLOT, *const ez = esite + ws * ESLOT;
+                    if (has_a) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    col.f[0][c] = first[2][c];
-                    col.f[1][c] = first[3][c];
-                    col.u1[c] = first[2][c] - first[1][c];
-                    col.u2[1][c] = first[3][c] - first[1][c];
-                    col.u2[0][c] = first[2][c] - first[0][c];
+                        for (int c = 0; c < 4; ++c) *reinterpret_cast<float2 *>(wz + c * WC) = sa.d[c].v;
+                    }
+                    if (tile_site) {
+                        F2 eq[4];
+                        stage_a_eq<S::COMP>(a, sa, lap[0], lap[1], eq);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) *reinterpret_cast<float2 *>(ez + c * EC) = eq[c].v;
+                    }
+                    __syncwarp();
+                    if (lane0) mbar_arrive_at(stored(ws));
+                    if (++ws == U) {
+                        ws = 0;
+                        read_phase ^= 1;
+                    }
+                    return true;
+                };
+                for (int i = 0;;) {
+                    if (!step(std::integral_constant<int, 0>{})) return;
+                    if (++i == n) break;
+                    if (!step(std::integral_constant<int, 1>{})) return;
+                    if (++i == n) break;
+                    if (!step(std::integral_constant<int, 2>{})) return;
+                    if (++i == n) break;
                 }
             }
-            bool ready = false;
-            auto step = [&](auto ph) {
-                constexpr int P = decltype(ph)::value;
-                take_plane(ready);
-                ready = mbar_test_at(landed(slot), landed_phase);
-                const bool free = mbar_test_at(win_read(ws), read_phase);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) col.in<P>(c) = F2(lds2(lf_smem + off_new + c * RC));
-                next_off(off_new);
-                F2 lap[4];
-                star4_column<P, RB, RC, S::COMP>(a, lf_smem + off_mid, col, lap);
-                next_off(off_mid);
-                const StageAPair sa = stage_a_pair<S::COMP>(a, col.mid<P>(0), col.mid<P>(1), col.mid<P>(2),
-                                                            col.mid<P>(3), lap[0], lap[1], lap[2], lap[3]);
-                need(free, win_read(ws), read_phase);
-                unsigned char *const wz = wsite + ws * WSLOT, *const ez = esite + ws * ESLOT;
-                if (has_a) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) *reinterpret_cast<float2 *>(wz + c * WC) = sa.d[c].v;
-                }
-                if (tile_site) {
-                    F2 eq[4];
-                    stage_a_eq<S::COMP>(a, sa, lap[0], lap[1], eq);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) *reinterpret_cast<float2 *>(ez + c * EC) = eq[c].v;
-                }
-                __syncwarp();
-                if (lane0) mbar_arrive_at(stored(ws));
-                if (++ws == U) {
-                    ws = 0;
-                    read_phase ^= 1;
-                }
-            };
-            for (int i = 0;;) {
-                step(std::integral_constant<int, 0>{});
-                if (++i == n) break;
-                step(std::integral_constant<int, 1>{});
-                if (++i == n) break;
-                step(std::integral_constant<int, 2>{});
-                if (++i == n || ended()) break;
-            }
-            if (ended()) break;
-        }
+        };
+        march();
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
         // ---- sweep B, a unit of the tile to a thread
@@ -477,11 +482,12 @@ __global__ void __launch_bounds__(S::THREADS, 1)
         int slot = 0, off_y = 4 * ((by + 4) * BX + bx + 4);  // ring slot of plane i, this site in it
         int ws = 0, wm = 0;                                  // window slots of steps i and i - 2
         uint32_t stored_phase = 0, landed_phase = 0;
-        auto peers_landed = [&]() {
-            need(mbar_test_at(peers(slot), landed_phase), peers(slot), landed_phase);
+        auto peers_landed = [&]() -> bool {
+            return need(mbar_test_at(peers(slot), landed_phase), peers(slot), landed_phase);
         };
-        auto release_plane = [&]() {  // after the warp's reads of it
-            if constexpr (Src::kPatches) peers_landed();  // every plane: a tile is told once per round of a slot
+        auto release_plane = [&]() -> bool {  // after the warp's reads of it
+            if constexpr (Src::kPatches)
+                if (!peers_landed()) return false;  // every plane: a tile is told once per round of a slot
             if (lane0) mbar_arrive_at(ring_read(slot));
             off_y += SLOT;
             if (++slot == NS) {
@@ -489,6 +495,7 @@ __global__ void __launch_bounds__(S::THREADS, 1)
                 off_y -= NS * SLOT;
                 landed_phase ^= 1;
             }
+            return true;
         };
         auto release_window = [&]() {
             if (lane0) mbar_arrive_at(win_read(wm));
@@ -500,66 +507,71 @@ __global__ void __launch_bounds__(S::THREADS, 1)
             for (int k = 0; k < 3; ++k) col.f[k][c] = col.u2[k][c] = F2(0.f);
             col.u1[c] = F2(0.f);
         }
-        for (FusedCursor cur = Src::begin(a); Src::valid(cur); Src::next(cur, a)) {
-            const FusedItem w = Src::template item<TX, TY>(a, maps, cur);
-            const bool in_box = w.x0 + bx < w.nx;
-            int64_t off = w.base + (int64_t)(w.x0 + bx + a.ox) + (int64_t)(w.y0 + by + oy) * w.js + (int64_t)w.z0 * w.ks;
-            const int n = w.len + 4;
-            bool ready = false;
-            auto step = [&](auto ph, int i) {
-                constexpr int P = decltype(ph)::value;
-                need(ready, stored(ws), stored_phase);
-                const unsigned char *const wz = wsite + ws * WSLOT;
-                if (++ws == U) {
-                    ws = 0;
-                    stored_phase ^= 1;
+        auto march = [&]() {  // returns when it is done or a wait expired
+            for (FusedCursor cur = Src::begin(a); Src::valid(cur); Src::next(cur, a)) {
+                const FusedItem w = Src::template item<TX, TY>(a, maps, cur);
+                const bool in_box = w.x0 + bx < w.nx;
+                int64_t off = w.base + (int64_t)(w.x0 + bx + a.ox) + (int64_t)(w.y0 + by + oy) * w.js + (int64_t)w.z0 * w.ks;
+                const int n = w.len + 4;
+                bool ready = false;
+                auto step = [&](auto ph, int i) -> bool {
+                    constexpr int P = decltype(ph)::value;
+                    if (!need(ready, stored(ws), stored_phase)) return false;
+                    const unsigned char *const wz = wsite + ws * WSLOT;
+                    if (++ws == U) {
+                        ws = 0;
+                        stored_phase ^= 1;
+                    }
+                    ready = mbar_test_at(stored(ws), stored_phase);
+                    const bool here = mbar_test_at(landed(slot), landed_phase);  // long since: sweep A has read the plane
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) col.in<P>(c) = F2(lds2(wz + c * WC));
+                    if (i >= 4) {
+                        // (E, Q) of plane i with its d3, d4, stored at step i - 2, and its psi_n, Pi_n
+                        if (!need(here, landed(slot), landed_phase)) return false;
+                        F2 lap[4], e[4], y[4], o[4];
+                        star4_column<P, WB, WC, S::COMP>(a, wsite + wm * WSLOT, col, lap);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            e[c] = F2(lds2(esite + wm * ESLOT + c * EC));
+                            y[c] = F2(lds2(lf_smem + off_y + c * RC));
+                        }
+                        stage_b_pair<S::COMP>(a, col.mid<P>(0), col.mid<P>(1), col.mid<P>(2), col.mid<P>(3), lap, e, y, o);
+                        if constexpr (Src::kPatches)
+                            if (!peers_landed()) return false;
+                        if (in_box) {
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) *reinterpret_cast<float2 *>(a.out[c] + off) = o[c].v;
+                        }
+                        off += w.ks;
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            F2 z1, z2;
+                            col.sums<P>(c, z1, z2);
+                        }
+                    }
+                    __syncwarp();
+                    if (!release_plane()) return false;
+                    if (i >= 2) release_window();
+                    return true;
+                };
+                for (int i = 0;;) {
+                    if (!step(std::integral_constant<int, 0>{}, i)) return;
+                    if (++i == n) break;
+                    if (!step(std::integral_constant<int, 1>{}, i)) return;
+                    if (++i == n) break;
+                    if (!step(std::integral_constant<int, 2>{}, i)) return;
+                    if (++i == n) break;
                 }
-                ready = mbar_test_at(stored(ws), stored_phase);
-                const bool here = mbar_test_at(landed(slot), landed_phase);  // long since: sweep A has read the plane
-#pragma unroll
-                for (int c = 0; c < 4; ++c) col.in<P>(c) = F2(lds2(wz + c * WC));
-                if (i >= 4) {
-                    // (E, Q) of plane i with its d3, d4, stored at step i - 2, and its psi_n, Pi_n
-                    need(here, landed(slot), landed_phase);
-                    F2 lap[4], e[4], y[4], o[4];
-                    star4_column<P, WB, WC, S::COMP>(a, wsite + wm * WSLOT, col, lap);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        e[c] = F2(lds2(esite + wm * ESLOT + c * EC));
-                        y[c] = F2(lds2(lf_smem + off_y + c * RC));
-                    }
-                    stage_b_pair<S::COMP>(a, col.mid<P>(0), col.mid<P>(1), col.mid<P>(2), col.mid<P>(3), lap, e, y, o);
-                    if constexpr (Src::kPatches) peers_landed();
-                    if (in_box) {
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) *reinterpret_cast<float2 *>(a.out[c] + off) = o[c].v;
-                    }
-                    off += w.ks;
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        F2 z1, z2;
-                        col.sums<P>(c, z1, z2);
-                    }
-                }
-                __syncwarp();
-                release_plane();
-                if (i >= 2) release_window();
-            };
-            for (int i = 0;;) {
-                step(std::integral_constant<int, 0>{}, i);
-                if (++i == n) break;
-                step(std::integral_constant<int, 1>{}, i);
-                if (++i == n) break;
-                step(std::integral_constant<int, 2>{}, i);
-                if (++i == n || ended()) break;
+                // the item's last planes: sweep A is done with them, and nothing reads the last two window slots
+                for (int k = 0; k < 4; ++k)
+                    if (!release_plane()) return;
+                release_window();
+                release_window();
             }
-            if (ended()) break;
-            // the item's last planes: sweep A is done with them, and nothing reads the last two window slots
-            for (int k = 0; k < 4; ++k) release_plane();
-            release_window();
-            release_window();
-        }
+        };
+        march();
     }
     // no tile leaves while another may still tell it of a plane
     if constexpr (Src::kPatches) cluster_meet();

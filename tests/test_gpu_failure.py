@@ -83,3 +83,72 @@ def test_nonfinite_cells_are_counted(axs, dtype):
     import ctypes as C
     axs._lib.call("axs_count_nonfinite", C.byref(axs.fab(t, 2)), cnt.data_ptr(), None)
     assert int(cnt.item()) == 4
+
+
+@pytest.mark.parametrize("polls", [0, 1, 2, 5, 16, 64])
+def test_expired_waits_of_the_fused_step_store_nothing_unfinished(axs, polls):
+    """However few polls the waits have, wherever they then run out: a cell the
+    FP32 one-pass step has stored holds the step's result, every other cell what
+    it held before."""
+    L = axs._lib
+    n, bg = 64, axs.Background.expanding(2.0, 1.0, lambda0=2.0)
+    v = _state(n, 11, torch.float32).cuda()
+    lv = axs.PeriodicLevel(n, 0.5, dtype=torch.float32)
+    lv.tile_config = [cid for cid, name in lv.tile_configs() if name == "f32 fused 32x16 columns"][0]
+    lv.set_state(v)
+    right, dst = torch.zeros_like(lv.state), torch.full_like(lv.state, -77.0)
+    lv.step_to(right, bg, 1.0, 0.0, 0.1)
+    lv.device_status()
+    prev = L.set_device_wait_polls(polls)
+    try:
+        lv.step_to(dst, bg, 1.0, 0.0, 0.1)
+        torch.cuda.synchronize()
+    finally:
+        L.set_device_wait_polls(prev)
+    expired = False
+    try:
+        lv.device_status()
+    except L.AxsError as err:
+        expired = True
+        assert err.status == L.AXS_ERR_DEVICE_TIMEOUT
+    assert expired or polls > 0
+    ox, oy = lv.layout.x_offset, lv.layout.y_offset
+    got, want = (t[:, :, oy:oy + n, ox:ox + n] for t in (dst, right))
+    assert bool(((got == want) | (got == -77.0)).all()) and (expired or torch.equal(got, want))
+
+
+@pytest.mark.parametrize("polls", [0, 1, 2, 5, 16, 64])
+@pytest.mark.parametrize("n", [32, 64])  # clusters of 2 and 8 tiles
+def test_expired_waits_of_the_patch_step_store_nothing_unfinished(axs, n, polls):
+    """The same for patches, which are stepped in place by clusters of blocks that
+    wait for one another; the next step is right once the state is loaded again."""
+    from axion_strings_adaptive_gb300.amr import Patches
+    L = axs._lib
+    bg = axs.Background.expanding(2.0, 1.0, lambda0=2.0)
+    p = Patches(n, 200, 0.25, dtype=torch.float32)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    p.state.copy_(torch.randn(p.state.shape, generator=g, device="cuda") + 2.0)
+    before = p.state.clone()
+    p.step(bg, 1.0, 0.3, 0.05)
+    p.device_status()
+    right = p.state.clone()
+    assert not torch.equal(right, before)
+    p.state.copy_(before)
+    prev = L.set_device_wait_polls(polls)
+    try:
+        p.step(bg, 1.0, 0.3, 0.05)
+        torch.cuda.synchronize()
+    finally:
+        L.set_device_wait_polls(prev)
+    expired = False
+    try:
+        p.device_status()
+    except L.AxsError as err:
+        expired = True
+        assert err.status == L.AXS_ERR_DEVICE_TIMEOUT
+    assert expired or polls > 0
+    assert bool(((p.state == right) | (p.state == before)).all()) and (expired or torch.equal(p.state, right))
+    p.state.copy_(before)
+    p.step(bg, 1.0, 0.3, 0.05)
+    p.device_status()
+    assert torch.equal(p.state, right)
