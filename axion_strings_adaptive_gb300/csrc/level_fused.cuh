@@ -173,14 +173,27 @@ struct FusedBoxes {
 // that takes patches in turn; cs holds the elements of a patch in a component
 // plane, maps two tensor maps a patch (the second boxes the state). A plane is
 // overwritten by sweep B once it has landed in every tile of its patch: a tile
-// tells the others plane by plane (the kernel's peer barriers). 1638 patches of
-// 32^3: 0.86 ms a step, against 1.13 with all taps from shared memory, one patch
-// a cluster and a cluster barrier per plane; with a release at cluster scope in
-// what a tile tells the others, 1.07.
+// tells the others of every kTell planes (the kernel's peer barriers, one per kTell
+// ring slots; sweep A is 4 planes ahead of sweep B, so 4 have landed before the first
+// is to be stored). The telling releases and sweep B's wait acquires at cluster scope,
+// which puts the stores after the other tiles' loads. 1638 patches of 32^3: 0.82 ms a
+// step, against 1.13 with all taps from shared memory, one patch a cluster and a
+// cluster barrier per plane; telling of every plane costs 1.10, and doing that without
+// release and acquire, which no memory model orders, 0.86.
+// A peer barrier counts ntiles arrivals a round, whoever they come from. It
+// completes a round only when every tile has told of its planes, although one tile's
+// word may arrive after another's of the next round: a tile tells of round r + 1 (the
+// planes NS on) only after its own barrier has completed round r, since sweep B frees
+// the slots after that. Suppose a barrier were the first of all to complete a round r
+// that tile Z has not told of. Of the ntiles (r + 1) arrivals it has counted (rounds
+// from 0), at most r are Z's, so more than r + 1 are another tile's: that one has told
+// of round r + 1, and its own barrier completed round r earlier. And telling means
+// having landed, whichever tile hears of it first.
 struct FusedPatches {
     static constexpr bool kMapsInTable = true;
     static constexpr bool kPatches = true;
     static constexpr int kRows = 4, kPlanes = 4;  // ghost rows and planes below the valid cells
+    static constexpr int kTell = 4;               // sides are multiples of 32: items of whole groups
     __device__ __forceinline__ static FusedCursor begin(const SweepArgs<float> &a)
     {
         return {(int)blockIdx.x / a.ntiles, a.n_items};
@@ -250,8 +263,10 @@ __global__ void __launch_bounds__(S::THREADS, 1)
     extern __shared__ __align__(128) unsigned char lf_smem[];
     unsigned char *const win = lf_smem + (size_t)NS * SLOT, *const eqw = win + (size_t)U * WSLOT;
     // ring slots: landed, and read (by sweep B, last); window slots: stored, and read;
-    // of patches, ring slots: landed in every tile of the patch
-    __shared__ uint64_t bars[3 * NS + 2 * U];
+    // of patches, groups of ring slots: landed in every tile of the patch
+    constexpr int TELL = FusedPatches::kTell;
+    static_assert(NS % TELL == 0, "whole groups");
+    __shared__ uint64_t bars[2 * NS + 2 * U + NS / TELL];
     __shared__ int failed;
     const int tid = threadIdx.x, warp = tid >> 5;
     const bool lane0 = (tid & 31) == 0;
@@ -261,7 +276,7 @@ __global__ void __launch_bounds__(S::THREADS, 1)
         for (int k = 0; k < NS; ++k) {
             mbar_init(&bars[k], 1);
             mbar_init(&bars[NS + k], S::WB);
-            if constexpr (Src::kPatches) mbar_init(&bars[2 * NS + 2 * U + k], (uint32_t)a.ntiles);
+            if (Src::kPatches && k % TELL == 0) mbar_init(&bars[2 * NS + 2 * U + k / TELL], (uint32_t)a.ntiles);
         }
         for (int k = 0; k < U; ++k) {
             mbar_init(&bars[2 * NS + k], S::WA);
@@ -284,10 +299,10 @@ __global__ void __launch_bounds__(S::THREADS, 1)
     auto ring_read = [&](int k) { return bar0 + 8u * (NS + k); };
     auto stored = [&](int k) { return bar0 + 8u * (2 * NS + k); };
     auto win_read = [&](int k) { return bar0 + 8u * (2 * NS + U + k); };
-    auto peers = [&](int k) { return bar0 + 8u * (2 * NS + 2 * U + k); };
-    auto slow_wait = [&](uint32_t bar, uint32_t phase) -> bool {
+    auto peers = [&](int k) { return bar0 + 8u * (2 * NS + 2 * U + k / TELL); };
+    auto slow_wait = [&](uint32_t bar, uint32_t phase, auto cluster) -> bool {
         for (uint32_t it = 0; it < a.wait_polls; ++it) {
-            if (mbar_try_wait_at(bar, phase)) return true;
+            if (mbar_try_wait_at<decltype(cluster)::value>(bar, phase)) return true;
             if ((it & 63) == 63 && *(volatile int *)&failed) return false;
         }
         if (*(volatile int *)&failed) return false;
@@ -295,9 +310,11 @@ __global__ void __launch_bounds__(S::THREADS, 1)
         *(volatile int *)&failed = 1;
         return false;
     };
-    auto need = [&](bool ready, uint32_t bar, uint32_t phase) -> bool {  // the whole warp's
+    constexpr std::false_type here_only{};
+    // the whole warp's wait (cluster: for what another block of the cluster has told)
+    auto need = [&](bool ready, uint32_t bar, uint32_t phase, auto cluster) -> bool {
         if (__all_sync(0xffffffffu, ready)) return true;
-        return __all_sync(0xffffffffu, slow_wait(bar, phase)) != 0;
+        return __all_sync(0xffffffffu, slow_wait(bar, phase, cluster)) != 0;
     };
 
     // March of an item. Planes are numbered from z0 - 4. Step i = 0 .. len + 3: sweep A
@@ -329,7 +346,7 @@ __global__ void __launch_bounds__(S::THREADS, 1)
                 const int xc = a.ox - 4 + p.x0;  // padded column of the box's first column (16-byte aligned)
                 const bool lo = !Src::kPatches && p.y0 == 0, hi = !Src::kPatches && p.y0 + TY == p.ny;
                 for (int k = 0; k < p.len + 8; ++k) {
-                    if (!(ok = slow_wait(ring_read(slot), phase))) break;
+                    if (!(ok = slow_wait(ring_read(slot), phase, here_only))) break;
                     unsigned char *dst = lf_smem + (size_t)slot * SLOT;
                     uint64_t *bar = &bars[slot];
                     mbar_arrive_expect_tx(bar, S::SLOT_BYTES);
@@ -360,6 +377,21 @@ __global__ void __launch_bounds__(S::THREADS, 1)
             // (after an expired wait; bounded as well).
             for (int64_t v = sent > NS ? sent - NS : 0; v < sent; ++v)
                 mbar_wait_bounded(&bars[v % NS], (uint32_t)((v / NS) & 1), 1u << 20);
+        } else if (Src::kPatches && warp == S::WA + S::WB + 1) {
+            // ---- the warp that tells the patch's tiles, this one too, of the planes that
+            // have landed here (lane: the tile told)
+            int slot = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (FusedCursor cur = Src::begin(a); ok && Src::valid(cur); Src::next(cur, a))
+                for (int k = 0; k < a.nx + 2 * 4; ++k) {
+                    if (!(ok = need(false, landed(slot), phase, here_only))) break;
+                    if (slot % TELL == TELL - 1 && (tid & 31) < a.ntiles) mbar_arrive_cluster(peers(slot), tid & 31);
+                    if (++slot == NS) {
+                        slot = 0;
+                        phase ^= 1;
+                    }
+                }
         }
     } else
     if (warp < S::WA) {
@@ -396,9 +428,7 @@ __global__ void __launch_bounds__(S::THREADS, 1)
             if (off >= NS * SLOT) off -= NS * SLOT;
         };
         auto take_plane = [&](bool ready) -> bool {
-            if (!need(ready, landed(slot), landed_phase)) return false;
-            if constexpr (Src::kPatches)
-                if (tid < a.ntiles) mbar_arrive_cluster(peers(slot), tid);  // tid: the tile told
+            if (!need(ready, landed(slot), landed_phase, here_only)) return false;
             if (++slot == NS) {
                 slot = 0;
                 landed_phase ^= 1;
@@ -442,7 +472,7 @@ __global__ void __launch_bounds__(S::THREADS, 1)
                     next_off(off_mid);
                     const StageAPair sa = stage_a_pair<S::COMP>(a, col.mid<P>(0), col.mid<P>(1), col.mid<P>(2),
                                                                 col.mid<P>(3), lap[0], lap[1], lap[2], lap[3]);
-                    if (!need(free, win_read(ws), read_phase)) return false;
+                    if (!need(free, win_read(ws), read_phase, here_only)) return false;
                     unsigned char *const wz = wsite + ws * WSLOT, *const ez = esite + ws * ESLOT;
                     if (has_a) {
 #pragma unroll
@@ -482,12 +512,12 @@ __global__ void __launch_bounds__(S::THREADS, 1)
         int slot = 0, off_y = 4 * ((by + 4) * BX + bx + 4);  // ring slot of plane i, this site in it
         int ws = 0, wm = 0;                                  // window slots of steps i and i - 2
         uint32_t stored_phase = 0, landed_phase = 0;
+        // at the first plane of a group: the group has landed in all tiles
         auto peers_landed = [&]() -> bool {
-            return need(mbar_test_at(peers(slot), landed_phase), peers(slot), landed_phase);
+            if (slot % TELL != 0) return true;
+            return need(mbar_test_at<true>(peers(slot), landed_phase), peers(slot), landed_phase, std::true_type{});
         };
-        auto release_plane = [&]() -> bool {  // after the warp's reads of it
-            if constexpr (Src::kPatches)
-                if (!peers_landed()) return false;  // every plane: a tile is told once per round of a slot
+        auto release_plane = [&]() {  // after the warp's reads of it
             if (lane0) mbar_arrive_at(ring_read(slot));
             off_y += SLOT;
             if (++slot == NS) {
@@ -495,7 +525,6 @@ __global__ void __launch_bounds__(S::THREADS, 1)
                 off_y -= NS * SLOT;
                 landed_phase ^= 1;
             }
-            return true;
         };
         auto release_window = [&]() {
             if (lane0) mbar_arrive_at(win_read(wm));
@@ -516,7 +545,7 @@ __global__ void __launch_bounds__(S::THREADS, 1)
                 bool ready = false;
                 auto step = [&](auto ph, int i) -> bool {
                     constexpr int P = decltype(ph)::value;
-                    if (!need(ready, stored(ws), stored_phase)) return false;
+                    if (!need(ready, stored(ws), stored_phase, here_only)) return false;
                     const unsigned char *const wz = wsite + ws * WSLOT;
                     if (++ws == U) {
                         ws = 0;
@@ -524,11 +553,14 @@ __global__ void __launch_bounds__(S::THREADS, 1)
                     }
                     ready = mbar_test_at(stored(ws), stored_phase);
                     const bool here = mbar_test_at(landed(slot), landed_phase);  // long since: sweep A has read the plane
+                    // every group, stored or not: it keeps the rounds of `peers` apart
+                    if constexpr (Src::kPatches)
+                        if (!peers_landed()) return false;
 #pragma unroll
                     for (int c = 0; c < 4; ++c) col.in<P>(c) = F2(lds2(wz + c * WC));
                     if (i >= 4) {
                         // (E, Q) of plane i with its d3, d4, stored at step i - 2, and its psi_n, Pi_n
-                        if (!need(here, landed(slot), landed_phase)) return false;
+                        if (!need(here, landed(slot), landed_phase, here_only)) return false;
                         F2 lap[4], e[4], y[4], o[4];
                         star4_column<P, WB, WC, S::COMP>(a, wsite + wm * WSLOT, col, lap);
 #pragma unroll
@@ -537,8 +569,6 @@ __global__ void __launch_bounds__(S::THREADS, 1)
                             y[c] = F2(lds2(lf_smem + off_y + c * RC));
                         }
                         stage_b_pair<S::COMP>(a, col.mid<P>(0), col.mid<P>(1), col.mid<P>(2), col.mid<P>(3), lap, e, y, o);
-                        if constexpr (Src::kPatches)
-                            if (!peers_landed()) return false;
                         if (in_box) {
 #pragma unroll
                             for (int c = 0; c < 4; ++c) *reinterpret_cast<float2 *>(a.out[c] + off) = o[c].v;
@@ -552,7 +582,7 @@ __global__ void __launch_bounds__(S::THREADS, 1)
                         }
                     }
                     __syncwarp();
-                    if (!release_plane()) return false;
+                    release_plane();
                     if (i >= 2) release_window();
                     return true;
                 };
@@ -565,8 +595,9 @@ __global__ void __launch_bounds__(S::THREADS, 1)
                     if (++i == n) break;
                 }
                 // the item's last planes: sweep A is done with them, and nothing reads the last two window slots
-                for (int k = 0; k < 4; ++k)
-                    if (!release_plane()) return;
+                if constexpr (Src::kPatches)
+                    if (!peers_landed()) return;
+                for (int k = 0; k < 4; ++k) release_plane();
                 release_window();
                 release_window();
             }

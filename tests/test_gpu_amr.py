@@ -443,3 +443,22 @@ def test_fp32_fill_equals_fp64_fill(axs, block, theta, whole):
             # blocks (1, 0, 1) and (1, 0, 2) are neighbours in z
             if order[q] == (1, 0, 1):
                 np.testing.assert_array_equal(a[:, -4:, 4:-4, 6:-6], valid[order.index((1, 0, 2))][:, :4])
+
+
+@pytest.mark.parametrize("n,count", [(32, 1500), (64, 190)])  # clusters of 2 and 8 blocks, several patches each
+def test_tiles_of_a_patch_keep_off_planes_their_neighbours_still_load(axs, n, count):
+    """Patches are stepped in place by the tiles of a cluster at once. A plane that
+    were overwritten before a neighbouring tile has loaded it would show in that
+    patch alone: equal patches must stay equal, step after step."""
+    from axion_strings_adaptive_gb300.amr import Patches
+    bg = axs.Background.expanding(2.0, 1.0, lambda0=2.0)
+    p = Patches(n, count, 0.25, dtype=torch.float32)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    one = torch.randn((4, p.layout.patch_elems), generator=g, device="cuda") * 0.3 + 1.0
+    p.state.view(4, count, -1).copy_(one[:, None])
+    for s in range(12):
+        p.step(bg, 1.0, 0.02 * s, 0.02)
+    p.device_status()
+    got = p.state.view(4, count, -1)
+    assert bool(torch.isfinite(got).all()) and not torch.equal(got[:, 0], one)
+    assert torch.equal(got, got[:, :1].expand(-1, count, -1))
