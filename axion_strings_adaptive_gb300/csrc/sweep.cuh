@@ -279,6 +279,14 @@ __device__ __forceinline__ void lap_pair(const SweepArgs<float> &a, const float 
 struct TapSum {
     long long hi, lo;
 };
+// The high word of wT 2^(E - 26 - 28), E = (top >> 20) - 1023, by its exponent field.
+// Unsigned: the first sum passes 2^31 for most spacings and taps.
+__host__ __device__ constexpr int lap_scale_hi(int wt_hi, int top)
+{
+    return (int)((unsigned)wt_hi + ((unsigned)top & 0x7ff00000u) - ((1023u + 54u) << 20));
+}
+// dx = 0.1 (1/(12 dx^2) = 8.33), taps in [1, 2)
+static_assert(lap_scale_hi(0x4020aaaa, 0x3fffffff) == 0x3cc0aaaa, "no overflow on the way (a constant expression has none)");
 __device__ __forceinline__ void add_tap(TapSum &s, double f, int top)
 {
     const int h = __double2hiint(f), l = __double2loint(f);
@@ -309,10 +317,7 @@ __device__ __forceinline__ double lap_site(const SweepArgs<double> &a, double f0
         }
         add_tap(c, f0, top);
         const long long t = (16 * s1.hi - s2.hi - 90 * c.hi) + ((16 * s1.lo - s2.lo - 90 * c.lo) >> 26);
-        // 1/(12 dx^2) 2^(E - 26 - 28), E = (top >> 20) - 1023, by its exponent field
-        const double scale = __hiloint2double(__double2hiint(a.wT) + (top & 0x7ff00000) - ((1023 + 54) << 20),
-                                              __double2loint(a.wT));
-        return (double)t * scale;
+        return (double)t * __hiloint2double(lap_scale_hi(__double2hiint(a.wT), top), __double2loint(a.wT));
     }
     if (mx >= 0x7ff00000) {
         // an infinity or a NaN decides the sum alone (a run that has blown up is
