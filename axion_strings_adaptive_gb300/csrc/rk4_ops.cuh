@@ -311,6 +311,11 @@ template <typename T> inline void fill_step_constants(SweepArgs<T> &a, double dx
     a.wC = T(-7.5 * inv_dx2);
     // lap_site scales wT by powers of two within 2^+-554
     a.wT = T(inv_dx2 > 0x1p-400 && inv_dx2 < 0x1p400 ? inv_dx2 / 12.0 : 0.0);
+    if constexpr (std::is_same<T, double>::value) {
+        // 1 - 12 dx^2 wT from exact products (at most 2^-51, so the remainder fits)
+        const double x = 12.0 * a.wT, xl = std::fma(12.0, a.wT, -x), p = dx * dx, pl = std::fma(dx, dx, -p);
+        if (a.wT != 0.0) a.wT_lo = (int)std::nearbyint((std::fma(-x, p, 1.0) - xl * p - x * pl) * 0x1p64);
+    }
     a.h = T(dt);
     a.h_half = T(0.5 * dt);
     a.h2_quarter = T(0.25 * dt * dt);

@@ -22,6 +22,7 @@
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "axs_internal.cuh"
@@ -44,6 +45,7 @@ template <typename T> struct SweepArgs {
                                  // stencil arrays' layout (0 unless their rows are shifted, refined patches)
     T wA, wB, wC;                // lap = wA*S1 + wB*S2 + wC*f0 (S1/S2: sums of +-1 / +-2 neighbours)
     T wT;                        // 1/(12 dx^2): lap = wT (16 S1 - S2 - 90 f0); 0: not to be used (lap_site)
+    int wT_lo;                   // 2^64 times its relative remainder, 1 - 12 dx^2 wT (FP64)
     StageCoef<T> c1, c2, c4;     // stage coefficients at t, t + h/2, t + h
     T h, h_half, h2_quarter, h2_half, h_sixth, h_third, h2_sixth;
     // remainders of the FP32 weights and step fractions (exact value - FP32 value),
@@ -268,7 +270,11 @@ __device__ __forceinline__ void lap_pair(const SweepArgs<float> &a, const float 
 // and only T is converted. A tap m 2^e enters as (m >> 26) p and (m & 2^26 - 1) p
 // with p = +-2^(28 - (E - e)): two multiply-adds do the shift, the sign and the
 // sum. The sums are exact while every tap's exponent lies within 28 of E; T is
-// cut below 2^(E - 54). Against exact rationals its error is 3e-17 of the
+// rounded to multiples of 2^(E - 54). wT's own rounding would weigh every site's
+// Laplacian alike (2^-54 low for dx = 1/2: white noise after 10 steps was 1.3 (psi) and
+// 1.6 (Pi) times as far off as with the plain sum, now 1.1 and 1.2; fields cut off at 3
+// cells and more are nearer throughout), so T takes its remainder, where T has
+// more bits than the product keeps. Against exact rationals its error is 3e-17 of the
 // largest tap / dx^2 (rms, smooth fields; 3e-19 on nearly constant ones), where
 // the plain FP64 sum has 4e-16 (7e-16), and 3e-16 against 4e-16 on rough fields,
 // where the result's own rounding decides. Step at 256^3: 6.30 -> 3.74 ms, the
@@ -309,14 +315,15 @@ __device__ __forceinline__ double lap_site(const SweepArgs<double> &a, double f0
     // exponent fields: normal numbers from 2^-500 to 2^500, at most 28 apart
     const int top = mx | 0xfffff;
     if (__double2hiint(a.wT) != 0 && mn >= (523 << 20) && mx < (1523 << 20) && top - mn < (29 << 20)) {
-        TapSum s1{0, 0}, s2{0, 0}, c{0, 0};
+        TapSum s1{0, 0}, s2{0, -(1 << 25)}, c{0, 0};  // 2^25: the low sum is rounded, not cut
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
             add_tap(s1, n1[k], top);
             add_tap(s2, n2[k], top);
         }
         add_tap(c, f0, top);
-        const long long t = (16 * s1.hi - s2.hi - 90 * c.hi) + ((16 * s1.lo - s2.lo - 90 * c.lo) >> 26);
+        long long t = (16 * s1.hi - s2.hi - 90 * c.hi) + ((16 * s1.lo - s2.lo - 90 * c.lo) >> 26);
+        t += __mulhi((int)(t >> 32), a.wT_lo);
         return (double)t * __hiloint2double(lap_scale_hi(__double2hiint(a.wT), top), __double2loint(a.wT));
     }
     if (mx >= 0x7ff00000) {

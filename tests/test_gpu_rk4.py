@@ -338,3 +338,40 @@ def test_f32_rhs_of_part_of_a_box_equals_the_boxs(axs, ng):
         out = axs.new_fab((nx, ny, nz), 1, dtype=torch.float32)
         axs.eval_rhs(part, out, ng, 1, 0.5, c)
         assert torch.equal(axs.valid(out, 1), big[:, z:z + nz, y:y + ny, x:x + nx]), (x, y, z, nx, ny, nz)
+
+
+@pytest.mark.parametrize("dx", [0.5, 0.1, 0.3])
+def test_f64_laplacian_weighs_no_site_alike_wrong(axs, dx):
+    """What all sites' Laplacians have in common as an error: the slope of Pi's error after
+    one step on its increment, against extended precision. dt = 3/128 makes h/6, h/3 and
+    h^2/6 exact, so 1/(12 dx^2) is the one rounded weight; rounded to 53 bits and
+    used as it is, it gives slopes of -5.6e-17, -3.1e-17 and -7.0e-17. Bound: 2^-56 =
+    1.4e-17. (The rounding errors of 8192 values, 1.4e-16 of Pi at most each, give the
+    slope an uncertainty of 2e-18 where increments are of Pi's size, which they exceed.)"""
+    n, dt, ld = 16, 3.0 / 128.0, np.longdouble
+    v = np.random.default_rng(8).standard_normal((4, n, n, n))
+    v[2:] *= 0.2
+    bg = axs.Background.expanding(2.0, 1.0, lambda0=2.0)
+    lv = axs.PeriodicLevel(n, dx, dtype=torch.float64)
+    lv.set_state(_to_dev(v))
+    lv.advance(bg, 1.0, 0.0, dt, 1)
+    lv.device_status()
+    got = lv.get_state().cpu().numpy()
+
+    def rhs(y, tau):
+        c = bg.rhs_coeffs(tau)
+        out = np.concatenate([y[2:], y[:2] * ld(c.kappa) - ld(c.lambda_) / 2 * ((y[:2] ** 2).sum(0) - ld(c.R2)) * y[:2]])
+        lap = -90 * y[:2]
+        for ax in (1, 2, 3):
+            for k, w in ((1, 16), (2, -1)):
+                lap = lap + w * (np.roll(y[:2], k, ax) + np.roll(y[:2], -k, ax))
+        out[2:] += lap / (12 * ld(dx) * ld(dx))
+        return out
+
+    y, h = v.astype(ld), ld(dt)
+    k1 = rhs(y, 1.0)
+    k2 = rhs(y + h / 2 * k1, 1.0 + dt / 2)
+    k3 = rhs(y + h / 2 * k2, 1.0 + dt / 2)
+    ref = y + h / 6 * (k1 + 2 * k2 + 2 * k3 + rhs(y + h * k3, 1.0 + dt))
+    err, inc = (got - ref)[2:], (ref - y)[2:]
+    assert abs(float((err * inc).sum() / (inc ** 2).sum())) < 2.0 ** -56
