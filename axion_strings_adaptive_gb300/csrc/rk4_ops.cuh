@@ -128,7 +128,8 @@ __device__ __forceinline__ void stage_a(const SweepArgs<T> &a, const T (&lap)[4]
             const double l1 = lap[0][v], l2 = lap[1][v];
             double f11, f12, f21, f22;
             rhs_pair_f64(a.c1, p1, p2, l1, l2, f11, f12);
-            rhs_pair_f64(a.c2, p1 + a1, p2 + a2, fma(a.h_half, lap[2][v], l1), fma(a.h_half, lap[3][v], l2), f21, f22);
+            rhs_pair_f64(a.c2, fma(a.h_half, ctr[2][v], p1), fma(a.h_half, ctr[3][v], p2),
+                         fma(a.h_half, lap[2][v], l1), fma(a.h_half, lap[3][v], l2), f21, f22);
             const double hq1 = 2.0 * a1, hq2 = 2.0 * a2;
             const double s1 = (f11 + f21) + l1, s2 = (f12 + f22) + l2;
             o[0][v] = fma(a.h2_quarter, f11, a1);
