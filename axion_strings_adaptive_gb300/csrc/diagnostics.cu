@@ -22,6 +22,7 @@
 #include <type_traits>
 
 #include "axs_internal.cuh"
+#include "fp64_pos.cuh"
 #include "sweep.cuh"
 #include "winding.cuh"
 
@@ -162,49 +163,6 @@ __device__ __forceinline__ bool diff1_pairs(float m2, float m1, float p1, float 
            __fadd_rn(r, __fsub_rn(rest, bound)) == r;
 }
 
-// A positive double within float range cut to float, and a normal float
-// widened, both by integer operations.
-__device__ __forceinline__ bool float_sized(double d)
-{
-    const int h = __double2hiint(d);
-    return h > 0x39b00000 && h < 0x46300000;  // about 2^-100 to 2^100
-}
-__device__ __forceinline__ float cut_to_float(double d)
-{
-    return __int_as_float(__funnelshift_l(__double2loint(d), __double2hiint(d) - 0x38000000, 3));
-}
-__device__ __forceinline__ double widen_normal(float x)
-{
-    const int u = __float_as_int(x);
-    return __hiloint2double((u >> 3) + 0x38000000, u << 29);
-}
-
-// 1/d and sqrt(d) of d > 0 in FP64 from a float estimate, for the few FP64
-// operations they take (3 and 5): 1/d by one step of third order, r (1 + e + e^2)
-// with e = 1 - d r (the truncated geometric series; e^3 < 2^-60), sqrt(d) by two
-// Newton steps on the residual d - s^2.
-__device__ __forceinline__ double recip_pos(double d)
-{
-    if (!float_sized(d)) return 1.0 / d;
-    const double r = widen_normal(__fdividef(1.f, cut_to_float(d)));
-    const double e = fma(-d, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-__device__ __forceinline__ double sqrt_pos(double d)
-{
-    if (!float_sized(d)) return sqrt(d);
-    const float y = rsqrtf(cut_to_float(d));
-    const double h = widen_normal(0.5f * y);
-    double s = d * widen_normal(y);
-    s = fma(fma(-s, s, d), h, s);
-    return fma(fma(-s, s, d), h, s);
-}
-// d >= 0, or a NaN, by its bits (a comparison is an FP64 operation)
-__device__ __forceinline__ bool positive(double d)
-{
-    return (__double2hiint(d) | __double2loint(d)) != 0 && __double2hiint(d) <= 0x7ff00000;
-}
-
 // The seven per-cell energy terms (EnergyKernel.hpp:130-190) and the masking
 // weight (Masking.hpp:75-93) from psi, Pi and the six diff1 values, in math
 // type M: double as the reference computes them, or float for the
@@ -334,7 +292,7 @@ __device__ __forceinline__ void cell_energy(const CellConst<double> &k, int sche
     term[5] = pot * s4;                                        // radial mass
     wgt = 1.0;
     if (scheme == AXS_MASK_B) {
-        wgt = (sqrt_pos(psi_sq) * k.inv_R >= k.threshold) ? 1.0 : 0.0;
+        wgt = root_reaches(psi_sq, k.inv_R, k.threshold) ? 1.0 : 0.0;
     } else if (scheme != AXS_MASK_NONE) {
         // 1 + r / f_a, r = |psi| / R - 1
         const double f = (1.0 - 0.70710678118654752440) + sqrt_pos(psi_sq) * (k.inv_R * 0.70710678118654752440);
