@@ -141,6 +141,7 @@ SIGNATURES = {
     "axs_level_layout_for": (_i32, [_i32, _i32, _i32, _i32, C.POINTER(LevelLayout)]),
     "axs_level_tile_config_count": (C.c_int, [_i32]),
     "axs_level_tile_config_name": (C.c_char_p, [_i32, _i32]),
+    "axs_level_tile_config_resolve": (_i32, [C.POINTER(LevelC)]),
     "axs_level_fill_ghosts": (_i32, [C.POINTER(LevelC), _ptr]),
     "axs_level_import_fab": (_i32, [C.POINTER(LevelC), C.POINTER(Fab), _ptr]),
     "axs_level_export_fab": (_i32, [C.POINTER(LevelC), C.POINTER(Fab), _ptr]),
@@ -183,6 +184,7 @@ SIGNATURES = {
     "axs_ensemble_box_layout": (_i32, [_i32, _i32, C.POINTER(_i32), _i32, C.POINTER(EnsembleBox)]),
     "axs_ensemble_tile_config_count": (_i32, [_i32]),
     "axs_ensemble_tile_config_name": (C.c_char_p, [_i32, _i32]),
+    "axs_ensemble_tile_config_id": (_i32, [_i32, C.c_char_p]),
     "axs_ensemble_init": (_i32, [C.POINTER(EnsembleC), C.POINTER(EnsemblePlan), _ptr]),
     "axs_ensemble_fill_ghosts": (_i32, [C.POINTER(EnsembleC), _ptr]),
     "axs_ensemble_rk4_advance": (_i32, [C.POINTER(EnsembleC), C.POINTER(EnsemblePlan), C.POINTER(BackgroundC), _dbl,

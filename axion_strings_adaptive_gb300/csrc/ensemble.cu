@@ -368,9 +368,10 @@ static bool fused_fits(const int32_t *dims, int nboxes, int ty)
     return true;
 }
 
-// The default (tile_config 0) is the first entry of its table that suits
-// every box: the fused step (0.58 ms per step on a mixed 32^3..128^3
-// ensemble on GB300), else the fastest two-sweep tiling there (1.01 ms). The
+// The default (tile_config 0) is, from a table's default entry on, the first that
+// suits every box: the fused step (0.58 ms per step on a mixed 32^3..128^3
+// ensemble on GB300), else the fastest two-sweep tiling there (1.01 ms). Ids are
+// positions: callers keep them, so new tilings go to the end of a table. The
 // 16-wide tiles leave no idle columns on boxes whose width is a multiple of
 // 16 but read 96-byte rows.
 static const EnsTiling kEnsF32[] = {
@@ -385,11 +386,12 @@ static const EnsTiling kEnsF32[] = {
     EnsConfig<float, 2, 32, 8, 8, 3, true>::entry("f32 v2 32x8 ring8 l2"),
 };
 static const EnsTiling kEnsF64[] = {
-    // small blocks: the level's default, for its reason (16x4: 1.03-1.12x as long)
-    EnsConfig<double, 1, 16, 8, 6, 4>::entry("f64 v1 16x8 ring6"),
     EnsConfig<double, 1, 32, 8, 6, 2>::entry("f64 v1 32x8 ring6"),
     EnsConfig<double, 1, 16, 16, 6, 2>::entry("f64 v1 16x16 ring6"),
+    // the default: the level's, for its reason (16x4: 1.03-1.12x as long)
+    EnsConfig<double, 1, 16, 8, 6, 4>::entry("f64 v1 16x8 ring6"),
 };
+static int ens_default(int32_t dtype) { return dtype == AXS_F64 ? 3 : 1; }
 
 static int ens_config_count(int32_t dtype)
 {
@@ -403,16 +405,16 @@ static const EnsTiling *ens_config(int32_t dtype, int32_t id)
     const int n = ens_config_count(dtype);
     if (n == 0 || id < 0 || id > n) return nullptr;
     const EnsTiling *tab = dtype == AXS_F64 ? kEnsF64 : kEnsF32;
-    return &tab[id == 0 ? 0 : id - 1];
+    return &tab[(id == 0 ? ens_default(dtype) : id) - 1];
 }
 
 // The tiling an ensemble runs for tile_config id: id 0 resolves to the first
-// entry that suits its boxes.
+// entry from the default on that suits its boxes.
 static const EnsTiling *ens_config_for(const axs_ensemble *e, int32_t id)
 {
     if (id != 0) return ens_config(e->dtype, id);
     const int n = ens_config_count(e->dtype);
-    for (int i = 1; i <= n; ++i) {
+    for (int i = ens_default(e->dtype); i <= n; ++i) {
         const EnsTiling *c = ens_config(e->dtype, i);
         if (!c->fused || fused_fits(e->dims, e->nboxes, c->ty)) return c;
     }
@@ -490,6 +492,17 @@ int axs_ensemble_box_layout(int32_t dtype, int32_t nboxes, const int32_t *dims, 
     out->x_offset = geo.g[box].ox;
     out->y_offset = geo.g[box].oy;
     return AXS_OK;
+}
+
+int32_t axs_ensemble_tile_config_id(int32_t dtype, const char *name)
+{
+    if (name == nullptr) return 0;
+    const int n = ens_config_count(dtype);
+    for (int i = 1; i <= n; ++i)
+        if (std::strcmp(ens_config(dtype, i)->name, name) == 0) return i;
+    // an earlier name of the fused step
+    if (dtype == AXS_F32 && std::strcmp(name, "f32 fused 32x16 ring6 t640") == 0) return 1;
+    return 0;
 }
 
 int32_t axs_ensemble_tile_config_count(int32_t dtype) { return ens_config_count(dtype); }

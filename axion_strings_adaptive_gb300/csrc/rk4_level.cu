@@ -305,18 +305,20 @@ static const TileConfigEntry kF32Configs[] = {
     {"f32 fused 32x16 ring7 t640", &FusedConfig<32, 16>::run, nullptr},
 };
 static const TileConfigEntry kF64Configs[] = {
+    {"f64 v1 32x8 ring6", &SweepConfig<double, 1, 32, 8, 6, 2>::run, nullptr},
+    {"f64 v2 32x8 ring6", &SweepConfig<double, 2, 32, 8, 6, 2>::run, nullptr},
+    {"f64 v2 32x16 ring6", &SweepConfig<double, 2, 32, 16, 6, 1>::run, nullptr},
+    {"f64 v1 32x4 ring7", &SweepConfig<double, 1, 32, 4, 7, 3>::run, nullptr},
+    {"f64 v1 32x8 ring6 l2", &SweepConfig<double, 1, 32, 8, 6, 2, true>::run, nullptr},
     // The default. FP64 sweeps alternate between the integer Laplacian sums and the
     // FP64 stage arithmetic; 4 blocks of four warps a SM are rarely in the same phase,
     // which two blocks of eight are (32x8: 3.51 ms a step at 256^3, this 2.79). 16x4, 6
     // or 7 blocks of two warps with half as many rows of halo again, took 1.04x as long
     // at 256^3, 1.06-1.09x at 96^3 to 224^3, 0.95-1.07x at 128^3 and below 96^3.
     {"f64 v1 16x8 ring6", &SweepConfig<double, 1, 16, 8, 6, 4>::run, nullptr},
-    {"f64 v1 32x8 ring6", &SweepConfig<double, 1, 32, 8, 6, 2>::run, nullptr},
-    {"f64 v2 32x8 ring6", &SweepConfig<double, 2, 32, 8, 6, 2>::run, nullptr},
-    {"f64 v2 32x16 ring6", &SweepConfig<double, 2, 32, 16, 6, 1>::run, nullptr},
-    {"f64 v1 32x4 ring7", &SweepConfig<double, 1, 32, 4, 7, 3>::run, nullptr},
-    {"f64 v1 32x8 ring6 l2", &SweepConfig<double, 1, 32, 8, 6, 2, true>::run, nullptr},
 };
+// Ids are positions: callers keep them, so new tilings go to the end of a table.
+constexpr int kDefaultF32 = 0, kDefaultF64 = 5;
 
 static int config_count(int32_t dtype)
 {
@@ -329,19 +331,26 @@ static int config_count(int32_t dtype)
 // One step, fused / two sweeps: 48^3 13.4 / 10.1 us, 64x35x70 14.8 / 11.5, 64^3 15.0 / 14.0,
 // 80^3 22.8 / 23.8; two steps 24.1 / 19.8, 27.0 / 22.6, 27.3 / 28.0, 39.8 / 47.0.
 constexpr int64_t kFusedLeastSites = 300000;
-static const TileConfigEntry kSmallF32Config = {"", &FusedConfig<32, 16>::Fallback::run,
-                                                &FusedConfig<32, 16, true>::Fallback::run};
+
+// The entry of a runner, the first of those that have it.
+static const TileConfigEntry *config_with(int32_t dtype, int (*run)(const SweepRunArgs &))
+{
+    const TileConfigEntry *tab = dtype == AXS_F64 ? kF64Configs : kF32Configs;
+    for (int i = 0; i < config_count(dtype); ++i)
+        if (tab[i].run == run) return &tab[i];
+    return nullptr;
+}
 
 static const TileConfigEntry *config_for(int32_t dtype, int32_t id)
 {
     const TileConfigEntry *tab = dtype == AXS_F64 ? kF64Configs : kF32Configs;
     if (id < 0 || id > config_count(dtype)) return nullptr;
-    return &tab[id == 0 ? 0 : id - 1];
+    return &tab[id == 0 ? (dtype == AXS_F64 ? kDefaultF64 : kDefaultF32) : id - 1];
 }
 static const TileConfigEntry *config_for(const axs_level *lv)
 {
     if (lv->tile_config == 0 && lv->dtype == AXS_F32 && (int64_t)lv->nx * lv->ny * lv->nz < kFusedLeastSites)
-        return &kSmallF32Config;
+        return config_with(AXS_F32, &FusedConfig<32, 16>::Fallback::run);
     return config_for(lv->dtype, lv->tile_config);
 }
 
@@ -351,7 +360,7 @@ using Runner = int (*)(const SweepRunArgs &);
 static Runner runner_for(const axs_level *lv, const TileConfigEntry *cfg)
 {
     if (lv->dtype == AXS_F32 && (lv->flags & AXS_LEVEL_COMPENSATED_FP32))
-        return cfg->run_comp != nullptr ? cfg->run_comp : kF32Configs[0].run_comp;
+        return cfg->run_comp != nullptr ? cfg->run_comp : kF32Configs[kDefaultF32].run_comp;
     return cfg->run;
 }
 
@@ -416,6 +425,18 @@ const char *axs_level_tile_config_name(int32_t dtype, int32_t id)
     if (dtype != AXS_F32 && dtype != AXS_F64) return nullptr;
     const TileConfigEntry *c = config_for(dtype, id);
     return c ? c->name : nullptr;
+}
+
+int32_t axs_level_tile_config_resolve(const axs_level *lv)
+{
+    if (lv == nullptr || (lv->dtype != AXS_F32 && lv->dtype != AXS_F64)) return 0;
+    const TileConfigEntry *cfg = config_for(lv);
+    if (cfg == nullptr) return 0;
+    if (lv->dtype == AXS_F32 && (lv->flags & AXS_LEVEL_COMPENSATED_FP32) && cfg->run_comp == nullptr)
+        cfg = &kF32Configs[kDefaultF32];
+    using Fused = FusedConfig<32, 16>;
+    cfg = config_with(lv->dtype, cfg->run == &Fused::run && !Fused::applies(lv) ? &Fused::Fallback::run : cfg->run);
+    return (int32_t)(cfg - (lv->dtype == AXS_F64 ? kF64Configs : kF32Configs)) + 1;
 }
 
 int axs_level_fill_ghosts(const axs_level *lv, void *stream)

@@ -66,6 +66,13 @@ class Ensemble:
         return [(i, lib.axs_ensemble_tile_config_name(d, i).decode())
                 for i in range(1, lib.axs_ensemble_tile_config_count(d) + 1)]
 
+    def tile_config_id(self, name: str) -> int:
+        """The id of a tiling by its name or an earlier one (axs_ensemble_tile_config_id)."""
+        cid = L.lib().axs_ensemble_tile_config_id(_DT[self.dtype], name.encode())
+        if cid == 0:
+            raise KeyError(name)
+        return cid
+
     def box_view(self, b: int, arena: torch.Tensor | None = None) -> torch.Tensor:
         """(ncomp, nz, ny, nx) view of box b's valid cells in an arena (default: the state)."""
         t = self.state if arena is None else arena

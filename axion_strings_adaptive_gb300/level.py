@@ -211,10 +211,15 @@ class PeriodicLevel:
         d = _DT[self.dtype]
         return [(i, lib.axs_level_tile_config_name(d, i).decode()) for i in range(1, lib.axs_level_tile_config_count(d) + 1)]
 
+    def running_config(self) -> tuple:
+        """(id, name) of the tiling this level's steps run (axs_level_tile_config_resolve)."""
+        cid = L.lib().axs_level_tile_config_resolve(C.byref(self.c))
+        return cid, L.lib().axs_level_tile_config_name(_DT[self.dtype], cid).decode()
+
     def autotune(self, bg: Background, tau_i: float, dt: float, steps: int = 4, repeats: int = 2,
                  stream=None) -> dict:
         """Time every compiled tiling on this level (the two-sweep tilings and
-        the one-pass fused step; full RK4 steps, CUDA events) and keep the
+        the one-pass fused step; full RK4 steps, CUDA events), each once, and keep the
         fastest. An even step count times the fused step alone (an odd one ends
         with a copy back to the state). The state is saved and restored, so the
         level's contents are unchanged. Returns {name: ms_per_step}."""
@@ -223,6 +228,8 @@ class PeriodicLevel:
         best = (float("inf"), self.c.tile_config)
         for cid, name in self.tile_configs():
             self.c.tile_config = cid
+            if self.running_config()[0] != cid:  # another entry's steps under this name
+                continue
             self.advance(bg, tau_i, 0.0, dt, 1, stream)  # warm-up (sets up the kernel)
             ms = float("inf")
             for _ in range(repeats):

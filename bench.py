@@ -605,11 +605,6 @@ def run_native(args):
                    "rk4_sweep_B": sum(b_.elapsed_time(c_) for a_, b_, c_ in marks) / steps}
         return ms, per, clocks
 
-    def level_config_name(level):
-        # tile_config 0 is the table's first entry (the default tiling)
-        return A._lib.lib().axs_level_tile_config_name(A._lib.AXS_F32 if level.dtype == torch.float32
-                                                       else A._lib.AXS_F64, level.tile_config).decode()
-
     # algorithmic words per site and launch (read + write, each compulsory word once)
     WORDS = {"rk4_sweep_A": 12, "rk4_sweep_B": 16, "rk4_fused_level": 8}
 
@@ -624,7 +619,7 @@ def run_native(args):
         lv32.tile_config = ids[args.tile_config]
     elif not args.no_autotune:
         tune32 = lv32.autotune(bg, TAU_I, DT)
-    cfg32 = level_config_name(lv32)
+    cfg32 = lv32.running_config()[1]
     ms, per32, clocks = timed_run(lv32, args.steps, args.warmup, sample_clocks=True)
     ms_max = allmax(ms)
     value = ws * n ** 3 * args.steps / (ms_max * 1e-3)
@@ -757,7 +752,7 @@ def run_native(args):
         ms64, per64, _ = timed_run(lv64, k64, 1)
         v64 = ws * n ** 3 * k64 / (allmax(ms64) * 1e-3)
         fp64 = {"value": v64, "ms_per_step": ms64 / k64, "steps": k64, "kernel_ms": per64,
-                "tile_config": level_config_name(lv64),
+                "tile_config": lv64.running_config()[1],
                 "autotune_ms_per_step": tune64}
         del lv64
         torch.cuda.empty_cache()

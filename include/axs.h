@@ -223,6 +223,11 @@ int axs_level_layout_for(int32_t dtype, int32_t nx, int32_t ny, int32_t nz, axs_
  * autotuner can time each on the caller's level and set axs_level.tile_config. */
 int axs_level_tile_config_count(int32_t dtype);
 const char *axs_level_tile_config_name(int32_t dtype, int32_t id);
+/* The id of the tiling that a level's steps run: what id 0 stands for on a level of
+ * its size, the two sweeps where the level does not suit the one-pass step, and the
+ * current entry for an earlier name of it. Reads the level's description, not its
+ * buffers; 0 for a bad dtype or id. */
+int32_t axs_level_tile_config_resolve(const axs_level *lv);
 
 /* Periodic ghost columns/rows of the 4 state components (call after writing
  * the state's valid cells by any other means). */
@@ -553,10 +558,10 @@ int axs_level_tag_cells(const axs_level *lv, const axs_tag_params *p, uint8_t *t
  * A two-sweep tiling runs every RK4 sweep as ONE persistent launch over the
  * work items of all boxes. The fused tiling runs every RK4 step as one launch
  * (plus one for the boxes' periodic padding), with the work arena's first 4
- * planes as the second state buffer; it takes boxes whose ny is a multiple of
- * 16 and whose nx is even. tile_config 0 is the first tiling (by id) that
- * suits every box: the fused one where it fits. After every advance the result
- * and its padding are in the state arena.
+ * planes as the second state buffer; it takes boxes with ny = 16 or ny >= 20.
+ * tile_config 0 is, in FP32, the first tiling (by id) that suits every box: the
+ * fused one where it fits. After every advance the result and its padding are
+ * in the state arena.
  * ------------------------------------------------------------------------- */
 typedef struct axs_ensemble {
     int32_t dtype;
@@ -576,7 +581,7 @@ typedef struct axs_ensemble_box {
 } axs_ensemble_box;
 
 typedef struct axs_ensemble_plan {
-    int32_t tile_config; /* in: index from axs_ensemble_tile_config_name (1..count), 0 = the first that suits */
+    int32_t tile_config; /* in: index from axs_ensemble_tile_config_name (1..count), 0 = the default */
     int32_t z_chunk;     /* in: target z planes per work item, 0 = automatic */
     int64_t n_items;     /* out: work items of one sweep (all boxes) */
     int32_t grid_a;      /* out: persistent grid of sweep A */
@@ -589,6 +594,8 @@ int axs_ensemble_sizes(int32_t dtype, int32_t nboxes, const int32_t *dims, int64
                        int64_t *work_bytes, int64_t *table_bytes);
 int axs_ensemble_box_layout(int32_t dtype, int32_t nboxes, const int32_t *dims, int32_t box, axs_ensemble_box *out);
 int32_t axs_ensemble_tile_config_count(int32_t dtype);
+/* The id of a tiling by name, earlier names of it included; 0: none has it. */
+int32_t axs_ensemble_tile_config_id(int32_t dtype, const char *name);
 const char *axs_ensemble_tile_config_name(int32_t dtype, int32_t id);
 
 /* Build the device table for plan->tile_config / plan->z_chunk and fill the

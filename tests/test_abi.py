@@ -256,3 +256,38 @@ def test_level_flags_are_checked_without_gpu(L):
     assert b"unknown level flags" in lib.axs_last_error()
     lv.flags = L.LEVEL_COMPENSATED_FP32
     assert lib.axs_level_rk4_advance(C.byref(lv), C.byref(bg), 1.0, 0.0, 0.1, 0, None) == L.AXS_OK  # no-op
+
+
+def test_tile_config_ids_and_names_stay(L):
+    """Ids are kept by callers: every id keeps its tiling. Names that the one-pass
+    step had before select it, and a level says which tiling it runs."""
+    lib = L.lib()
+    f32, f64 = L.AXS_F32, L.AXS_F64
+    names = lambda fn, dt, ids: [fn(dt, i).decode() for i in ids]  # noqa: E731
+    assert names(lib.axs_level_tile_config_name, f64, range(1, 6)) == \
+        ["f64 v1 32x8 ring6", "f64 v2 32x8 ring6", "f64 v2 32x16 ring6", "f64 v1 32x4 ring7", "f64 v1 32x8 ring6 l2"]
+    assert names(lib.axs_level_tile_config_name, f32, (2, 5, 13, 14)) == \
+        ["f32 v2 64x8 ring8", "f32 v2 32x8 ring8", "f32 v2 32x8 ring8 l2", "f32 v4 64x16 ring6 l2"]
+    assert names(lib.axs_ensemble_tile_config_name, f64, range(1, 4)) == \
+        ["f64 v1 32x8 ring6", "f64 v1 16x16 ring6", "f64 v1 16x8 ring6"]
+    assert names(lib.axs_ensemble_tile_config_name, f32, (2, 3, 9)) == \
+        ["f32 v2 64x8 ring8", "f32 v2 32x8 ring8", "f32 v2 32x8 ring8 l2"]
+    find = lib.axs_ensemble_tile_config_id
+    assert find(f32, b"f32 fused 32x16 ring6 t640") == find(f32, b"f32 fused 32x16 columns") == 1
+    assert find(f32, b"f32 v2 32x8 ring8") == 3 and find(f64, b"f64 v1 16x8 ring6") == 3
+    assert find(f32, b"f32") == find(f64, b"f32 v2 32x8 ring8") == find(7, b"f32 v2 32x8 ring8") == find(f32, None) == 0
+
+    def runs(dt, n, cid, flags=0):
+        lv = L.LevelC(None, None, dt, *n, 0.5, cid, flags)
+        got = lib.axs_level_tile_config_resolve(C.byref(lv))
+        return got and lib.axs_level_tile_config_name(dt, got).decode()
+
+    fused, sweeps = "f32 fused 32x16 columns", "f32 v2 32x8 ring8 l2"
+    assert runs(f32, (512, 512, 512), 0) == fused and runs(f32, (48, 48, 48), 0) == sweeps
+    assert runs(f64, (512, 512, 512), 0) == "f64 v1 16x8 ring6"
+    for cid in range(1, lib.axs_level_tile_config_count(f32) + 1):
+        name = lib.axs_level_tile_config_name(f32, cid).decode()
+        assert runs(f32, (64, 64, 64), cid) == (fused if "fused" in name else name)
+        assert runs(f32, (64, 18, 64), cid) == (sweeps if "fused" in name else name)  # no row count of its
+        assert runs(f32, (64, 64, 64), cid, L.LEVEL_COMPENSATED_FP32) == (sweeps if name == sweeps else fused)
+    assert runs(f32, (64, 64, 64), 99) == runs(7, (64, 64, 64), 0) == 0 and lib.axs_level_tile_config_resolve(None) == 0
