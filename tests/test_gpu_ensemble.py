@@ -152,3 +152,41 @@ def test_plan_must_match_ensemble(axs):
                torch.cuda.current_stream().cuda_stream)
     e.advance(bg, 1.0, 0.0, 0.1, 1)
     e.device_status()
+
+
+@pytest.mark.parametrize("steps", [3, 4])
+def test_fused_ensemble_with_overlapping_tile_rows(axs, steps):
+    """Boxes whose rows are no multiple of the tile's 16 (40 and 28: evenly spread
+    tile rows that overlap) have to run the one-pass step, odd counts and padding
+    included."""
+    bg = axs.Background.expanding(2.0, 1.0, lambda0=2.0)
+    ref = [lv.get_state() for lv in _levels(axs, DIMS, torch.float32, bg, steps)]
+    for zc in (0, 3, 7):
+        e = _ensemble(axs, DIMS, torch.float32)
+        e.init(e.tile_config_id("f32 fused 32x16 ring6 t640"), zc)
+        e.advance(bg, 1.0, 0.0, 0.1, steps)
+        e.device_status()
+        for b in range(len(DIMS)):
+            assert torch.equal(e.get_box(b), ref[b]), (zc, b)
+        after = e.state.clone()
+        e.fill_ghosts()
+        assert torch.equal(e.state, after)
+
+
+@pytest.mark.parametrize("ny", [9, 18])
+def test_fused_ensemble_refuses_other_row_counts(axs, ny):
+    """One box of 9 or of 18 rows: the one-pass step refuses the ensemble, and the
+    default is the two sweeps, bit for bit."""
+    from axion_strings_adaptive_gb300 import _lib as L
+    dims = [(32, 32, 32), (32, ny, 24), (16, 16, 8)]
+    bg = axs.Background.expanding(2.0, 1.0, lambda0=2.0)
+    ref = [lv.get_state() for lv in _levels(axs, dims, torch.float32, bg, 3)]
+    e = _ensemble(axs, dims, torch.float32)
+    with pytest.raises(L.AxsError) as err:
+        e.init(_fused_id(e), 0)
+    assert err.value.status == L.AXS_ERR_UNSUPPORTED
+    e.init(0, 0)
+    e.advance(bg, 1.0, 0.0, 0.1, 3)
+    e.device_status()
+    for b in range(len(dims)):
+        assert torch.equal(e.get_box(b), ref[b]), b
