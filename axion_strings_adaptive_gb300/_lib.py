@@ -141,7 +141,7 @@ SIGNATURES = {
     "axs_level_layout_for": (_i32, [_i32, _i32, _i32, _i32, C.POINTER(LevelLayout)]),
     "axs_level_tile_config_count": (C.c_int, [_i32]),
     "axs_level_tile_config_name": (C.c_char_p, [_i32, _i32]),
-    "axs_level_tile_config_resolve": (_i32, [C.POINTER(LevelC)]),
+    "axs_level_tile_config_resolve": (_i32, [C.POINTER(LevelC), _i32]),
     "axs_level_fill_ghosts": (_i32, [C.POINTER(LevelC), _ptr]),
     "axs_level_import_fab": (_i32, [C.POINTER(LevelC), C.POINTER(Fab), _ptr]),
     "axs_level_export_fab": (_i32, [C.POINTER(LevelC), C.POINTER(Fab), _ptr]),

@@ -326,11 +326,30 @@ static int config_count(int32_t dtype)
                             : (int)(sizeof(kF32Configs) / sizeof(kF32Configs[0]));
 }
 
-// The default of small FP32 levels: the fused step's march (12 planes to start, 20
-// warps in turn) and its padding launch take longer there than two short launches.
-// One step, fused / two sweeps: 48^3 13.4 / 10.1 us, 64x35x70 14.8 / 11.5, 64^3 15.0 / 14.0,
-// 80^3 22.8 / 23.8; two steps 24.1 / 19.8, 27.0 / 22.6, 27.3 / 28.0, 39.8 / 47.0.
-constexpr int64_t kFusedLeastSites = 300000;
+// The default of FP32 levels that are small, or thin in y or z: there the fused step's
+// march (12 planes to start on every chunk, 20 warps in turn) and its padding launch
+// take longer than the sweeps' two short launches. The rule compares what the two take
+// in microseconds: of the fused step the planes of its longest block and 2 a step, and
+// 5 more where the result comes back from the second buffer; of the two sweeps 9 a step
+// and 30 per million sites of whole 32 x 8 tiles. Measured, fused / two sweeps, a call of
+// one step and one of four: 64x64x80 23.2 / 21.8 us and 73.9 / 82.5; 256x20x100 31.5 / 27.3
+// and 107 / 111; 300x300x8 37.3 / 30.1 and 131 / 116; 256x16x100 26.1 / 22.8 and 90.7 / 82.5
+// (here the four are decided wrongly); 100x96x96 39.3 / 40.6 and 140 / 163; 8x200x200
+// 39.7 / 47.5 and 143 / 189 (either path runs whole tiles, so narrow levels need no rule of
+// their own). Over 364 calls on levels of 50 000 to 6 million sites the default takes 1.002 as
+// long as the better path, 1.11 at most; the fused step alone 1.053, the sweeps 1.136.
+static bool fused_pays(const axs_level *lv, int nsteps, bool copy_back)
+{
+    const int cols = (lv->nx + 31) / 32;
+    const double two = nsteps * (9.0 + 30e-6 * 32.0 * cols * ((lv->ny + 7) / 8 * 8) * lv->nz);
+    if (1.05 * two <= nsteps * 15.0) return false;  // a march of one plane takes longer
+    const int sms = device_sm_count() > 0 ? device_sm_count() : 152;
+    int zchunk = 0, grid = 0;
+    int64_t items = 0;
+    plan_chunks(cols * fused_tiles_ny(lv->ny, 16), lv->nz, sms, zchunk, items, grid);
+    const double planes = (double)((items + grid - 1) / grid) * (zchunk + 8) + 4.0;
+    return nsteps * (planes + 2.0) + (copy_back ? 5.0 : 0.0) < 1.05 * two;
+}
 
 // The entry of a runner, the first of those that have it.
 static const TileConfigEntry *config_with(int32_t dtype, int (*run)(const SweepRunArgs &))
@@ -347,9 +366,9 @@ static const TileConfigEntry *config_for(int32_t dtype, int32_t id)
     if (id < 0 || id > config_count(dtype)) return nullptr;
     return &tab[id == 0 ? (dtype == AXS_F64 ? kDefaultF64 : kDefaultF32) : id - 1];
 }
-static const TileConfigEntry *config_for(const axs_level *lv)
+static const TileConfigEntry *config_for(const axs_level *lv, int nsteps, bool in_place)
 {
-    if (lv->tile_config == 0 && lv->dtype == AXS_F32 && (int64_t)lv->nx * lv->ny * lv->nz < kFusedLeastSites)
+    if (lv->tile_config == 0 && lv->dtype == AXS_F32 && !fused_pays(lv, nsteps, in_place && (nsteps & 1)))
         return config_with(AXS_F32, &FusedConfig<32, 16>::Fallback::run);
     return config_for(lv->dtype, lv->tile_config);
 }
@@ -368,7 +387,7 @@ constexpr int kStagesOnly = 4;  // sweep mask: run_stages, in the default tiling
 static int run_sweeps(const axs_level *lv, const LevelGeom &g, const axs_background *bg, double tau_i, double t0,
                       double dt, int nsteps, int mask, cudaStream_t st)
 {
-    const TileConfigEntry *cfg = config_for(lv);
+    const TileConfigEntry *cfg = config_for(lv, nsteps, true);
     AXS_REQUIRE(cfg != nullptr, AXS_ERR_INVALID_ARGUMENT, "tile_config %d out of range (0..%d)", lv->tile_config,
                 config_count(lv->dtype));
     SweepRunArgs r{lv, &g, bg, tau_i, t0, dt, nsteps, mask, st, nullptr};
@@ -427,10 +446,11 @@ const char *axs_level_tile_config_name(int32_t dtype, int32_t id)
     return c ? c->name : nullptr;
 }
 
-int32_t axs_level_tile_config_resolve(const axs_level *lv)
+int32_t axs_level_tile_config_resolve(const axs_level *lv, int32_t nsteps)
 {
-    if (lv == nullptr || (lv->dtype != AXS_F32 && lv->dtype != AXS_F64)) return 0;
-    const TileConfigEntry *cfg = config_for(lv);
+    LevelGeom g;
+    if (lv == nullptr || nsteps < 1 || level_geom(lv->dtype, lv->nx, lv->ny, lv->nz, g)) return 0;
+    const TileConfigEntry *cfg = config_for(lv, nsteps, true);
     if (cfg == nullptr) return 0;
     if (lv->dtype == AXS_F32 && (lv->flags & AXS_LEVEL_COMPENSATED_FP32) && cfg->run_comp == nullptr)
         cfg = &kF32Configs[kDefaultF32];
@@ -554,7 +574,7 @@ int axs_level_rk4_step_to(const axs_level *lv, void *dst_state, const axs_backgr
         AXS_REQUIRE(bg->a_inv > 1.0, AXS_ERR_INVALID_ARGUMENT, "a_inv must exceed 1");
         AXS_REQUIRE(tau_i + t > 0.0, AXS_ERR_INVALID_ARGUMENT, "conformal time must stay positive");
     }
-    const TileConfigEntry *cfg = config_for(lv);
+    const TileConfigEntry *cfg = config_for(lv, 1, false);
     AXS_REQUIRE(cfg != nullptr, AXS_ERR_INVALID_ARGUMENT, "tile_config %d out of range (0..%d)", lv->tile_config,
                 config_count(lv->dtype));
     SweepRunArgs r{lv, &g, bg, tau_i, t, dt, 1, 3, (cudaStream_t)stream, dst_state};

@@ -211,9 +211,9 @@ class PeriodicLevel:
         d = _DT[self.dtype]
         return [(i, lib.axs_level_tile_config_name(d, i).decode()) for i in range(1, lib.axs_level_tile_config_count(d) + 1)]
 
-    def running_config(self) -> tuple:
-        """(id, name) of the tiling this level's steps run (axs_level_tile_config_resolve)."""
-        cid = L.lib().axs_level_tile_config_resolve(C.byref(self.c))
+    def running_config(self, nsteps: int = 2) -> tuple:
+        """(id, name) of the tiling that `nsteps` steps run (axs_level_tile_config_resolve)."""
+        cid = L.lib().axs_level_tile_config_resolve(C.byref(self.c), int(nsteps))
         return cid, L.lib().axs_level_tile_config_name(_DT[self.dtype], cid).decode()
 
     def autotune(self, bg: Background, tau_i: float, dt: float, steps: int = 4, repeats: int = 2,

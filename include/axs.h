@@ -223,11 +223,11 @@ int axs_level_layout_for(int32_t dtype, int32_t nx, int32_t ny, int32_t nz, axs_
  * autotuner can time each on the caller's level and set axs_level.tile_config. */
 int axs_level_tile_config_count(int32_t dtype);
 const char *axs_level_tile_config_name(int32_t dtype, int32_t id);
-/* The id of the tiling that a level's steps run: what id 0 stands for on a level of
- * its size, the two sweeps where the level does not suit the one-pass step, and the
- * current entry for an earlier name of it. Reads the level's description, not its
- * buffers; 0 for a bad dtype or id. */
-int32_t axs_level_tile_config_resolve(const axs_level *lv);
+/* The id of the tiling that nsteps steps of axs_level_rk4_advance run: what id 0 stands
+ * for on a level of its size, the two sweeps where the level does not suit the one-pass
+ * step, and the current entry for an earlier name of it. Reads the level's
+ * description, not its buffers; 0 for what axs_level_rk4_advance refuses of it. */
+int32_t axs_level_tile_config_resolve(const axs_level *lv, int32_t nsteps);
 
 /* Periodic ghost columns/rows of the 4 state components (call after writing
  * the state's valid cells by any other means). */

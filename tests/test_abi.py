@@ -277,9 +277,9 @@ def test_tile_config_ids_and_names_stay(L):
     assert find(f32, b"f32 v2 32x8 ring8") == 3 and find(f64, b"f64 v1 16x8 ring6") == 3
     assert find(f32, b"f32") == find(f64, b"f32 v2 32x8 ring8") == find(7, b"f32 v2 32x8 ring8") == find(f32, None) == 0
 
-    def runs(dt, n, cid, flags=0):
+    def runs(dt, n, cid, flags=0, steps=2):
         lv = L.LevelC(None, None, dt, *n, 0.5, cid, flags)
-        got = lib.axs_level_tile_config_resolve(C.byref(lv))
+        got = lib.axs_level_tile_config_resolve(C.byref(lv), steps)
         return got and lib.axs_level_tile_config_name(dt, got).decode()
 
     fused, sweeps = "f32 fused 32x16 columns", "f32 v2 32x8 ring8 l2"
@@ -290,4 +290,12 @@ def test_tile_config_ids_and_names_stay(L):
         assert runs(f32, (64, 64, 64), cid) == (fused if "fused" in name else name)
         assert runs(f32, (64, 18, 64), cid) == (sweeps if "fused" in name else name)  # no row count of its
         assert runs(f32, (64, 64, 64), cid, L.LEVEL_COMPENSATED_FP32) == (sweeps if name == sweeps else fused)
-    assert runs(f32, (64, 64, 64), 99) == runs(7, (64, 64, 64), 0) == 0 and lib.axs_level_tile_config_resolve(None) == 0
+    assert runs(f32, (64, 64, 64), 99) == runs(7, (64, 64, 64), 0) == lib.axs_level_tile_config_resolve(None, 2) == 0
+    # the default goes by what the steps take: thin and small levels, where a single step has
+    # its result copied back and the sweeps' launches are the shorter ones
+    for n, one, four in [((48, 48, 48), sweeps, sweeps), ((64, 64, 80), sweeps, fused), ((256, 20, 100), sweeps, fused),
+                         ((300, 300, 8), sweeps, sweeps), ((128, 300, 8), sweeps, fused), ((32, 128, 128), sweeps, fused),
+                         ((96, 96, 96), fused, fused), ((8, 200, 200), fused, fused), ((28, 160, 160), fused, fused),
+                         ((512, 36, 64), fused, fused), ((200, 150, 90), fused, fused), ((4, 16, 1), sweeps, sweeps),
+                         ((1024, 1024, 1024), fused, fused)]:
+        assert (runs(f32, n, 0, steps=1), runs(f32, n, 0, steps=4)) == (one, four), n
