@@ -863,11 +863,17 @@ constexpr int FTX = 32, FTY = 16;  // energy32_kernel's tile
 static_assert(FTX * FTY == 2 * kDiagThreads, "two cells per thread");
 constexpr int kStripW = 31, kStripRows = 8, kStripPairs = kStripRows / 2;
 constexpr int kStripQueue = 512;  // a warp's queued columns
+// Columns with pierced cells from which the columns next to them are queued as well, of the
+// strip's 31: from 16 on, fields cut off at 5 cells took 0.93 ms where this takes 0.86, the
+// others the same.
+constexpr int kStripDense = 24;
 constexpr int kFinderBlocks = 2;  // per SM
-static_assert(kStripQueue >= 3 * kStripW && kStripRows <= 8 && kStripRows % 2 == 0,
+static_assert(kStripQueue >= 3 * 32 && kStripRows <= 8 && kStripRows % 2 == 0,
               "an empty queue takes three planes' columns; rows are bits of a byte");
 // A lane's column of cells in a plane: pierced xy, yz, zx plaquettes, bit per row, in bits
-// 0-7, 8-15 and 16-23, the lane above; none pierced: to be taken through the exact path.
+// 0-7, 8-15 and 16-23, the lane in bits 24-28; none pierced: to be taken through the exact
+// path, or a column whose vertices the column before it takes.
+constexpr unsigned kVerticesOnly = 1u << 29;
 struct StripColumn {
     unsigned pierced;
     int z;
@@ -1000,31 +1006,60 @@ __device__ __noinline__ StripCounts strip_drain(const DiagView &v, const DiagCon
     float acc = 0.f, comp = 0.f;
     // VelocityKernel.hpp:37-141: gamma^2 v^2 of the 4 corners of every pierced plaquette of
     // a column (fields are zero outside the view's ghost region). The warp goes through the
-    // vertex rows that any lane needs together, so that its loads stay row segments.
+    // vertex rows that any lane needs together, so that its loads stay row segments. A lane
+    // computes the vertices at its own x, in planes z and z + 1; those at x + 1 come from the
+    // next lane where it has that column (a dense network's mostly do), else from memory
+    // too. A row's fields are fetched while the one before is computed. 320^3, pass with
+    // energies, list and velocities: white noise 1.35 -> 1.22 ms (1.20 with gamma^2 v^2 at every
+    // vertex instead), fields cut off at 3 cells 1.21 -> 1.09 (1.12), at 5 cells 0.98 -> 0.86
+    // (1.06), at 8 cells 0.78 -> 0.68 (1.04); without the fetch ahead 1.26, 1.16, 1.00, 0.73.
     auto velocity = [&](int x, int y0, int z, unsigned pierced) {
-        const int x1 = v.wx && x + 1 == v.nx ? 0 : x + 1, z1 = v.wz && z + 1 == v.nz ? 0 : z + 1;
-        const bool onx = v.wx || x + 1 < v.nx + v.ox, onz = v.wz || z + 1 < v.nz + v.oz;
-        const T *p0 = job.base + x + v.ox + (int64_t)(z + v.oz) * v.ks, *p1 = p0 + (int64_t)(z1 - z) * v.ks;
-        const int64_t right = x1 - x;
-        // vertices (x, y) and (x + 1, y) of plane z (up = 0) or z + 1
-        auto gv = [&](int y, int up) -> F2 {
-            const int yw = v.wy && y == v.ny ? 0 : y;
-            const bool on = (v.wy || y < v.ny + v.oy) && (!up || onz);
-            const T *c = (up ? p1 : p0) + (int64_t)(yw + v.oy) * v.js;
-            F2 f[4];
+        const int z1 = v.wz && z + 1 == v.nz ? 0 : z + 1;
+        const bool onz = v.wz || z + 1 < v.nz + v.oz;
+        const T *p0 = job.base + v.ox + (int64_t)v.oy * v.js + (int64_t)(z + v.oz) * v.ks;
+        const int64_t up = (int64_t)(z1 - z) * v.ks;
+        // the fields at the vertices (xv, y) of planes z and z + 1
+        auto fetch = [&](int xv, int y, F2 (&f)[4]) {
+            const int xw = v.wx && xv == v.nx ? 0 : xv, yw = v.wy && y == v.ny ? 0 : y;
+            const bool on = (v.wx || xv < v.nx + v.ox) && (v.wy || y < v.ny + v.oy);
+            const T *c = p0 + xw + (int64_t)yw * v.js;
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
                 f[m].v.x = on ? (float)__ldg(c + m * v.cs) : 0.f;
-                f[m].v.y = on && onx ? (float)__ldg(c + m * v.cs + right) : 0.f;
+                f[m].v.y = on && onz ? (float)__ldg(c + m * v.cs + up) : 0.f;
             }
-            return vertex_gv(f[0], f[1], f[2], f[3], q);
         };
         const unsigned mine = (pierced | pierced >> 8 | pierced >> 16) & 0xffu, vertices = mine | mine << 1;
-        F2 low(0.f), low1(0.f);  // rows k and k + 1, planes z and z + 1
-        for (unsigned rows = __reduce_or_sync(0xffffffffu, vertices); rows; rows &= rows - 1) {
+        // whether the next lane has column x + 1, and the rows that the lane before takes from this one
+        const int x_next = __shfl_down_sync(0xffffffffu, x, 1), y_next = __shfl_down_sync(0xffffffffu, y0, 1),
+                  z_next = __shfl_down_sync(0xffffffffu, z, 1);
+        const bool next = lane < 31 && x_next == x + 1 && y_next == y0 && z_next == z;
+        const unsigned asked = __shfl_up_sync(0xffffffffu, next ? vertices : 0u, 1);
+        const unsigned own = lane ? vertices | asked : vertices;
+        F2 low(0.f), low1(0.f);  // rows k and k + 1 at x and x + 1, planes z and z + 1
+        unsigned rows = __reduce_or_sync(0xffffffffu, vertices);
+        F2 f[4], f1[4];  // a row ahead
+#pragma unroll
+        for (int m = 0; m < 4; ++m) f[m] = f1[m] = F2(0.f);
+        auto fetch_row = [&]() {
+            const int y = __ffs(rows) - 1;
+            if (own >> y & 1) fetch(x, y0 + y, f);
+            if (!next && (vertices >> y & 1)) fetch(x + 1, y0 + y, f1);
+        };
+        if (rows) fetch_row();
+        while (rows) {
             const int y = __ffs(rows) - 1, k = y - 1;
-            if (vertices >> y & 1) {
-                const F2 high = gv(y0 + y, 0), high1 = gv(y0 + y, 1);
+            const bool here = vertices >> y & 1;
+            const F2 c0 = f[0], c1 = f[1], c2 = f[2], c3 = f[3], d0 = f1[0], d1 = f1[1], d2 = f1[2], d3 = f1[3];
+            rows &= rows - 1;
+            if (rows) fetch_row();
+            const F2 g = vertex_gv(c0, c1, c2, c3, q);
+            F2 g1;
+            g1.v.x = __shfl_down_sync(0xffffffffu, g.v.x, 1);
+            g1.v.y = __shfl_down_sync(0xffffffffu, g.v.y, 1);
+            if (here && !next) g1 = vertex_gv(d0, d1, d2, d3, q);
+            if (here) {
+                const F2 high(g.v.x, g1.v.x), high1(g.v.y, g1.v.y);
                 if ((mine << 1) >> y & 1) {
                     float s = 0.f;  // corners 000 100 110 010, 000 010 011 001, 000 001 101 100
                     if (pierced >> k & 1) s += low.v.x + low.v.y + high.v.y + high.v.x;
@@ -1039,10 +1074,14 @@ __device__ __noinline__ StripCounts strip_drain(const DiagView &v, const DiagCon
             }
         }
     };
-    for (int i0 = 0; i0 < n; i0 += 32) {
-        const StripColumn e = i0 + lane < n ? queue[i0 + lane] : StripColumn{0u, 0};
-        const unsigned pierced = e.pierced & 0xffffffu;
-        const int dx = e.pierced >> 24;
+    // Velocities: 31 columns at a time, the last lane with the first of the next 31, which it
+    // only computes the vertices of.
+    constexpr int kTake = VEL ? 31 : 32;
+    for (int i0 = 0; i0 < n; i0 += kTake) {
+        const StripColumn e = i0 + lane < n ? queue[i0 + lane] : StripColumn{kVerticesOnly, 0};
+        const bool take = lane < kTake && !(e.pierced & kVerticesOnly);
+        const unsigned pierced = take ? e.pierced & 0xffffffu : 0u;
+        const int dx = e.pierced >> 24 & 31u;
         const int64_t plane = (int64_t)v.nx * v.ny;
         if (job.list != nullptr) {
             int incl = __popc(pierced);
@@ -1062,7 +1101,7 @@ __device__ __noinline__ StripCounts strip_drain(const DiagView &v, const DiagCon
             }
         }
         // the pierced cells, then the exact path, four columns at a time, a row a lane
-        unsigned exact = __ballot_sync(0xffffffffu, i0 + lane < n && !pierced), some = pierced;
+        unsigned exact = __ballot_sync(0xffffffffu, take && !pierced), some = pierced;
         int x = job.x0 + dx, y = job.y0, z = e.z;
         while (true) {
             if constexpr (VEL) velocity(x, y, z, some);
@@ -1284,13 +1323,14 @@ __global__ void __launch_bounds__(kDiagThreads, kFinderBlocks)
                             if (keep >> k & 1) tags[cell + (int64_t)v.nx * k] = any >> k & 1;
                 }
                 cnt_p += __popc(pxy | pyz << 8 | pzx << 16);
-                // queue the pierced cells (where anyone asks which they are), and the column of an inexact lane
                 // queue the lane's column if it is inexact, or pierced where anyone asks which cells are
                 const bool put = inexact || ((VEL || list != nullptr) && any != 0);
-                const unsigned with = __ballot_sync(0xffffffffu, put);
-                if (put)
-                    queue[queued + __popc(with & ((1u << lane) - 1))] =
-                        StripColumn{pxy | pyz << 8 | pzx << 16 | (unsigned)lane << 24, zs + j - 1};
+                unsigned with = __ballot_sync(0xffffffffu, put);
+                // with velocities, on a plane with many: also the columns next to them, for their vertices
+                if (VEL && __popc(with) >= kStripDense) with |= with << 1;
+                if (with >> lane & 1)
+                    queue[queued + __popc(with & ((1u << lane) - 1))] = StripColumn{
+                        pxy | pyz << 8 | pzx << 16 | (unsigned)lane << 24 | (put ? 0u : kVerticesOnly), zs + j - 1};
                 queued += __popc(with);
             }
             X0 = X1;
@@ -1305,7 +1345,7 @@ __global__ void __launch_bounds__(kDiagThreads, kFinderBlocks)
             if (j + 1 <= len) step(j + 1, p0, p1, p2);
             if (j + 2 <= len) step(j + 2, p1, p2, p0);
             j += 3;
-        } while (j <= len && queued <= kStripQueue - 3 * kStripW);
+        } while (j <= len && queued <= kStripQueue - 3 * 32);
         zs += min(j - 1, len);  // the last vertex plane's cells are still to do
         if (queued) {
             __syncwarp();
