@@ -190,3 +190,16 @@ def test_fused_ensemble_refuses_other_row_counts(axs, ny):
     e.device_status()
     for b in range(len(dims)):
         assert torch.equal(e.get_box(b), ref[b]), b
+
+
+@pytest.mark.parametrize("n,count", [(24, 16), (40, 6), (48, 4), (64, 2)])
+def test_small_fused_ensembles_have_an_item_a_block(axs, n, count):
+    """Few boxes, which can be cut so that every SM has one work item at most: a
+    second item on some of them doubles the step's length. Whatever the cut, the
+    step is the levels', bit for bit (the other tests' z-chunk targets)."""
+    dims = [(n, n, n)] * count
+    e = _ensemble(axs, dims, torch.float32)
+    e.init(_fused_id(e), 0)
+    tiles = count * -(-n // 32) * -(-n // 16)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert tiles <= e.plan.n_items <= sms
