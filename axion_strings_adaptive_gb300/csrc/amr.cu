@@ -931,12 +931,6 @@ static int fill_smem_attr()
 // ring cells are copies, by their 32-byte pieces of rows. 256^3 with 1638 patches of
 // 32^3: 1.09 -> 0.72 ms, blending 1.15 -> 0.83 ms (tiles of 16 x 16 columns in three
 // passes through shared memory, 45 % of their columns in the ring).
-#ifndef FOFF
-#define FOFF uint32_t
-#endif
-#ifndef FB
-#define FB 4
-#endif
 constexpr int kFillThreads = 128;
 constexpr int kFillRow = 28;  // parents of a row segment: 32 lanes less two on either side
 // ring widths in parents; in x the ring's 6 cells and the 2 of padding next to them, whole 32-byte

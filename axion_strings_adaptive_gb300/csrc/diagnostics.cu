@@ -10,8 +10,10 @@
 // field at each corner, fmod fold into (-pi, pi], lround of the sum / 2 pi.
 // Edges whose |dtheta| lies within 1e-12 of pi are counted as "near ties":
 // only there could a different correctly-rounded-to-1-ulp atan2 flip a fold.
-// All per-cell energy/velocity arithmetic is FP64 whatever the field
-// precision; sums go per thread -> warp shuffle -> block -> per-block partial
+// Per-cell energy/velocity terms are FP64 whatever the field precision, unless the
+// caller asks for FP32 terms on FP32 fields (per_cell_fp32); of FP32 fields the
+// gradients are floats, as the reference has them, formed without FP64 where that is
+// sure to give the same float. Sums go per thread -> warp shuffle -> block -> per-block partial
 // in scratch -> a single-block finalize in a fixed order (deterministic, no
 // floating-point atomics).
 #include <climits>
@@ -443,8 +445,8 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
             zin = v.wz || (z >= -v.oz && z < v.nz + v.oz);
             return (int64_t)(wrap_or_self(z, v.nz, v.wz) + v.oz) * v.ks;
         };
-        // psi of plane z (za - 2 <= z <= za + len + 1) sits in slot (z - za + 2) mod 6,
-        // Pi of vertex plane z (za <= z <= za + len) in slot (z - za) mod 3
+        // psi of plane z (za - 2 <= z <= za + len + 1) sits in slot (z - za + 2) mod
+        // kPsiSlots, Pi of vertex plane z (za <= z <= za + len) in slot (z - za) mod kPiSlots
         auto psi_slot = [&](int z) { return (z - za + 2) % kPsiSlots; };
         auto load_psi = [&](int z) {
             bool zin;

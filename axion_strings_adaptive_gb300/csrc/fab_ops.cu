@@ -307,7 +307,7 @@ __device__ __forceinline__ double twice(double x)
     return __dmul_rn(2.0, x);
 }
 
-// FP64 form of rk4_combine_kernel below: the same expressions, cells numbered
+// FP64 form of rk4_combine_f32_kernel below: the same expressions, cells numbered
 // through (FP64-bound like the RHS; rows of any length fill the warps),
 // components on grid y. 97x75x50: 29.3 -> 21.9 us, 96^3: 53 -> 50.
 __global__ void __launch_bounds__(256) rk4_combine_f64_kernel(const axs_fab d, const axs_fab u, const axs_fab k1,
@@ -346,21 +346,20 @@ __global__ void lincomb_kernel(const axs_fab d, const axs_fab x, T b, const axs_
     }
 }
 
-// FP32; FP64 above
-template <typename T>
-__global__ void rk4_combine_kernel(const axs_fab d, const axs_fab u, const axs_fab k1, const axs_fab k2,
-                                   const axs_fab k3, const axs_fab k4, T h6, int ncomp)
+// FP32: rows of cells, a warp each (FP64 above)
+__global__ void rk4_combine_f32_kernel(const axs_fab d, const axs_fab u, const axs_fab k1, const axs_fab k2,
+                                       const axs_fab k3, const axs_fab k4, float h6, int ncomp)
 {
     const int rows = d.ny * d.nz * ncomp, lane = threadIdx.x & 31;
     for (int r = row_warp(); r < rows; r += row_warps()) {
         const RowIdx q = row_index(r, d.ny, d.nz);
         auto row = [&](const axs_fab &f) {
-            return static_cast<const T *>(f.data) + q.c * f.cstride + fab_off(f, 0, q.j, q.k);
+            return static_cast<const float *>(f.data) + q.c * f.cstride + fab_off(f, 0, q.j, q.k);
         };
-        const T *ur = row(u), *a = row(k1), *b = row(k2), *c = row(k3), *e = row(k4);
-        T *dr = static_cast<T *>(d.data) + q.c * d.cstride + fab_off(d, 0, q.j, q.k);
+        const float *ur = row(u), *a = row(k1), *b = row(k2), *c = row(k3), *e = row(k4);
+        float *dr = static_cast<float *>(d.data) + q.c * d.cstride + fab_off(d, 0, q.j, q.k);
         for (int i0 = lane; i0 < d.nx; i0 += 64) {
-            T v[2][5];
+            float v[2][5];
 #pragma unroll
             for (int w = 0; w < 2; ++w) {
                 const int i = i0 + 32 * w;
@@ -370,7 +369,7 @@ __global__ void rk4_combine_kernel(const axs_fab d, const axs_fab u, const axs_f
             for (int w = 0; w < 2; ++w) {
                 const int i = i0 + 32 * w;
                 if (i < d.nx) {
-                    const T sum = rn_add(rn_add(rn_add(v[w][0], rn_mul(T(2), v[w][1])), rn_mul(T(2), v[w][2])), v[w][3]);
+                    const float sum = rn_add(rn_add(rn_add(v[w][0], rn_mul(2.f, v[w][1])), rn_mul(2.f, v[w][2])), v[w][3]);
                     dr[i] = rn_add(v[w][4], rn_mul(h6, sum));
                 }
             }
@@ -798,7 +797,7 @@ int axs_rk4_combine(const axs_fab *dst, const axs_fab *uold, const axs_fab *k1, 
         rk4_combine_f64_kernel<<<cell_grid(*dst, 4), 256, 0, st>>>(*dst, *uold, *k1, *k2, *k3, *k4, dt / 6.0,
                                                                   cell_count(*dst));
     else
-        rk4_combine_kernel<float><<<g, 256, 0, st>>>(*dst, *uold, *k1, *k2, *k3, *k4, (float)(dt / 6.0), 4);
+        rk4_combine_f32_kernel<<<g, 256, 0, st>>>(*dst, *uold, *k1, *k2, *k3, *k4, (float)(dt / 6.0), 4);
     return launch_status("rk4_combine");
 }
 

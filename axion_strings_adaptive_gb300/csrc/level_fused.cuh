@@ -20,7 +20,7 @@
 // sweeps; in return sweep A runs on (TX+4)(TY+4) sites per TX*TY.
 //
 // Columns in registers. The march is bound by the shared-memory pipe, the FP32
-// pipe and issue together (76 %, 64 % and 65 % busy), not by HBM, so the work
+// pipe and issue together (70 %, 62 % and 71 % busy at 256^3), not by HBM, so the work
 // per plane is kept to arithmetic. A thread owns two neighbouring sites for the
 // whole march and keeps their column, of (psi, Pi) for sweep A or (d3, d4) for
 // sweep B, in registers as the differences the z taps are made of
@@ -35,7 +35,7 @@
 // warps of 80 registers fill the register file (one CTA per SM); setmaxnreg
 // moves the producer's to the others (88 for sweep A, 96 for sweep B: at 80
 // both spilled and ran 40 % slower).
-// Measured, this kernel alone at 512^3: 1.64 ms, against 2.57 ms with all taps
+// Measured, this kernel alone at 512^3: 1.67 ms, against 2.57 ms with all taps
 // from shared memory and a block barrier per plane; the same columns in 12
 // warps that ran both sweeps took 2.34 ms (three warps a scheduler left the
 // latencies of shared loads and additions open). Window slots: with 5 instead

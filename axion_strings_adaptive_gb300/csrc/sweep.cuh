@@ -225,10 +225,11 @@ __device__ __forceinline__ void rhs_adjoint_pair(const StageCoef<T> &c, T u1, T 
 
 // The FP32 Laplacian of two neighbouring sites x, x+1 from their taps: xl =
 // f(x-2, x-1), f0 = f(x, x+1), xr = f(x+2, x+3) along the row, the y neighbour
-// pairs, and the z neighbours' sums z1 = sum(f+-1 - f0), z2 = sum(f+-2 - f0). The stencil as differences from the centre, lap = wA
-// sum(f+-1 - f0) + wB sum(f+-2 - f0): a neighbour within a factor 2 of f0 gives
-// an exact difference, so the -30 f0 term of the plain sum does not cancel
-// against the neighbours. f - f0 is formed as f + (-f0), the same IEEE result.
+// pairs, and the z neighbours' sums z1 = sum(f+-1 - f0), z2 = sum(f+-2 - f0). The
+// stencil as differences from the centre, lap = wA sum(f+-1 - f0) + wB sum(f+-2 - f0):
+// a neighbour within a factor 2 of f0 gives an exact difference, so the -30 f0 term of
+// the plain sum does not cancel against the neighbours. f - f0 is formed as f + (-f0),
+// the same IEEE result.
 // Every FP32 sweep evaluates its stencils through this function. The x+-1 taps
 // go site by site: their pairs straddle the register pairs the packed
 // instructions need, and f(x+1) - f(x) serves both sites (negated, exactly).
@@ -279,9 +280,9 @@ __device__ __forceinline__ void lap_pair(const SweepArgs<float> &a, const float 
 // the plain FP64 sum has 4e-16 (7e-16), and 3e-16 against 4e-16 on rough fields,
 // where the result's own rounding decides. Step at 256^3: 6.30 -> 3.74 ms, the
 // FP64 pipe now 65 % busy with the stage arithmetic (78 operations a site and
-// step against 154), and 3.03 ms in smaller blocks (the FP64 tilings). Other taps (a zero or subnormal, one of
-// 2^-28 of its neighbours, exponents whose scale would leave the double range)
-// take the FP64 sum.
+// step against 154), and 3.03 ms in smaller blocks (the FP64 tilings). Other taps (a
+// zero or subnormal, one of 2^-28 of its neighbours, exponents whose scale would leave
+// the double range) take the FP64 sum.
 struct TapSum {
     long long hi, lo;
 };
@@ -327,8 +328,10 @@ __device__ __forceinline__ double lap_site(const SweepArgs<double> &a, double f0
         return (double)t * __hiloint2double(lap_scale_hi(__double2hiint(a.wT), top), __double2loint(a.wT));
     }
     if (mx >= 0x7ff00000) {
-        // an infinity or a NaN decides the sum alone (a run that has blown up is
-        // full of them): its class, in FP32
+        // an infinity or a NaN decides the sum alone: its class, in FP32. (The FP64 sum gives
+        // the same. This keeps a run that has blown up from taking twice as long until
+        // someone looks, and finite fields are no faster without it: two steps at 256^3
+        // 5583 / 5600 us, on NaN 5035 / 10817.)
         auto f = [](double x) {
             const int h = __double2hiint(x);
             const bool finite = (h & 0x7ff00000) != 0x7ff00000, inf = ((h & 0xfffff) | __double2loint(x)) == 0;
@@ -353,7 +356,7 @@ __device__ __forceinline__ double lap_site(const SweepArgs<double> &a, double f0
 // neighbour lies within a factor 2 of f0), so the -30 f0 term of the stencil
 // does not cancel against the neighbour sums: lap = wA sum(f+-1 - f0) +
 // wB sum(f+-2 - f0), two sites per packed instruction where V is even. FP64:
-// the plain weighted sums.
+// lap_site, the weighted sums as integers.
 template <typename T, int V, bool COMP = false>
 __device__ __forceinline__ void star_laplacian(const SweepArgs<T> &a, const T *zm2p, const T *zm1p, const T *P0,
                                                const T *zp1p, const T *zp2p, int at, int bx, T (&lap)[V],
