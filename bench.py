@@ -709,7 +709,7 @@ def run_native(args):
         diag["tagger"] = {"ms": min(t_ev), "n_error_buf": 4, "block": 32, "tagged_fraction": n_tagged / n ** 3}
         del tags
 
-    # ---------------- adjoint step cost on the same FP32 box (recompute sweep A + adjoint sweeps B and A)
+    # ---------------- adjoint step cost on the same FP32 box (stages recomputed, adjoint sweeps B and A)
     adj = None
     if not args.no_adjoint:
         from axion_strings_adaptive_gb300 import adjoint as ADJ
@@ -732,9 +732,9 @@ def run_native(args):
         ms_adj = allmax(ea0.elapsed_time(ea1)) / ka
         fwd_ms = ms_max / args.steps
         adj = {"ms_per_step": ms_adj, "forward_ms_per_step": fwd_ms, "adjoint_over_forward": ms_adj / fwd_ms,
-               "steps": ka, "dtype": "f32", "algorithmic_bytes_per_site": 44 * es32,  # stages 4 + 4, sweep B 16, sweep A 20 words
-               "achieved_gbs": 44 * es32 * n ** 3 / (ms_adj * 1e-3) / 1e9,
-               "kernels_per_step": ["rk4_sweep_A (recompute u3,u4)", "adjoint_sweep_B", "adjoint_sweep_A",
+               "steps": ka, "dtype": "f32", "algorithmic_bytes_per_site": 46 * es32,  # stages 4 + 4 words, sweep B 10 + 8, sweep A 16 + 4
+               "achieved_gbs": 46 * es32 * n ** 3 / (ms_adj * 1e-3) / 1e9,
+               "kernels_per_step": ["stages (recompute u3, u4)", "adjoint_sweep_B", "adjoint_sweep_A",
                                     "lambda_bar_finalize"],
                "finite": bool(torch.isfinite(buf.abar).all())}
         del buf, stored
@@ -819,7 +819,7 @@ def run_native(args):
                 "fp64_rounded_ic_vs_fp64": compare(ref, out[("fp64_rounded_ic", mk)]),
                 "fp64_fp32_storage_vs_fp64": compare(ref, out[("fp64_fp32_storage", mk)])}
         # step times of the legs (the 400-step advance, diagnostics excluded; FP32 levels on
-        # the default tiling, odd first segments on its two-sweep fallback)
+        # the default tiling; an odd segment ends with a copy back)
         precision["ms_per_step"] = {k: step_ms[k] for k in ("fp32", "fp32_compensated", "fp64")}
         fin = precision["by_step"][str(ps)]["fp32_vs_fp64"]
         precision["total_energy_rel_err"] = fin["total_energy_rel_err"]
