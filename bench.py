@@ -7,13 +7,15 @@ FP32 fields (the reference's default PRECISION=FLOAT), FP64 background.
 One "step" = one classic-RK4 step of the whole box: one launch of the one-pass
 fused step, or sweep A and sweep B, whichever tiling the autotuner picks.
 
-Reported on one JSON line: whole-job site-updates/s (value), the FP64 path on
-the same box, FP32-vs-FP64 energy / xi / string-count error after a short
-evolution, the roofline of the dominant step kernel, an end-to-end number
-through the C ABI with host buffers, the CPU oracle baseline and the SM
-clocks sampled during the timed region.
+Reported on one JSON line of a few KB: whole-job site-updates/s (value), the
+roofline of the dominant step kernel, an end-to-end number through the C ABI with
+host buffers, the CPU oracle baseline, the SM clocks sampled during the timed
+region, and under `legs` the main figures of the other measurements: the FP64 path on
+the same box, FP32-vs-FP64 energy error, diagnostics, the adjoint, gradients,
+batching, refined levels, the drop-in calls. --report FILE writes everything that was
+measured (tens of KB: boxes, directions, autotuner times, parts of a step).
 
-  python bench.py [--gpus N] [--steps K] [--warmup W] [--impl native|reference]
+  python bench.py [--gpus N] [--steps K] [--warmup W] [--impl native|reference] [--report FILE]
 """
 from __future__ import annotations
 
@@ -54,6 +56,52 @@ def _config(n, extra=None):
     if extra:
         c.update(extra)
     return c
+
+
+# ---------------------------------------------------------------- the printed line
+# Whole entries of the full report, and the figures of the legs that go on the line.
+LINE_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+             "vs_baseline", "dtype", "data", "config", "cpu_baseline", "clocks", "gpu_launches", "tile_config")
+ROOFLINE_KEYS = ("bound", "achieved", "peak", "unit", "frac", "traffic", "kernel", "peak_source",
+                 "algorithmic_bytes_per_launch")
+E2E_KEYS = ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "ms_per_step", "serial_value",
+            "link_gbs_per_direction")
+LEG_FIGURES = ("fp64.value", "fp64.ms_per_step", "fp64.tile_config", "fp32_over_fp64", "precision.steps",
+               "precision.total_energy_rel_err", "precision.max_energy_rel_err", "diagnostics.per_cell_fp64.ms",
+               "diagnostics.per_cell_fp32.ms", "diagnostics.string_finder_only.ms", "diagnostics.tagger.ms",
+               "adjoint.ms_per_step", "adjoint.achieved_gbs", "adjoint_over_forward",
+               "differentiation.max_rel_err_fp32_vs_fd", "differentiation.grad_psi_rel_err_fp32_vs_fp64",
+               "differentiation.timing_ms.fp32.forward", "differentiation.timing_ms.fp32.backward",
+               "batching.graph_ms", "batching.graph_site_updates_per_s", "batching.speedup_vs_per_box_levels",
+               "scale.ms_per_coarse_step", "scale.site_updates_per_s", "scale_1024.ms_per_coarse_step",
+               "scale_1024.site_updates_per_s", "scale_1024.unavailable", "dropin.f32.ms_per_step",
+               "dropin.f64.ms_per_step")
+
+
+def compact(report):
+    """The printed line of a full report: figures to 9 digits, no long texts."""
+    def short(v):
+        if isinstance(v, float):
+            return float(f"{v:.9g}")
+        if isinstance(v, dict):
+            return {k: short(x) for k, x in v.items()}
+        if isinstance(v, list):
+            return [short(x) for x in v]
+        return v[:200] if isinstance(v, str) else v
+
+    line = {k: report[k] for k in LINE_KEYS if k in report}
+    for part, keys in (("roofline", ROOFLINE_KEYS), ("e2e", E2E_KEYS)):
+        if report.get(part):
+            line[part] = {k: report[part][k] for k in keys if k in report[part]}
+    legs = {}
+    for path in LEG_FIGURES:
+        v = report
+        for k in path.split("."):
+            v = v.get(k) if isinstance(v, dict) else None
+        if v is not None:
+            legs[path] = v
+    line["legs"] = legs
+    return short(line)
 
 
 # ---------------------------------------------------------------- clocks
@@ -922,7 +970,10 @@ def run_native(args):
                 "adjoint": adj, "adjoint_over_forward": adj["adjoint_over_forward"] if adj else None,
                 "differentiation": differentiation, "batching": batching, "scale": scale,
                 "scale_1024": scale_1024, "dropin": dropin}
-        print(json.dumps(line), flush=True)
+        if args.report:
+            with open(args.report, "w") as f:
+                json.dump(line, f, indent=1)
+        print(json.dumps(compact(line)), flush=True)
     if ws > 1:
         dist.destroy_process_group()
 
@@ -933,6 +984,7 @@ def main():
     ap.add_argument("--steps", type=int, default=20)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", choices=["native", "reference"], default="native")
+    ap.add_argument("--report", default=None, help="file for the full report (native arm)")
     ap.add_argument("--n", type=int, default=N_DEFAULT)
     ap.add_argument("--ref-n", type=int, default=N_DEFAULT)
     ap.add_argument("--precision-steps", type=int, default=400)
