@@ -336,18 +336,17 @@ static int config_count(int32_t dtype)
 // and 107 / 111; 300x300x8 37.3 / 30.1 and 131 / 116; 256x16x100 26.1 / 22.8 and 90.7 / 82.5
 // (here the four are decided wrongly); 100x96x96 39.3 / 40.6 and 140 / 163; 8x200x200
 // 39.7 / 47.5 and 143 / 189 (either path runs whole tiles, so narrow levels need no rule of
-// their own). Over 364 calls on levels of 50 000 to 6 million sites the default takes 1.002 as
-// long as the better path, 1.11 at most; the fused step alone 1.053, the sweeps 1.136.
+// their own). Over 364 calls on levels of 50 000 to 6 million sites the default takes 1.001 as
+// long as the better path, 1.12 at most; the fused step alone 1.053, the sweeps 1.135.
 static bool fused_pays(const axs_level *lv, int nsteps, bool copy_back)
 {
     const int cols = (lv->nx + 31) / 32;
     const double two = nsteps * (9.0 + 30e-6 * 32.0 * cols * ((lv->ny + 7) / 8 * 8) * lv->nz);
     if (1.05 * two <= nsteps * 15.0) return false;  // a march of one plane takes longer
-    const int sms = device_sm_count() > 0 ? device_sm_count() : 152;
-    int zchunk = 0, grid = 0;
-    int64_t items = 0;
-    plan_chunks(cols * fused_tiles_ny(lv->ny, 16), lv->nz, sms, zchunk, items, grid);
-    const double planes = (double)((items + grid - 1) / grid) * (zchunk + 8) + 4.0;
+    // the cut with the most chunks that are all in work at once, or whole columns in turn
+    const int sms = device_sm_count() > 0 ? device_sm_count() : 152, ntiles = cols * fused_tiles_ny(lv->ny, 16);
+    const int chunks = std::min(std::max(1, sms / ntiles), (int)lv->nz), turns = (ntiles + sms - 1) / sms;
+    const double planes = (double)turns * ((lv->nz + chunks - 1) / chunks + 8) + 4.0;
     return nsteps * (planes + 2.0) + (copy_back ? 5.0 : 0.0) < 1.05 * two;
 }
 
