@@ -604,7 +604,7 @@ def run_native(args):
         a pair returns the state to the level's state buffer; a single step
         copies it back, so an odd K ends with one of those. Returns (total ms,
         {kernel: mean ms per launch}, clocks)."""
-        fused = "fused" in level_config_name(level)
+        fused = "fused" in level.running_config()[1]
         for w in range(warmup):
             level.advance(bg, TAU_I, t_start + w * DT, DT, 1)
         t0 = t_start + warmup * DT
