@@ -735,13 +735,16 @@ __global__ void __launch_bounds__(kDiagThreads, 2) diag_kernel(const DiagView v,
                             const double g001 = sm.gv[t1][ly][lx], g101 = sm.gv[t1][ly][lx + 1];
                             const double g011 = sm.gv[t1][ly + 1][lx];
                             double s = 0.0;
-                            if (w[0]) s += g000 + g100 + g110 + g010;
-                            if (w[1]) s += g000 + g010 + g011 + g001;
-                            if (w[2]) s += g000 + g001 + g101 + g100;
+                            long long c = 0;
+                            if (w[0]) { s += g000 + g100 + g110 + g010; c += 4; }
+                            if (w[1]) { s += g000 + g010 + g011 + g001; c += 4; }
+                            if (w[2]) { s += g000 + g001 + g101 + g100; c += 4; }
                             vsum += s;
+                            cnt[2] += c;
                         }
+                    } else {
+                        if (q.want_vel) cnt[2] += 4 * ((w[0] != 0) + (w[1] != 0) + (w[2] != 0));
                     }
-                    if (q.want_vel) cnt[2] += 4 * ((w[0] != 0) + (w[1] != 0) + (w[2] != 0));
                 }
             }
             if constexpr (!FAST) {
