@@ -471,3 +471,19 @@ def test_per_cell_fp32_energy_tiles_of_every_remainder(axs, nx, ny, nz, ng):
             np.testing.assert_allclose(list(got.energy_sums), list(ref.energy_sums), rtol=0,
                                        atol=2e-6 * max(abs(e) for e in list(ref.energy_sums)[:12]))
             np.testing.assert_allclose(got.energy_sums[12], ref.energy_sums[12], rtol=2e-6)
+
+
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("want", [(0, 0, 1), (0, 1, 1), (1, 0, 1)])
+def test_velocities_with_and_without_the_other_sums(axs, want, fp32):
+    """The velocity sum and its corner count do not depend on what else is asked for:
+    the count exactly, the sum to the rounding of FP32 terms (1e-6) or of FP64 sums."""
+    n, ng = (37, 20, 18), 2
+    v = np.random.default_rng(6).standard_normal((4, n[2], n[1], n[0]))
+    t = axs.new_fab(n, ng, dtype=torch.float32)
+    t.copy_(_dev(np.pad(v, ((0, 0),) + ((ng, ng),) * 3, mode="wrap"), torch.float32))
+    par = lambda w, f: axs._lib.DiagParams(0.5, 1.3, 2.0, 0.4, 1.0, 1, 0.8, axs._lib.BOUNDARY_GHOSTS, *w, f)  # noqa: E731
+    full, _ = _run_diag(axs, t, ng, par((1, 1, 1), 0))
+    got, _ = _run_diag(axs, t, ng, par(want, fp32))
+    assert full.vel_count == 4 * full.n_p_plain > 0 and got.vel_count == full.vel_count
+    assert got.vel_sum == pytest.approx(full.vel_sum, rel=1e-6 if fp32 else 1e-12, abs=1e-6 * full.vel_count if fp32 else 0)
