@@ -375,3 +375,22 @@ def test_f64_laplacian_weighs_no_site_alike_wrong(axs, dx):
     ref = y + h / 6 * (k1 + 2 * k2 + 2 * k3 + rhs(y + h * k3, 1.0 + dt))
     err, inc = (got - ref)[2:], (ref - y)[2:]
     assert abs(float((err * inc).sum() / (inc ** 2).sum())) < 2.0 ** -56
+
+
+@pytest.mark.parametrize("shape", [(4, 2, 1), (16, 8, 2), (34, 9, 97), (98, 75, 50), (18, 130, 33), (130, 34, 7), (64, 64, 64)])
+def test_f64_chunk_plans_cover_every_plane(axs, shape):
+    """The FP64 sweeps' chunks of planes, planned by the fullest SM's work: levels of a
+    few planes and of one chunk, uneven last chunks, more tiles than SMs and fewer. Every
+    tiling has another plan and leaves the same bits, padding included; three steps."""
+    nx, ny, nz = shape
+    v = torch.from_numpy(np.random.default_rng(nx + ny + nz).standard_normal((4, nz, ny, nx))).cuda()
+    v[:2] += 1.5
+    bg = axs.Background.expanding(2.0, 1.0, lambda0=2.0)
+    ref = None
+    for cid, name in [(0, "default")] + axs.PeriodicLevel((16, 8, 2), 0.5, dtype=torch.float64).tile_configs():
+        lv = axs.PeriodicLevel(shape, 0.5, dtype=torch.float64, tile_config=cid)
+        lv.set_state(v)
+        lv.advance(bg, 1.0, 0.0, 0.05, 3)
+        lv.device_status()
+        ref = lv.state.clone() if ref is None else ref
+        assert torch.equal(lv.state, ref), name
